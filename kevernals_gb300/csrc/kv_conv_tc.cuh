@@ -1,29 +1,54 @@
 // kv_conv_tc.cuh -- 3x3x3 convolution as an implicit GEMM on the Blackwell
 // tensor cores: TMA tile loads into swizzled shared memory, tcgen05.mma with
-// the accumulator in tensor memory (TMEM), tcgen05.ld epilogue.
+// the accumulators in tensor memory (TMEM), tcgen05.ld epilogue.
 //
-// GEMM view (channels-last activations [D][H][W][C], BF16):
-//   D[m][n] = sum over taps t and input channels k of A_t[m][k] * B_t[n][k]
-//   m: a CTA tile of 128*T voxels (T = 1, 2 or 4 sub-tiles of 128, one MMA
-//      each, all sharing the stage's weight slice), BW x BH x BD (x, y, z)
-//      with BW = min(W, 128), BH = min(H, 128*T / BW), BD = the rest;
-//      n: output channels (N = 16..256),
-//   k: input channels of the (possibly concatenated) input, in segments of
-//      16 / 32 / 64 channels (one TMA box each; 128-channel inputs are two
-//      segments).
-// A_t is the input shifted by tap t = (dz,dy,dx): the TMA box starts at
-// (x0+dx, y0+dy, z0+dz); coordinates outside the volume read zeros, which is
-// the convolution's zero padding.  B_t is the weight slice w[n][t][k]
-// ([Cout][27][Cin] layout, K contiguous), also one TMA box per segment.
-// Both operands are K-major with the swizzle matching the segment's row
-// width (32 / 64 / 128 bytes); one tcgen05.mma (M=128, N, K=16, BF16 in,
-// FP32 accumulate) per 16 channels.
+// GEMM view (channels-last activations [D][H][W][C], BF16): M = voxels, N =
+// output channels, K = 27 taps x input channels.
 //
-// Warp roles (192 threads): warp 0 issues the TMA loads into a ring of
-// stages (one tap of every segment per stage), warp 1 owns the TMEM
-// allocation and issues the MMAs (one elected thread), warps 2-5 drain the
-// accumulator (each warp reads its 32 TMEM lanes = 32 voxels), add the bias,
-// apply ReLU, convert to BF16 and store.  The CTA is persistent over tiles.
+// What bounds it and why it is cut this way.  A tile load per tap reads every
+// activation 27 times through L2, and an MMA of N = 16 output channels reads
+// 128 rows of A from shared memory (32 cycles at 128 B a cycle) for 8 cycles
+// of arithmetic.  So a CTA marches along z over a column of the volume
+// (BW x BY voxels, x by y): each input plane is loaded once, with a halo of
+// one voxel, 16 channels at a time, and
+//   * the nine (dy, dx) taps are the same shared-memory tile read from
+//     another first row: a voxel is one 32-byte row, rows lie BW + 2 to the
+//     next y, so a tap is a row offset of the operand's start address;
+//   * the three dz taps are stacked along N: plane z times [W(dz=0) W(dz=1)
+//     W(dz=2)] is added to the accumulators of the output planes z + 1, z and
+//     z - 1 with one read of A.  Each 128-voxel sub-tile keeps three
+//     accumulators (slots) in TMEM; output plane z uses slot (-z) mod 3, so the
+//     three lie in the order of dz, cyclically.  Where the cycle wraps the MMA
+//     is split in two, or, where shared memory allows it, the weights are kept
+//     as five groups dz = 0 1 2 0 1 and the MMA starts at the rotated one.
+// An output plane is finished with dz = 2, read out, and its slot zeroed for
+// the plane three further on: every MMA accumulates.  Sums run over dz, then
+// (dy, dx), then 16-channel segments -- the tap order of the mma.sync kernel,
+// with equal bits -- so a plane's segments are all in shared memory at once.
+// The weights stay there for the CTA's life where they fit beside the plane
+// buffers; else they stream through a ring, one (dy, dx) of up to four
+// segments at a time, each piece used for every sub-tile.
+//
+// M = 128 rows are 128 consecutive voxels of the padded plane: either one y
+// row (BW = 128; sub-tile t = row t) or, where the volume is narrower,
+// consecutive rows with their halo columns in between, whose results are not
+// stored.  The host takes the shape with the least estimated time.
+//
+// Measured on a GB300, against a kernel that loaded one tile per tap and
+// issued one N = Cout MMA per tap and 16 channels: 32+16 -> 16 channels at
+// 128 x 256 x 128 voxels 1434 -> 230 us (755 TFLOP/s); the thirteen layers of
+// the U-Net at 128 x 512 x 512 voxels 31.9 -> 6.0 ms, forward and
+// backward-data at 128 x 256 x 128 8.1 -> 2.1 ms.
+//
+// Warp roles (352 threads): warp 0 issues the TMA loads of the planes and of
+// streamed weights, warps 1 and 10 issue the MMAs of the even and
+// the odd sub-tiles (an MMA takes ~45 cycles and a sub-tile's waits, commit and
+// address set-up ~240: two issuers keep the tensor pipe fed; one took 284 us
+// where two take 203 on the layer below; warp 1 owns the TMEM allocation),
+// warps 2-9 drain the accumulators (each warp
+// its 32 TMEM lanes = 32 voxels; two sets of four warps take the sub-tiles in
+// turn), add the bias, apply ReLU or the caller's mask, convert to BF16 and
+// store.  The CTA is persistent over its share of (column, plane) units.
 // Every wait on an mbarrier is bounded: on timeout the thread records an
 // error code, raises the CTA's abort flag and every role winds down, so a
 // fault in the pipeline ends the kernel with a status instead of a hang.
@@ -31,6 +56,7 @@
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 
@@ -38,33 +64,38 @@
 
 namespace convtc {
 
-constexpr int kThreads = 192;
-constexpr int kMaxSeg = 4;        // input channel segments (e.g. 64 + 64 + 64 for 192 channels)
+constexpr int kThreads = 352;
+constexpr int kIssuers = 2;       // warps that issue MMAs
+constexpr int kEpilogueSets = 2;  // sets of four warps that drain accumulators
 constexpr int kTileM = 128;
+constexpr int kSeg = 16;          // channels per segment: one K step, one 32-byte row per voxel
+constexpr int kRow = kSeg * 2;    // bytes of a row
+constexpr int kMaxT = 10;         // sub-tiles per column (512 TMEM columns / 3 slots of 16)
+constexpr int kMaxStages = 4;     // plane buffers
+constexpr int kMaxChunks = 8;     // ring of streamed weights
+constexpr int kChunkSegs = 4;     // segments in one piece of streamed weights
 constexpr uint32_t kWaitLimit = 1u << 22;   // try_wait rounds before a wait is declared failed
 
-struct SegInfo {
-    int n;                        // number of segments
-    int kseg[kMaxSeg];            // channels in each segment (16, 32 or 64)
-    int src[kMaxSeg];             // which activation map (0 or 1)
-    int c0[kMaxSeg];              // first channel of the segment within its activation tensor
-    int kglob[kMaxSeg];           // first channel of the segment within the concatenated input
-    uint32_t a_off[kMaxSeg];      // byte offset of the segment's A tile within a stage
-    uint32_t b_off[kMaxSeg];      // byte offset of the segment's B tile within a stage
-};
-
 struct Params {
-    SegInfo seg;
-    int N;                        // output channels
+    int nseg, nseg1;              // input segments; the first nseg1 come from the first tensor
+    int N, ncg;                   // output channels; groups of CG channels, one per CTA
     int D, H, W;                  // this level's volume
-    int BW, BH, BD;               // tile extent in x, y and z (BW * BH * BD = 128 * T)
-    int T;                        // 128-voxel sub-tiles (MMAs) per tile
-    long long tiles;
-    uint32_t stage_bytes, stages, tmem_cols;
-    uint32_t tx_bytes;            // bytes the TMA loads of one stage deliver
-    uint32_t idesc;               // tcgen05 instruction descriptor
+    int BW, BY, pitch;            // column extent in x and y; rows from one y to the next (BW + 2)
+    int T, mstep;                 // sub-tiles; rows between their first rows
+    uint32_t pitch_magic;         // ceil(2^20 / pitch): row / pitch by multiplication
+    int tiles_x;                  // columns in x
+    long long units;              // columns x planes, of one channel group
+    int groups;                   // dz groups of the weights in shared memory (3 or 5)
+    int resident;                 // the weights stay in shared memory
+    uint32_t stages, a_bytes;     // plane buffers; bytes of one segment of a plane
+    uint32_t a_tx;                // bytes the TMA load of one segment of a plane delivers
+    uint32_t b_off;               // first byte of the weights
+    uint32_t b_seg_bytes;         // weights of one segment (resident: nine taps, streamed: one)
+    uint32_t chunks;              // ring of streamed weights, kChunkSegs segments each
+    uint32_t tmem_cols;
     const float *bias;            // nullptr: none
     int relu;
+    const __nv_bfloat16 *mask;    // nullptr: none; else outputs where mask <= 0 become 0
     __nv_bfloat16 *out;           // [voxels][N]
     int *status;                  // 0 ok; set on a failed wait
 };
@@ -95,17 +126,26 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                       uint32_t accumulate) {
+// One thread of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(pred));
+    return pred != 0;
+}
+
+// D += A B, issued by one thread; the descriptors' low words (start address) differ from MMA to MMA, the high word is
+// the same for every operand.
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
+            "{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, 1, 0;\n mov.b64 a, {%1, %3};\n mov.b64 b, {%2, %3};\n"
+            " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n}\n" ::"r"(tmem_d),
+            "r"(alo), "r"(blo), "r"(hi), "r"(idesc)
+            : "memory");
 }
 
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+    if (elect_one())
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
 
@@ -118,47 +158,87 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Shared-memory matrix descriptor of a K-major operand tile whose rows are
-// `row_bytes` (32 / 64 / 128) long, stored with the matching swizzle by TMA:
-// start address >> 4 (bits 0-13), leading byte offset (unused for swizzled
-// K-major tiles, 16 bytes) >> 4 (16-29), stride byte offset = 8 rows >> 4
-// (32-45), descriptor version 1 (46-47), swizzle mode (61-63:
-// 6 = 32 B, 4 = 64 B, 2 = 128 B).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t row_bytes) {
-    const uint64_t layout = row_bytes == 128 ? 2ull : (row_bytes == 64 ? 4ull : 6ull);
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFFu);
-    d |= (uint64_t)1u << 16;
-    d |= (uint64_t)(((8u * row_bytes) >> 4) & 0x3FFFu) << 32;
-    d |= 1ull << 46;
-    d |= layout << 61;
-    return d;
+// zeroes 16 columns of the warp's 32 lanes
+__device__ __forceinline__ void tc_zero16(uint32_t taddr) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+        "r"(0u)
+        : "memory");
 }
 
+// Shared-memory matrix descriptor of a K-major operand tile of 32-byte rows
+// stored with the 32-byte swizzle by TMA: start address >> 4 (bits 0-13),
+// leading byte offset (unused for swizzled K-major tiles, 16 bytes) >> 4
+// (16-29), stride byte offset = 8 rows >> 4 (32-45), descriptor version 1
+// (46-47), swizzle mode (61-63: 6 = 32 B).  The swizzle follows the address
+// (TMA wrote the tile from a 1024-byte boundary), so a start address at any
+// row reads the rows from there on.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1u << 16) | ((uint64_t)((8u * kRow) >> 4) << 32) |
+           (1ull << 46) | (6ull << 61);
+}
+
+// The MMAs of NT taps (nine, or the one that `a` and the weights start at) of NS segments for one sub-tile, tap by
+// tap, one piece (n1 == 0) or two; called by a converged warp, issued by one thread.
+template <int NT, int NS>
+__device__ __forceinline__ void issue_taps(uint32_t t0, uint32_t t1, uint32_t a, uint32_t b0, uint32_t b1, uint32_t hi,
+                                           uint32_t id0, uint32_t id1, int n1, uint32_t y_step, uint32_t tap_step,
+                                           uint32_t a_seg, uint32_t b_seg) {
+    if (elect_one()) {
+        if (n1 == 0) {
+#pragma unroll
+            for (int tap = 0; tap < NT; ++tap)
+#pragma unroll
+                for (int s = 0; s < NS; ++s)
+                    tc_mma(t0, a + (tap / 3) * y_step + (tap % 3) * (kRow >> 4) + s * a_seg,
+                           b0 + tap * tap_step + s * b_seg, hi, id0);
+        } else {
+#pragma unroll
+            for (int tap = 0; tap < NT; ++tap)
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    const uint32_t as = a + (tap / 3) * y_step + (tap % 3) * (kRow >> 4) + s * a_seg;
+                    tc_mma(t0, as, b0 + tap * tap_step + s * b_seg, hi, id0);
+                    tc_mma(t1, as, b1 + tap * tap_step + s * b_seg, hi, id1);
+                }
+        }
+    }
+    __syncwarp();
+}
+
+template <int CG>
 __global__ void __launch_bounds__(kThreads, 1)
-    conv3_tc_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
-                    const __grid_constant__ CUtensorMap map_b, const __grid_constant__ Params P) {
+    conv3_march_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
+                       const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b2,
+                       const __grid_constant__ Params P) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_full, acc_empty, drain_bar;
+    __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_full[kMaxT], acc_empty[kMaxT],
+        b_full[kMaxChunks], b_empty[kMaxChunks], drain_bar[kIssuers];
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_flag;
-    __shared__ unsigned long long issued_sh, consumed_sh;   // stages loaded by TMA / consumed by MMA
+    __shared__ unsigned long long issued_sh, b_issued_sh;   // planes / pieces of weights loaded by TMA
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // stage ring, 1024-byte aligned (the 128-byte swizzle repeats every 8 rows)
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (uint32_t s = 0; s < P.stages; ++s) {
             mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
+            mbar_init(&empty_bar[s], kIssuers);
         }
-        mbar_init(&acc_full, 1);
-        mbar_init(&acc_empty, 4);
-        mbar_init(&drain_bar, 1);
+        for (int t = 0; t < P.T; ++t) {
+            mbar_init(&acc_full[t], 1);
+            mbar_init(&acc_empty[t], 4);
+        }
+        for (int i = 0; i < kMaxChunks; ++i) {
+            mbar_init(&b_full[i], 1);
+            mbar_init(&b_empty[i], kIssuers);
+        }
+        for (int i = 0; i < kIssuers; ++i) mbar_init(&drain_bar[i], 1);
         issued_sh = 0;
-        consumed_sh = 0;
+        b_issued_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -173,137 +253,273 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_sh;
-    const int tiles_x = P.W / P.BW, tiles_y = P.H / P.BH;   // tiles_z = D / BD
+    if (warp >= 2 && warp < 6) {   // every accumulator starts at zero
+        for (uint32_t c = 0; c < P.tmem_cols; c += 16) tc_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c);
+        tc_wait_st();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+
+    // this CTA's channel group and its range of (column, plane) units
+    const int cg = (int)blockIdx.x % P.ncg;
+    const long long part = (long long)blockIdx.x / P.ncg, parts = (long long)gridDim.x / P.ncg;
+    const long long u_begin = P.units * part / parts, u_end = P.units * (part + 1) / parts;
 
     if (warp == 0) {
         // ---------------------------------------------------------- TMA producer
         if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
-            for (long long tile = blockIdx.x; tile < P.tiles && !abort_flag; tile += gridDim.x) {
-                const int tx = (int)(tile % tiles_x);
-                const long long r = tile / tiles_x;
-                const int ty = (int)(r % tiles_y), tz = (int)(r / tiles_y);
-                const int x0 = tx * P.BW, y0 = ty * P.BH, z0 = tz * P.BD;
-                for (int tap = 0; tap < 27; ++tap) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag, P.status, 1)) break;
-                    mbar_arrive_expect_tx(&full_bar[stage], P.tx_bytes);
-                    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                    const uint32_t sb = base + stage * P.stage_bytes;
-                    for (int s = 0; s < P.seg.n; ++s) {
-                        const CUtensorMap *ma = P.seg.src[s] == 0 ? &map_a0 : &map_a1;
-                        tma_load_4d(sb + P.seg.a_off[s], ma, &full_bar[stage], P.seg.c0[s], x0 + dx, y0 + dy,
-                                    z0 + dz);
-                        tma_load_3d(sb + P.seg.b_off[s], &map_b, &full_bar[stage], P.seg.kglob[s], tap, 0);
+            if (P.resident) {
+                mbar_arrive_expect_tx(&b_full[0], P.b_seg_bytes * (uint32_t)P.nseg);
+                for (int s = 0; s < P.nseg; ++s) {
+                    const uint32_t sb = base + P.b_off + (uint32_t)s * P.b_seg_bytes;
+                    if (P.groups == 5) {
+                        for (int tap = 0; tap < 9; ++tap) {
+                            const uint32_t tb = sb + (uint32_t)(tap * 5 * CG * kRow);
+                            tma_load_4d(tb, &map_b, &b_full[0], s * kSeg, cg * CG, 0, tap);
+                            tma_load_4d(tb + 3u * CG * kRow, &map_b2, &b_full[0], s * kSeg, cg * CG, 0, tap);
+                        }
+                    } else {
+                        tma_load_4d(sb, &map_b, &b_full[0], s * kSeg, cg * CG, 0, 0);
                     }
+                }
+                b_issued_sh = 1;
+            }
+            uint32_t stage = 0, phase = 0, chunk = 0, bphase = 0;
+            bool ok = true;
+            for (long long u = u_begin; u < u_end && ok;) {
+                const int col = (int)(u / P.D), zs = (int)(u % P.D);
+                const int ze = (int)(u_end - u < P.D - zs ? zs + (u_end - u) : P.D);
+                const int x0 = (col % P.tiles_x) * P.BW, y0 = (col / P.tiles_x) * P.BY;
+                for (int z = max(zs - 1, 0); z <= min(ze, P.D - 1) && ok; ++z) {
+                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag, P.status, 1)) { ok = false; break; }
+                    mbar_arrive_expect_tx(&full_bar[stage], P.a_tx * (uint32_t)P.nseg);
+                    const uint32_t sb = base + stage * (uint32_t)P.nseg * P.a_bytes;
+                    for (int s = 0; s < P.nseg; ++s)
+                        tma_load_4d(sb + (uint32_t)s * P.a_bytes, s < P.nseg1 ? &map_a0 : &map_a1, &full_bar[stage],
+                                    (s < P.nseg1 ? s : s - P.nseg1) * kSeg, x0 - 1, y0 - 1, z);
                     ++issued_sh;
                     if (++stage == P.stages) { stage = 0; phase ^= 1u; }
+                    if (P.resident) continue;
+                    for (int tap = 0; tap < 9 && ok; ++tap)
+                        for (int s0 = 0; s0 < P.nseg; s0 += kChunkSegs) {
+                            const int ns = min(kChunkSegs, P.nseg - s0);
+                            if (!mbar_wait(&b_empty[chunk], bphase ^ 1u, &abort_flag, P.status, 7)) { ok = false; break; }
+                            mbar_arrive_expect_tx(&b_full[chunk], P.b_seg_bytes * (uint32_t)ns);
+                            const uint32_t cb = base + P.b_off + chunk * (uint32_t)kChunkSegs * P.b_seg_bytes;
+                            for (int s = 0; s < ns; ++s)
+                                tma_load_4d(cb + (uint32_t)s * P.b_seg_bytes, &map_b, &b_full[chunk],
+                                            (s0 + s) * kSeg, cg * CG, 0, tap);
+                            ++b_issued_sh;
+                            if (++chunk == P.chunks) { chunk = 0; bphase ^= 1u; }
+                        }
                 }
+                u += ze - zs;
             }
         }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            // descriptors of stage 0; a later stage, K step or sub-tile only adds
-            // its byte offset >> 4 to the start-address field (shared-memory
-            // addresses stay below 2^18, so the 14-bit field never carries)
-            uint64_t desc_a[kMaxSeg], desc_b[kMaxSeg];
-#pragma unroll
-            for (int s = 0; s < kMaxSeg; ++s) {
-                desc_a[s] = smem_desc(base + P.seg.a_off[s], (uint32_t)P.seg.kseg[s] * 2u);
-                desc_b[s] = smem_desc(base + P.seg.b_off[s], (uint32_t)P.seg.kseg[s] * 2u);
-            }
-            uint32_t stage = 0, phase = 0, acc_phase = 0;
-            for (long long tile = blockIdx.x; tile < P.tiles && !abort_flag; tile += gridDim.x) {
-                if (!mbar_wait(&acc_empty, acc_phase ^ 1u, &abort_flag, P.status, 2)) break;
-                acc_phase ^= 1u;
+    } else if (warp == 1 || warp == 10) {
+        // ---------------------------------------------------------- MMA issuers
+        const int issuer = warp == 1 ? 0 : 1;
+        // The whole warp runs this role converged (every wait's outcome is agreed on by a vote) and one elected
+        // thread issues: the operands of tcgen05.mma live in uniform registers, and values computed in a
+        // one-thread branch would have to be moved there MMA by MMA.
+        //
+        // kind::f16 instruction descriptor: FP32 accumulator (bits 4-5 = 1), BF16 A
+        // and B (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bits 17-22, M >> 4 at 24-28
+        constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileM >> 4) << 24);
+        constexpr uint32_t kIdescN = (uint32_t)(CG >> 3) << 17;   // per dz group
+        constexpr uint32_t kGroup = (uint32_t)(CG * kRow) >> 4;
+        constexpr uint32_t kRowStep = kRow >> 4;
+        const uint32_t ubase = __shfl_sync(0xffffffffu, base, 0), utmem = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint32_t lo0 = (uint32_t)smem_desc(ubase), hi = (uint32_t)(smem_desc(0) >> 32);
+        const uint32_t tap_step = (uint32_t)P.groups * kGroup, y_step = (uint32_t)P.pitch * kRowStep;
+        const uint32_t a_seg = P.a_bytes >> 4, b_seg = P.b_seg_bytes >> 4;
+        auto wait = [&](uint64_t *bar, uint32_t parity, int code) {
+            return __all_sync(0xffffffffu, mbar_wait(bar, parity, &abort_flag, P.status, code));
+        };
+        uint32_t stage = 0, phase = 0, plane_phase = 0, chunk = 0, bphase = 0;
+        bool ok = true;
+        if (P.resident && u_begin < u_end) ok = wait(&b_full[0], 0, 8);
+        for (long long u = u_begin; u < u_end && ok;) {
+            const int zs = (int)(u % P.D);
+            const int ze = (int)(u_end - u < P.D - zs ? zs + (u_end - u) : P.D);
+            for (int z = max(zs - 1, 0); z <= min(ze, P.D - 1) && ok; ++z) {
+                // dz groups of plane z that fall on output planes zs .. ze-1 (plane z + 1 - dz), and the
+                // slot of dz = 0; one piece, or two where the slots wrap
+                const int dlo = max(0, z + 2 - ze), dhi = min(2, z + 1 - zs);
+                const int c = (2 * (z + 1)) % 3;          // (-(z + 1)) mod 3
+                int n0, b0, d0, n1 = 0, b1 = 0, d1 = 0;   // pieces: groups, first weight group, first slot
+                if (P.groups == 5 && dlo == 0 && dhi == 2) {
+                    n0 = 3;
+                    b0 = (3 - c) % 3;
+                    d0 = 0;
+                } else {
+                    const int wrap = min(max(3 - c, dlo), dhi + 1);   // first dz past the wrap
+                    n0 = wrap - dlo;
+                    b0 = dlo;
+                    d0 = dlo + c;
+                    n1 = dhi + 1 - wrap;
+                    b1 = wrap;
+                    d1 = wrap + c - 3;
+                    if (n0 == 0) {
+                        n0 = n1;
+                        b0 = b1;
+                        d0 = d1;
+                        n1 = 0;
+                    }
+                }
+                const uint32_t id0 = kIdesc + (uint32_t)n0 * kIdescN, id1 = kIdesc + (uint32_t)n1 * kIdescN;
+                const uint32_t bo0 = (uint32_t)b0 * kGroup, bo1 = (uint32_t)b1 * kGroup;
+                if (!wait(&full_bar[stage], phase, 3)) { ok = false; break; }
                 tc_fence_after();
-                bool ok = true;
-                for (int tap = 0; tap < 27 && ok; ++tap) {
-                    if (!mbar_wait(&full_bar[stage], phase, &abort_flag, P.status, 3)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t so = (uint64_t)((stage * P.stage_bytes) >> 4);
-#pragma unroll
-                    for (int s = 0; s < kMaxSeg; ++s) {
-                        if (s >= P.seg.n) break;
-                        const uint64_t sub = (uint64_t)((kTileM * P.seg.kseg[s] * 2) >> 4);   // one sub-tile
-                        for (int k = 0; k < P.seg.kseg[s]; k += 16) {
-                            const uint64_t ko = (uint64_t)((k * 2) >> 4);                   // 32 B per K step
-                            const uint64_t bd = desc_b[s] + so + ko;
-                            for (int j = 0; j < P.T; ++j)   // sub-tile j: rows 128j.., TMEM columns jN..
-                                tc_mma(tmem + (uint32_t)(j * P.N), desc_a[s] + so + ko + (uint64_t)j * sub, bd,
-                                       P.idesc, (tap > 0 || s > 0 || k > 0) ? 1u : 0u);
+                const uint32_t da0 = lo0 + ((stage * (uint32_t)P.nseg * P.a_bytes) >> 4), db0 = lo0 + (P.b_off >> 4);
+                if (P.resident) {
+                    for (int t = issuer; t < P.T; t += kIssuers) {
+                        if (!wait(&acc_empty[t], plane_phase ^ 1u, 2)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t dt = utmem + (uint32_t)(t * 3 * CG);
+                        const uint32_t t0 = dt + (uint32_t)(d0 * CG), t1 = dt + (uint32_t)(d1 * CG);
+                        const uint32_t at = da0 + (uint32_t)(t * P.mstep) * kRowStep;
+                        switch (P.nseg) {
+                        case 1: issue_taps<9, 1>(t0, t1, at, db0 + bo0, db0 + bo1, hi, id0, id1, n1, y_step, tap_step, a_seg, b_seg); break;
+                        case 2: issue_taps<9, 2>(t0, t1, at, db0 + bo0, db0 + bo1, hi, id0, id1, n1, y_step, tap_step, a_seg, b_seg); break;
+                        case 3: issue_taps<9, 3>(t0, t1, at, db0 + bo0, db0 + bo1, hi, id0, id1, n1, y_step, tap_step, a_seg, b_seg); break;
+                        default: issue_taps<9, 4>(t0, t1, at, db0 + bo0, db0 + bo1, hi, id0, id1, n1, y_step, tap_step, a_seg, b_seg); break;
+                        }
+                        tc_commit(&acc_full[t]);   // the plane's sums are in
+                    }
+                } else {
+                    for (int tap = 0; tap < 9 && ok; ++tap) {
+                        const uint32_t ay = da0 + (uint32_t)(tap / 3) * y_step + (uint32_t)(tap % 3) * kRowStep;
+                        for (int s0 = 0; s0 < P.nseg; s0 += kChunkSegs) {
+                            if (!wait(&b_full[chunk], bphase, 9)) { ok = false; break; }
+                            tc_fence_after();
+                            const uint32_t db = db0 + chunk * (uint32_t)kChunkSegs * b_seg;
+                            for (int t = issuer; t < P.T; t += kIssuers) {
+                                if (tap == 0 && s0 == 0) {
+                                    if (!wait(&acc_empty[t], plane_phase ^ 1u, 2)) { ok = false; break; }
+                                    tc_fence_after();
+                                }
+                                const uint32_t dt = utmem + (uint32_t)(t * 3 * CG);
+                                const uint32_t t0 = dt + (uint32_t)(d0 * CG), t1 = dt + (uint32_t)(d1 * CG);
+                                const uint32_t at = ay + (uint32_t)(t * P.mstep) * kRowStep + (uint32_t)s0 * a_seg;
+                                switch (P.nseg - s0) {
+                                case 1: issue_taps<1, 1>(t0, t1, at, db + bo0, db + bo1, hi, id0, id1, n1, 0u, 0u, a_seg, b_seg); break;
+                                case 2: issue_taps<1, 2>(t0, t1, at, db + bo0, db + bo1, hi, id0, id1, n1, 0u, 0u, a_seg, b_seg); break;
+                                case 3: issue_taps<1, 3>(t0, t1, at, db + bo0, db + bo1, hi, id0, id1, n1, 0u, 0u, a_seg, b_seg); break;
+                                default: issue_taps<1, 4>(t0, t1, at, db + bo0, db + bo1, hi, id0, id1, n1, 0u, 0u, a_seg, b_seg); break;
+                                }
+                            }
+                            if (!ok) break;
+                            tc_commit(&b_empty[chunk]);
+                            if (++chunk == P.chunks) { chunk = 0; bphase ^= 1u; }
                         }
                     }
-                    tc_commit(&empty_bar[stage]);      // frees the stage when these MMAs are done
-                    ++consumed_sh;
-                    if (++stage == P.stages) { stage = 0; phase ^= 1u; }
+                    if (ok)
+                        for (int t = issuer; t < P.T; t += kIssuers) tc_commit(&acc_full[t]);
                 }
                 if (!ok) break;
-                tc_commit(&acc_full);                  // the tile's accumulator is complete
+                tc_commit(&empty_bar[stage]);      // frees the plane when these MMAs are done
+                if (++stage == P.stages) { stage = 0; phase ^= 1u; }
+                plane_phase ^= 1u;
             }
+            u += ze - zs;
         }
+        // every MMA has completed before TMEM is released (below)
+        tc_commit(&drain_bar[issuer]);
+        volatile int never = 0;
+        mbar_wait(&drain_bar[issuer], 0, &never, P.status, 6);
     } else {
-        // ---------------------------------------------------------- epilogue (warps 2-5)
+        // ---------------------------------------------------------- epilogue (warps 2-9)
         const int quarter = warp & 3;                  // TMEM lanes 32*quarter .. +31
-        uint32_t acc_phase = 0;
-        for (long long tile = blockIdx.x; tile < P.tiles; tile += gridDim.x) {
-            const bool got = mbar_wait(&acc_full, acc_phase, &abort_flag, P.status, 4);
-            if (!__all_sync(0xffffffffu, got)) break;    // warp-uniform: tcgen05.ld below is .sync.aligned
-            acc_phase ^= 1u;
-            tc_fence_after();
-            const int tx = (int)(tile % tiles_x);
-            const long long r = tile / tiles_x;
-            const int ty = (int)(r % tiles_y), tz = (int)(r / tiles_y);
-          for (int j = 0; j < P.T; ++j) {
-            const int m = j * kTileM + quarter * 32 + lane;   // voxel row of the tile
-            const int x = tx * P.BW + (m % P.BW), y = ty * P.BH + (m / P.BW) % P.BH;
-            const int z = tz * P.BD + m / (P.BW * P.BH);
-            const long long vox = ((long long)z * P.H + y) * P.W + x;
-            __nv_bfloat16 *dst = P.out + vox * P.N;
-            for (int c = 0; c < P.N; c += 16) {
-                uint32_t v[16];
-                tc_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(j * P.N + c), v);
-                tc_wait_ld();
-                __align__(16) __nv_bfloat162 o[8];
+        const int set = (warp - 2) >> 2;
+        uint32_t plane_phase = 0;
+        bool ok = true;
+        for (long long u = u_begin; u < u_end && ok;) {
+            const int col = (int)(u / P.D), zs = (int)(u % P.D);
+            const int ze = (int)(u_end - u < P.D - zs ? zs + (u_end - u) : P.D);
+            const int x0 = (col % P.tiles_x) * P.BW, y0 = (col / P.tiles_x) * P.BY;
+            for (int z = max(zs - 1, 0); z <= min(ze, P.D - 1) && ok; ++z) {
+                for (int t = set; t < P.T; t += kEpilogueSets) {
+                    const bool got = mbar_wait(&acc_full[t], plane_phase, &abort_flag, P.status, 4);
+                    if (!__all_sync(0xffffffffu, got)) { ok = false; break; }   // warp-uniform: tcgen05.ld is .sync.aligned
+                    tc_fence_after();
+                    const uint32_t row = (uint32_t)(t * P.mstep + quarter * 32 + lane);
+                    const uint32_t yy = (row * P.pitch_magic) >> 20, xx = row - yy * (uint32_t)P.pitch;
+                    const int x = x0 + (int)xx, y = y0 + (int)yy;
+                    const bool live = xx < (uint32_t)P.BW && yy < (uint32_t)P.BY && x < P.W && y < P.H;
+                    // plane z finishes output plane z - 1, and itself where no plane follows
+                    for (int zo = max(z - 1, zs); zo <= z; ++zo) {
+                        if (zo == z && !(z == P.D - 1 && ze == P.D)) break;
+                        const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) +
+                                            (uint32_t)((t * 3 + (2 * zo) % 3) * CG);
+                        uint32_t v[CG / 16][16];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float a = __uint_as_float(v[2 * j]), b = __uint_as_float(v[2 * j + 1]);
-                    if (P.bias != nullptr) {
-                        a += P.bias[c + 2 * j];
-                        b += P.bias[c + 2 * j + 1];
+                        for (int q = 0; q < CG / 16; ++q) tc_ld16(ta + (uint32_t)(16 * q), v[q]);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int q = 0; q < CG / 16; ++q) tc_zero16(ta + (uint32_t)(16 * q));
+                        if (live) {
+                            const size_t o = (((size_t)zo * P.H + y) * P.W + x) * P.N + cg * CG;
+#pragma unroll
+                            for (int q = 0; q < CG / 16; ++q) {
+                                __align__(16) __nv_bfloat162 r[8];
+                                __align__(16) __nv_bfloat162 m[8];
+                                if (P.mask != nullptr) {
+                                    const uint4 *ms = reinterpret_cast<const uint4 *>(P.mask + o + 16 * q);
+                                    reinterpret_cast<uint4 *>(m)[0] = __ldg(ms);
+                                    reinterpret_cast<uint4 *>(m)[1] = __ldg(ms + 1);
+                                }
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) {
+                                    float a = __uint_as_float(v[q][2 * j]), b = __uint_as_float(v[q][2 * j + 1]);
+                                    if (P.bias != nullptr) {
+                                        a += __ldg(P.bias + cg * CG + 16 * q + 2 * j);
+                                        b += __ldg(P.bias + cg * CG + 16 * q + 2 * j + 1);
+                                    }
+                                    if (P.relu) {
+                                        a = fmaxf(a, 0.f);
+                                        b = fmaxf(b, 0.f);
+                                    }
+                                    if (P.mask != nullptr) {
+                                        const float2 mf = __bfloat1622float2(m[j]);
+                                        if (!(mf.x > 0.f)) a = 0.f;
+                                        if (!(mf.y > 0.f)) b = 0.f;
+                                    }
+                                    r[j] = __floats2bfloat162_rn(a, b);
+                                }
+                                uint4 *d4 = reinterpret_cast<uint4 *>(P.out + o + 16 * q);
+                                d4[0] = reinterpret_cast<const uint4 *>(r)[0];
+                                d4[1] = reinterpret_cast<const uint4 *>(r)[1];
+                            }
+                        }
+                        __syncwarp();
                     }
-                    if (P.relu) {
-                        a = fmaxf(a, 0.f);
-                        b = fmaxf(b, 0.f);
-                    }
-                    o[j] = __floats2bfloat162_rn(a, b);
+                    tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[t]);
                 }
-                const uint4 *src = reinterpret_cast<const uint4 *>(o);
-                uint4 *d4 = reinterpret_cast<uint4 *>(dst + c);
-                d4[0] = src[0];
-                d4[1] = src[1];
+                plane_phase ^= 1u;
             }
-          }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty);
+            u += ze - zs;
         }
     }
 
     // wind down: every role has left its loop (all waits are bounded)
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && abort_flag) {
-        // after an abort, wait (bounded) for the TMA loads still in flight
+    if (threadIdx.x == 0) {
+        // loads still in flight after an abort: at most the last ones into each buffer (bounded waits; a load
+        // that was waited for already passes at once)
         volatile int never = 0;
-        for (unsigned long long q = consumed_sh; q < issued_sh; ++q)
-            mbar_wait(&full_bar[q % P.stages], (uint32_t)((q / P.stages) & 1u), &never, P.status, 5);
-    }
-    if (threadIdx.x == 32) {
-        // every MMA this thread issued has completed before TMEM is released
-        volatile int never = 0;
-        tc_commit(&drain_bar);
-        mbar_wait(&drain_bar, 0, &never, P.status, 6);
+        if (abort_flag) {
+            for (unsigned long long q = issued_sh > P.stages ? issued_sh - P.stages : 0; q < issued_sh; ++q)
+                mbar_wait(&full_bar[q % P.stages], (uint32_t)((q / P.stages) & 1u), &never, P.status, 5);
+            const unsigned long long nb = P.resident ? 1 : P.chunks;
+            for (unsigned long long q = b_issued_sh > nb ? b_issued_sh - nb : 0; q < b_issued_sh; ++q)
+                mbar_wait(&b_full[q % nb], (uint32_t)((q / nb) & 1u), &never, P.status, 5);
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -319,139 +535,190 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 using kvtma::encoder;
 
-inline CUtensorMapSwizzle swizzle_for(int row_bytes) {
-    return row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                            : (row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-}
-
-// Activation map: [D][H][W][C] BF16, box {kseg, BW, BH, BD}.
-inline bool encode_act(CUtensorMap *m, const void *ptr, int C, int D, int H, int W, int kseg, int BW, int BH,
-                       int BD) {
+// Activation map: [D][H][W][C] BF16, box {16, bx, by, 1}.
+inline bool encode_act(CUtensorMap *m, const void *ptr, int C, int D, int H, int W, int bx, int by) {
     cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D};
     cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    cuuint32_t box[4] = {(cuuint32_t)kseg, (cuuint32_t)BW, (cuuint32_t)BH, (cuuint32_t)BD};
+    cuuint32_t box[4] = {(cuuint32_t)kSeg, (cuuint32_t)bx, (cuuint32_t)by, 1};
     cuuint32_t es[4] = {1, 1, 1, 1};
     return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(ptr), dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(kseg * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Weight map: [N][27][K] BF16, box {kseg, 1, N}.
-inline bool encode_w(CUtensorMap *m, const void *ptr, int N, int K, int kseg) {
-    cuuint64_t dims[3] = {(cuuint64_t)K, 27, (cuuint64_t)N};
-    cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)27 * K * 2};
-    cuuint32_t box[3] = {(cuuint32_t)kseg, 1, (cuuint32_t)N};
-    cuuint32_t es[3] = {1, 1, 1};
-    return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(kseg * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+// Weight map: [N][27][K] BF16 seen as (K, N, 3 dz, 9 (dy, dx)), box {16, cg, dz, taps}.
+inline bool encode_w(CUtensorMap *m, const void *ptr, int N, int K, int cg, int dz, int taps) {
+    cuuint64_t dims[4] = {(cuuint64_t)K, (cuuint64_t)N, 3, 9};
+    cuuint64_t strides[3] = {(cuuint64_t)27 * K * 2, (cuuint64_t)9 * K * 2, (cuuint64_t)K * 2};
+    cuuint32_t box[4] = {(cuuint32_t)kSeg, (cuuint32_t)cg, (cuuint32_t)dz, (cuuint32_t)taps};
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    return encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(ptr), dims, strides, box, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 inline uint32_t align1k(uint32_t x) { return (x + 1023u) & ~1023u; }
 
-// The tile of M = 128*T voxels of a D x H x W volume: BW = min(W, 128),
-// BH = min(H, M / BW), BD = the rest (at most 256, the TMA box limit); false
-// when the volume is not a whole number of such tiles (the dimensions must
-// be powers of two below the tile extents or multiples of them).
-inline bool tile_shape(int D, int H, int W, int &BW, int &BH, int &BD, int T = 1) {
-    const int M = kTileM * T;
-    BW = W < kTileM ? W : kTileM;
-    if (BW <= 0 || M % BW != 0 || W % BW != 0) return false;
-    BH = H < M / BW ? H : M / BW;
-    if (BH <= 0 || (M / BW) % BH != 0 || H % BH != 0 || BH > 256) return false;
-    BD = M / (BW * BH);
-    return BD <= 256 && D % BD == 0;
+// Whether a D x H x W volume is a whole number of 128-voxel boxes (BW =
+// min(W, 128), BH = min(H, 128 / BW), the rest in z): what the tensor-core
+// entry of the single-layer convolution accepts.
+inline bool tile_shape(int D, int H, int W) {
+    const int BW = W < kTileM ? W : kTileM;
+    if (BW <= 0 || kTileM % BW != 0 || W % BW != 0) return false;
+    const int BH = H < kTileM / BW ? H : kTileM / BW;
+    if (BH <= 0 || (kTileM / BW) % BH != 0 || H % BH != 0) return false;
+    return D % (kTileM / (BW * BH)) == 0;
 }
 
-// out[v][N] = conv3(in1 (c1 channels) ++ in2 (c2 channels), w [N][27][c1+c2]) + bias, ReLU optional.
+// The largest group of output channels, a multiple of 16 up to 64 that divides N.
+inline int channel_group(int N) {
+    for (int g = 64; g > 16; g -= 16)
+        if (N % g == 0) return g;
+    return 16;
+}
+
+// Shape of one launch: column extent, sub-tiles, plane buffers and weights in
+// shared memory, chosen by the estimated time of the busiest CTA.  An MMA of n
+// dz groups takes max(shared-memory reads of A and B at 128 B a cycle, n * CG /
+// 2 cycles of arithmetic), measured 46 cycles at CG = 16, n = 3; loads come at
+// about 32 B a cycle and SM out of L2; waits, commits and address set-up cost
+// about 300 cycles a sub-tile (resident weights) or a piece of weights, shared
+// by two issuers; draining a sub-tile takes about 300 + 10 CG cycles a set of
+// warps.  A single plane buffer exposes its load.
+inline bool plan_shape(Params &P, int CG, int sm_count, int *grid, size_t *smem) {
+    const uint32_t budget = 224u * 1024u;
+    const int max_t = std::min(kMaxT, 512 / (3 * CG));
+    const int parts = sm_count / P.ncg > 0 ? sm_count / P.ncg : 1;
+    auto mma = [&](int n) {
+        const double rd = (kTileM * kRow + n * CG * kRow) / 128.0, ar = n * CG / 2.0;
+        return rd > ar ? rd : ar;
+    };
+    const double whole = mma(3), split = (mma(3) + 2 * (mma(2) + mma(1))) / 3;
+    double best = 1e300;
+    for (int wide = 0; wide < 6; ++wide) {
+        // one y row per sub-tile (wide == 0), or consecutive rows of a narrower column
+        const int BW = wide == 0 ? kTileM : (wide == 1 ? P.W : 256 >> wide);   // W, 64, 32, 16, 8
+        if (wide == 0 ? P.W < kTileM : (wide == 1 ? P.W > 254 : BW >= P.W)) continue;
+        const int pitch = BW + 2;
+        for (int T = 1; T <= max_t; ++T) {
+            if (wide != 0 && T * kTileM < BW) continue;
+            int BY = wide == 0 ? T : (T * kTileM - BW) / pitch + 1;
+            if (BY > 254) continue;
+            if (BY > P.H) {
+                if (wide == 0 || (P.H - 1) * pitch + BW <= (T - 1) * kTileM) continue;   // fewer sub-tiles do
+                BY = P.H;
+            }
+            const int mstep = wide == 0 ? pitch : kTileM;
+            const int tx = (P.W + BW - 1) / BW, ty = (P.H + BY - 1) / BY;
+            const long long units = (long long)tx * ty * P.D;
+            const uint32_t rows = (uint32_t)std::max((BY + 2) * pitch, (T - 1) * mstep + kTileM + 2 * pitch + 2);
+            const uint32_t a_bytes = align1k(rows * kRow), plane_bytes = a_bytes * (uint32_t)P.nseg;
+            for (int mode = 0; mode < 3; ++mode) {   // resident x 5 groups, resident x 3, streamed x 3
+                if (mode < 2 && P.nseg > kChunkSegs) continue;
+                const int groups = mode == 0 ? 5 : 3;
+                const uint32_t b_seg = (uint32_t)((mode < 2 ? 9 : 1) * groups * CG * kRow);
+                const uint32_t piece = b_seg * (uint32_t)kChunkSegs;
+                for (uint32_t bufs = 1; bufs <= (mode < 2 ? 4u : 2u); ++bufs) {
+                    uint32_t chunks = 0, b_bytes;
+                    if (mode < 2) {
+                        b_bytes = align1k(b_seg * (uint32_t)P.nseg);
+                    } else {
+                        if (bufs * plane_bytes + 2 * piece > budget) continue;
+                        chunks = std::min<uint32_t>(kMaxChunks, (budget - bufs * plane_bytes) / piece);
+                        b_bytes = align1k(chunks * piece);
+                    }
+                    if (bufs * plane_bytes + b_bytes > budget) continue;
+                    const int tiles = (T + kIssuers - 1) / kIssuers;   // of one issuer
+                    const int pieces = mode < 2 ? tiles : 9 * ((P.nseg + kChunkSegs - 1) / kChunkSegs);
+                    const double compute = 9.0 * T * P.nseg * (mode == 0 ? whole : split) + 150.0 * pieces;
+                    const double load_a = (double)P.nseg * (BY + 2) * pitch * kRow / 32.0;
+                    const double load_b = mode < 2 ? 0.0 : 27.0 * P.nseg * CG * kRow / 32.0;
+                    const double drain = (T + kEpilogueSets - 1) / kEpilogueSets * (300.0 + 10.0 * CG);
+                    double plane = bufs == 1 ? std::max(compute, load_b) + load_a + 1500.0
+                                             : std::max(compute, load_a + load_b) + (bufs == 2 ? 200.0 : 0.0);
+                    plane = std::max(plane, drain) + (mode == 2 || T <= 2 ? drain : 0.0);
+                    const long long per = (units + parts - 1) / parts;
+                    const double cols = 1.0 + (double)per / P.D;
+                    const double total = plane * (per + 0.8 * 2 * cols) + (mode < 2 ? b_bytes / 32.0 : 0.0);
+                    if (total >= best) continue;
+                    best = total;
+                    P.BW = BW;
+                    P.BY = BY;
+                    P.pitch = pitch;
+                    P.T = T;
+                    P.mstep = mstep;
+                    P.pitch_magic = ((1u << 20) + pitch - 1) / pitch;
+                    P.tiles_x = tx;
+                    P.units = units;
+                    P.groups = groups;
+                    P.resident = mode < 2;
+                    P.stages = bufs;
+                    P.a_bytes = a_bytes;
+                    P.a_tx = (uint32_t)((BY + 2) * pitch * kRow);
+                    P.b_off = bufs * plane_bytes;
+                    P.b_seg_bytes = b_seg;
+                    P.chunks = chunks;
+                    *grid = (int)std::min<long long>(parts, units) * P.ncg;
+                    *smem = (size_t)bufs * plane_bytes + b_bytes + 1024;
+                }
+            }
+        }
+    }
+    return best < 1e300;
+}
+
+// out[v][N] = conv3(in1 (c1 channels) ++ in2 (c2 channels), w [N][27][c1+c2]) + bias, ReLU optional, zero where
+// `mask` (a tensor like out; nullptr: none) is not positive.
 // Returns a message on a configuration this kernel does not cover (nullptr: launched).
 inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 *in2, int c2,
-                          const __nv_bfloat16 *w, const float *bias, bool relu, __nv_bfloat16 *out, int N, int D,
-                          int H, int W, int *status, int sm_count, cudaStream_t stream) {
+                          const __nv_bfloat16 *w, const float *bias, bool relu, const __nv_bfloat16 *mask,
+                          __nv_bfloat16 *out, int N, int D, int H, int W, int *status, int sm_count,
+                          cudaStream_t stream) {
     if (encoder() == nullptr) return "cuTensorMapEncodeTiled is not available";
     const int K = c1 + c2;
     auto ok_c = [](int c) { return c == 16 || c == 32 || c == 64 || c == 128; };
     if (!ok_c(c1) || (c2 != 0 && !ok_c(c2))) return "input channels must be 16, 32, 64 or 128";
     if (N % 16 != 0 || N < 16 || N > 256) return "output channels must be a multiple of 16 up to 256";
-    int kseg = c1 < 64 ? c1 : 64;
-    if (c2 != 0 && c2 < kseg) kseg = c2;
-    // sub-tiles per tile: as many as keep T*N <= 128 TMEM columns and a stage
-    // within 64 KB (narrow layers need several MMAs per stage to keep the
-    // tensor pipe busy between TMA round trips)
-    int T = 1;
-    for (int t = 4; t > 1; t /= 2) {
-        int bw, bh, bd;
-        if (t * N <= 128 && (kTileM * t + N) * K * 2 <= 64 * 1024 && tile_shape(D, H, W, bw, bh, bd, t)) {
-            T = t;
-            break;
-        }
-    }
-    int BW, BH, BD;
-    if (!tile_shape(D, H, W, BW, BH, BD, T)) return "volume is not a whole number of 128-voxel tiles";
+    if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(mask)) % 16 != 0)
+        return "output or mask is not 16-byte aligned";
+    const int CG = channel_group(N);
     Params P{};
-    P.seg.n = 0;
-    for (int src = 0; src < 2; ++src) {
-        const int C = src == 0 ? c1 : c2;
-        for (int c0 = 0; c0 < C; c0 += kseg) {
-            if (P.seg.n == kMaxSeg) return "too many input channel segments";
-            const int s = P.seg.n++;
-            P.seg.kseg[s] = kseg;
-            P.seg.src[s] = src;
-            P.seg.c0[s] = c0;
-            P.seg.kglob[s] = (src == 0 ? 0 : c1) + c0;
-        }
-    }
-    uint32_t off = 0;
-    for (int s = 0; s < P.seg.n; ++s) {
-        P.seg.a_off[s] = off;
-        off = align1k(off + (uint32_t)kTileM * T * kseg * 2);
-    }
-    for (int s = 0; s < P.seg.n; ++s) {
-        P.seg.b_off[s] = off;
-        off = align1k(off + (uint32_t)N * kseg * 2);
-    }
-    P.stage_bytes = off;
-    P.tx_bytes = (uint32_t)(kTileM * T + N) * K * 2;
-    const uint32_t budget = 200u * 1024u;
-    P.stages = budget / P.stage_bytes;
-    if (P.stages > 8) P.stages = 8;
-    if (P.stages < 2) return "stage does not fit in shared memory";
-    P.tmem_cols = 32;
-    while (P.tmem_cols < (uint32_t)(N * T)) P.tmem_cols <<= 1;
-    P.T = T;
+    P.nseg = K / kSeg;
+    P.nseg1 = c1 / kSeg;
     P.N = N;
+    P.ncg = N / CG;
     P.D = D;
     P.H = H;
     P.W = W;
-    P.BW = BW;
-    P.BH = BH;
-    P.BD = BD;
-    P.tiles = (long long)(D / BD) * (H / BH) * (W / BW);
-    // kind::f16 instruction descriptor: FP32 accumulator (bits 4-5 = 1), BF16 A
-    // and B (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bits 17-22, M >> 4 at 24-28
-    P.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+    int grid = 0;
+    size_t smem = 0;
+    if (!plan_shape(P, CG, sm_count, &grid, &smem)) return "no tile shape for this volume";
+    P.tmem_cols = 32;
+    while (P.tmem_cols < (uint32_t)(3 * CG * P.T)) P.tmem_cols <<= 1;
     P.bias = bias;
     P.relu = relu ? 1 : 0;
+    P.mask = mask;
     P.out = out;
     P.status = status;
-    CUtensorMap ma0, ma1, mb;
-    if (!encode_act(&ma0, in1, c1, D, H, W, kseg, BW, BH, BD)) return "activation tensor map rejected";
-    if (!encode_act(&ma1, c2 ? in2 : in1, c2 ? c2 : c1, D, H, W, kseg, BW, BH, BD))
+    CUtensorMap ma0, ma1, mb, mb2;
+    if (!encode_act(&ma0, in1, c1, D, H, W, P.pitch, P.BY + 2)) return "activation tensor map rejected";
+    if (!encode_act(&ma1, c2 ? in2 : in1, c2 ? c2 : c1, D, H, W, P.pitch, P.BY + 2))
         return "activation tensor map rejected";
-    if (!encode_w(&mb, w, N, K, kseg)) return "weight tensor map rejected";
-    const size_t smem = (size_t)P.stages * P.stage_bytes + 1024;
-    if (cudaFuncSetAttribute(conv3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return "shared memory request rejected";
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, conv3_tc_kernel, kThreads, smem) != cudaSuccess ||
-        per_sm < 1)
-        return "occupancy query failed";
-    if ((uint32_t)per_sm * P.tmem_cols > 512u) per_sm = (int)(512u / P.tmem_cols);
-    long long grid = (long long)sm_count * per_sm;
-    if (grid > P.tiles) grid = P.tiles;
-    conv3_tc_kernel<<<(unsigned)grid, kThreads, smem, stream>>>(ma0, ma1, mb, P);
-    return nullptr;
+    const bool per_tap = P.resident && P.groups == 5;   // dz = 0 1 2 and dz = 0 1 of one (dy, dx) per load
+    if (!encode_w(&mb, w, N, K, CG, 3, per_tap || !P.resident ? 1 : 9) || !encode_w(&mb2, w, N, K, CG, 2, 1))
+        return "weight tensor map rejected";
+    auto go = [&](auto kernel) -> const char * {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            return "shared memory request rejected";
+        kernel<<<(unsigned)grid, kThreads, smem, stream>>>(ma0, ma1, mb, mb2, P);
+        return nullptr;
+    };
+    switch (CG) {
+    case 16: return go(conv3_march_kernel<16>);
+    case 32: return go(conv3_march_kernel<32>);
+    case 48: return go(conv3_march_kernel<48>);
+    default: return go(conv3_march_kernel<64>);
+    }
 }
 
 }  // namespace convtc

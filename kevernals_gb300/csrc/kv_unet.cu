@@ -399,47 +399,23 @@ kv_status ensure_workspace(kv_unet *u, int D, int H, int W, bool grads) {
     return KV_OK;
 }
 
-// forward convolution over all output channels (chunks of <= 64)
+// forward or backward-data convolution of one layer
 kv_status conv3(kv_unet *u, int layer, const bf16 *in1, const bf16 *in2, bf16 *out, int lvl, bool weights_t,
                 int c_in_override = -1) {
     const kv_unet::Conv &L = u->conv[layer];
     kv_ctx *ctx = u->ctx;
     const int D = u->D >> lvl, H = u->H >> lvl, W = u->W >> lvl;
-    const long long nvox = (long long)D * H * W;
     // forward: in1 (c1) ++ in2 (c2) -> cout with W; backward-data: in1 = dPre (cout) -> c1 + c2 with Wt
     const int c1 = weights_t ? L.cout : L.c1, c2 = weights_t ? 0 : L.c2;
     const int cout = weights_t ? (c_in_override > 0 ? c_in_override : L.c1 + L.c2) : L.cout;
     const bf16 *w = weights_t ? u->wt + L.w : u->pb + L.w;
     const float *bias = weights_t ? nullptr : u->p + L.b;
-    const int blocks = (int)((nvox / 16 + 3) / 4);
     LaunchTimer lt(ctx, weights_t ? "unet_conv_dgrad" : "unet_conv_fwd");
-    int bw, bh, bd;
-    if (convtc::tile_shape(D, H, W, bw, bh, bd)) {
-        // tcgen05 / TMA implicit GEMM (kv_conv_tc.cuh)
-        const char *why = convtc::launch(in1, c1, in2, c2, w, bias, !weights_t, out, cout, D, H, W, u->tc_status,
-                                         ctx->sm_count, ctx->stream);
-        if (why != nullptr) return kv_fail(ctx, KV_ERR_UNSUPPORTED, "tensor-core convolution: %s", why);
-        KV_CHECK_LAUNCH(ctx, "unet conv3 (tcgen05)");
-        return KV_OK;
-    }
-    // volumes that are not a whole number of 128-voxel tiles (the deepest
-    // levels of small inputs): warp-level mma.sync
-    for (int n0 = 0; n0 < cout; n0 += 64) {
-        const int nc = cout - n0 < 64 ? cout - n0 : 64;
-        const bool relu = !weights_t;
-        switch (nc) {
-        case 16: relu ? unet::conv3_fwd<2, true><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W)
-                      : unet::conv3_fwd<2, false><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W); break;
-        case 32: relu ? unet::conv3_fwd<4, true><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W)
-                      : unet::conv3_fwd<4, false><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W); break;
-        case 48: relu ? unet::conv3_fwd<6, true><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W)
-                      : unet::conv3_fwd<6, false><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W); break;
-        case 64: relu ? unet::conv3_fwd<8, true><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W)
-                      : unet::conv3_fwd<8, false><<<blocks, 128, 0, ctx->stream>>>(in1, c1, in2, c2, w, bias, out, cout, n0, D, H, W); break;
-        default: return kv_fail(ctx, KV_ERR_UNSUPPORTED, "conv chunk of %d channels", nc);
-        }
-    }
-    KV_CHECK_LAUNCH(ctx, "unet conv3");
+    // tcgen05 / TMA implicit GEMM (kv_conv_tc.cuh); covers every level of every volume the network takes
+    const char *why = convtc::launch(in1, c1, in2, c2, w, bias, !weights_t, nullptr, out, cout, D, H, W, u->tc_status,
+                                     ctx->sm_count, ctx->stream);
+    if (why != nullptr) return kv_fail(ctx, KV_ERR_UNSUPPORTED, "tensor-core convolution: %s", why);
+    KV_CHECK_LAUNCH(ctx, "unet conv3 (tcgen05)");
     return KV_OK;
 }
 
@@ -825,8 +801,8 @@ extern "C" kv_status kv_unet_set_state(kv_unet *u, const float *state, int64_t s
 // One 3x3x3 convolution of the network's kind on caller buffers (device
 // pointers, BF16 bit patterns): the operator behind every U-Net layer, for
 // callers and tests that need a single layer.  kernel: 0 = the tensor-core
-// (tcgen05 / TMA) kernel where the volume tiles, else mma.sync; 1 = tcgen05
-// only; 2 = mma.sync only.
+// (tcgen05 / TMA) kernel where it covers the call, else mma.sync; 1 = tcgen05
+// only, for volumes of whole 128-voxel tiles; 2 = mma.sync only.
 extern "C" kv_status kv_conv3_bf16(kv_ctx *ctx, const uint16_t *in1, int32_t c1, const uint16_t *in2, int32_t c2,
                                    const uint16_t *w, const float *bias, int32_t relu, uint16_t *out, int32_t cout,
                                    int32_t D, int32_t H, int32_t W, int32_t kernel) {
@@ -839,16 +815,19 @@ extern "C" kv_status kv_conv3_bf16(kv_ctx *ctx, const uint16_t *in1, int32_t c1,
     const bf16 *a = reinterpret_cast<const bf16 *>(in1), *b = reinterpret_cast<const bf16 *>(in2);
     const bf16 *wb = reinterpret_cast<const bf16 *>(w);
     bf16 *o = reinterpret_cast<bf16 *>(out);
-    int bw, bh, bd;
-    const bool tiles = convtc::tile_shape(D, H, W, bw, bh, bd);
+    const bool tiles = convtc::tile_shape(D, H, W);
     if (kernel == 1 && !tiles)
         return kv_fail(ctx, KV_ERR_UNSUPPORTED, "kv_conv3_bf16: the volume is not a whole number of 128-voxel tiles");
-    if (kernel != 2 && tiles) {
-        const char *why = convtc::launch(a, c1, c2 ? b : nullptr, c2, wb, bias, relu != 0, o, cout, D, H, W,
+    // volumes that are not whole tiles take the tensor-core kernel too where it covers the call, else mma.sync; the
+    // two sum in the same order, with equal bits
+    if (kernel != 2) {
+        const char *why = convtc::launch(a, c1, c2 ? b : nullptr, c2, wb, bias, relu != 0, nullptr, o, cout, D, H, W,
                                          ctx->d_status, ctx->sm_count, ctx->stream);
-        if (why != nullptr) return kv_fail(ctx, KV_ERR_UNSUPPORTED, "tensor-core convolution: %s", why);
-        KV_CHECK_LAUNCH(ctx, "kv_conv3_bf16 (tcgen05)");
-        return KV_OK;
+        if (why == nullptr) {
+            KV_CHECK_LAUNCH(ctx, "kv_conv3_bf16 (tcgen05)");
+            return KV_OK;
+        }
+        if (tiles) return kv_fail(ctx, KV_ERR_UNSUPPORTED, "tensor-core convolution: %s", why);
     }
     if (W % 16 != 0 || c1 % 16 != 0 || c2 % 16 != 0 || cout % 16 != 0)
         return kv_fail(ctx, KV_ERR_UNSUPPORTED, "kv_conv3_bf16: mma.sync needs W, channels multiples of 16");

@@ -97,3 +97,28 @@ def test_conv_layer_tcgen05_vs_mma_sync_and_fp64(ctx, shape):
     _, rne = _bf16_bits(ref.astype(np.float32))
     assert np.mean(got == rne) > 0.99
     assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 4e-3
+
+
+# column shapes of the z-marching kernel: rows left over in y, one plane, a
+# share that starts inside a column, several rows of a narrow volume per
+# sub-tile (128, 64, 48, 32 and 16 voxels wide, and 192), weights that stay in
+# shared memory and weights that stream, channel groups of 16, 32, 48 and 64
+COLUMNS = [
+    (1, 1, 128, 16, 0, 16), (3, 11, 128, 16, 0, 16), (37, 23, 128, 32, 16, 16), (5, 3, 256, 16, 0, 48),
+    (7, 14, 64, 64, 32, 32), (3, 6, 64, 32, 0, 96), (2, 20, 32, 128, 64, 64), (4, 24, 16, 128, 0, 128),
+    (2, 5, 192, 32, 0, 32), (3, 7, 48, 64, 0, 64), (1, 2, 16, 64, 0, 192), (9, 1, 384, 16, 128, 80),
+]
+
+
+@pytest.mark.parametrize("shape", COLUMNS, ids=["x".join(map(str, s[:3])) + f"_{s[3]}+{s[4]}to{s[5]}" for s in COLUMNS])
+def test_conv_columns_equal_mma_sync(ctx, shape):
+    """The default route against the mma.sync kernel: the same sums in the same order, equal bits."""
+    pytest.importorskip("torch")
+    D, H, W, c1, c2, cout = shape
+    rng = np.random.default_rng(sum(shape))
+    a, _ = _bf16_bits(rng.standard_normal((D, H, W, c1)).astype(np.float32))
+    b, _ = _bf16_bits(rng.standard_normal((D, H, W, max(c2, 1))).astype(np.float32))
+    w, _ = _bf16_bits((rng.standard_normal((cout, 27, c1 + c2)) / np.sqrt(27 * (c1 + c2))).astype(np.float32))
+    bias = (rng.standard_normal(cout) * 0.1).astype(np.float32)
+    got = _conv(ctx, a, c1, b, c2, w, bias, True, cout, (D, H, W), 0)
+    assert np.array_equal(got, _conv(ctx, a, c1, b, c2, w, bias, True, cout, (D, H, W), 2))
