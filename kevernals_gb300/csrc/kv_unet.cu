@@ -19,6 +19,7 @@
 #include "kv_conv_tc.cuh"
 #include "kv_internal.h"
 #include "kv_unet_kernels.cuh"
+#include "kv_wgrad_tc.cuh"
 
 #include <cmath>
 #include <cstring>
@@ -424,18 +425,11 @@ kv_status wgrad(kv_unet *u, int layer, const bf16 *dpre, const bf16 *in1, const 
     kv_ctx *ctx = u->ctx;
     const int D = u->D >> lvl, H = u->H >> lvl, W = u->W >> lvl;
     const long long nvox = (long long)D * H * W;
-    const int cin = L.c1 + L.c2;
-    const int ntw = cin % 64 == 0 ? 8 : (cin % 32 == 0 ? 4 : 2);
-    const int groups = cin / (8 * ntw);
-    long long chunk = 16384;
-    while (chunk > 1024 && (nvox + chunk - 1) / chunk < ctx->sm_count / 4) chunk /= 2;
-    dim3 grid((unsigned)((nvox + chunk - 1) / chunk), 27, (L.cout / 16) * groups);
-    float *dw = u->g + L.w;
-    LaunchTimer lt(ctx, "unet_conv_wgrad");
-    switch (ntw) {
-    case 8: unet::conv3_wgrad<8><<<grid, 128, 0, ctx->stream>>>(dpre, L.cout, in1, L.c1, in2, L.c2, dw, D, H, W, (int)chunk); break;
-    case 4: unet::conv3_wgrad<4><<<grid, 128, 0, ctx->stream>>>(dpre, L.cout, in1, L.c1, in2, L.c2, dw, D, H, W, (int)chunk); break;
-    default: unet::conv3_wgrad<2><<<grid, 128, 0, ctx->stream>>>(dpre, L.cout, in1, L.c1, in2, L.c2, dw, D, H, W, (int)chunk); break;
+    {
+        LaunchTimer lt(ctx, "unet_conv_wgrad");
+        const char *why = wgradtc::launch(dpre, L.cout, in1, L.c1, in2, L.c2, u->g + L.w, D, H, W, u->tc_status,
+                                          ctx->sm_count, ctx->stream);
+        if (why != nullptr) return kv_fail(ctx, KV_ERR_UNSUPPORTED, "weight gradient: %s", why);
     }
     {
         LaunchTimer lb(ctx, "unet_bias_grad");

@@ -95,3 +95,24 @@ def test_training_reduces_loss_and_checkpoint_roundtrip(ctx, tmp_path):
     l_a = net.train_step(x, t, lr=1e-3)
     l_b = other.train_step(x, t, lr=1e-3)
     assert l_a == l_b
+
+
+# rows left over in a column, columns of 96 and 48 voxels, a single plane at the deepest level, shares of one plane.
+# The bounds are those of test_gradients_match_fp64_reference: the BF16 roundings along the chain of layers set them,
+# whatever the size.
+@pytest.mark.parametrize("shape", [(8, 8, 128), (8, 24, 384), (24, 40, 128)])
+def test_gradients_over_column_shapes(ctx, shape):
+    net = engine.UNet(ctx, seed=3)
+    params = perturbed(net, 3)
+    x = smooth_input(shape, 1)
+    t = x * 0.7 + 0.05
+    loss, g = net.gradients(x, t)
+    p = torch.tensor(params, dtype=torch.float64, requires_grad=True)
+    lr = ((ref.forward(torch.from_numpy(x).double(), ref.unpack(p)) - torch.from_numpy(t).double()) ** 2).mean()
+    lr.backward()
+    gr = p.grad.numpy()
+    assert loss == pytest.approx(lr.item(), rel=1e-2)
+    for cin, co, w, b in ref.layout()["convs"]:
+        o = slice(w, w + co * 27 * cin)
+        assert np.linalg.norm(g[o] - gr[o]) < 8e-2 * np.linalg.norm(gr[o])
+    assert np.dot(g, gr) / (np.linalg.norm(g) * np.linalg.norm(gr)) > 0.998
