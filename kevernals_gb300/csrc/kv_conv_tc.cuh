@@ -36,9 +36,9 @@
 //
 // Measured on a GB300, against a kernel that loaded one tile per tap and
 // issued one N = Cout MMA per tap and 16 channels: 32+16 -> 16 channels at
-// 128 x 256 x 128 voxels 1434 -> 230 us (755 TFLOP/s); the thirteen layers of
-// the U-Net at 128 x 512 x 512 voxels 31.9 -> 6.0 ms, forward and
-// backward-data at 128 x 256 x 128 8.1 -> 2.1 ms.
+// 128 x 256 x 128 voxels 1434 -> 176 us (990 TFLOP/s); the thirteen layers of
+// the U-Net at 128 x 512 x 512 voxels 31.9 -> 5.4 ms, forward and
+// backward-data at 128 x 256 x 128 8.1 -> 1.9 ms.
 //
 // Warp roles (352 threads): warp 0 issues the TMA loads of the planes and of
 // streamed weights, warps 1 and 10 issue the MMAs of the even and
@@ -76,6 +76,12 @@ constexpr int kMaxChunks = 8;     // ring of streamed weights
 constexpr int kChunkSegs = 4;     // segments in one piece of streamed weights
 constexpr uint32_t kWaitLimit = 1u << 22;   // try_wait rounds before a wait is declared failed
 
+// Output layer of the network on the 16 channels h (rounded to BF16) of a voxel: y = x + (b + sum w h).
+struct Head {
+    const float *w, *b, *x;
+    float *y;
+};
+
 struct Params {
     int nseg, nseg1;              // input segments; the first nseg1 come from the first tensor
     int N, ncg;                   // output channels; groups of CG channels, one per CTA
@@ -96,7 +102,8 @@ struct Params {
     const float *bias;            // nullptr: none
     int relu;
     const __nv_bfloat16 *mask;    // nullptr: none; else outputs where mask <= 0 become 0
-    __nv_bfloat16 *out;           // [voxels][N]
+    __nv_bfloat16 *out;           // [voxels][N]; nullptr: not stored
+    Head head;                    // y == nullptr: none (N = 16 only)
     int *status;                  // 0 ok; set on a failed wait
 };
 
@@ -187,22 +194,27 @@ __device__ __forceinline__ void issue_taps(uint32_t t0, uint32_t t1, uint32_t a,
                                            uint32_t id0, uint32_t id1, int n1, uint32_t y_step, uint32_t tap_step,
                                            uint32_t a_seg, uint32_t b_seg) {
     if (elect_one()) {
-        if (n1 == 0) {
+        // unrolled over dx and the segments only: all 36 addresses at once spilled (230 us on the layer above, now 176)
+#pragma unroll 1
+        for (int dy = 0; dy < (NT + 2) / 3; ++dy) {
+            if (n1 == 0) {
 #pragma unroll
-            for (int tap = 0; tap < NT; ++tap)
+                for (int dx = 0; dx < (NT < 3 ? NT : 3); ++dx)
 #pragma unroll
-                for (int s = 0; s < NS; ++s)
-                    tc_mma(t0, a + (tap / 3) * y_step + (tap % 3) * (kRow >> 4) + s * a_seg,
-                           b0 + tap * tap_step + s * b_seg, hi, id0);
-        } else {
+                    for (int s = 0; s < NS; ++s)
+                        tc_mma(t0, a + dx * (kRow >> 4) + s * a_seg, b0 + dx * tap_step + s * b_seg, hi, id0);
+            } else {
 #pragma unroll
-            for (int tap = 0; tap < NT; ++tap)
+                for (int dx = 0; dx < (NT < 3 ? NT : 3); ++dx)
 #pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    const uint32_t as = a + (tap / 3) * y_step + (tap % 3) * (kRow >> 4) + s * a_seg;
-                    tc_mma(t0, as, b0 + tap * tap_step + s * b_seg, hi, id0);
-                    tc_mma(t1, as, b1 + tap * tap_step + s * b_seg, hi, id1);
-                }
+                    for (int s = 0; s < NS; ++s) {
+                        tc_mma(t0, a + dx * (kRow >> 4) + s * a_seg, b0 + dx * tap_step + s * b_seg, hi, id0);
+                        tc_mma(t1, a + dx * (kRow >> 4) + s * a_seg, b1 + dx * tap_step + s * b_seg, hi, id1);
+                    }
+            }
+            a += y_step;
+            b0 += 3 * tap_step;
+            b1 += 3 * tap_step;
         }
     }
     __syncwarp();
@@ -488,9 +500,22 @@ __global__ void __launch_bounds__(kThreads, 1)
                                     }
                                     r[j] = __floats2bfloat162_rn(a, b);
                                 }
-                                uint4 *d4 = reinterpret_cast<uint4 *>(P.out + o + 16 * q);
-                                d4[0] = reinterpret_cast<const uint4 *>(r)[0];
-                                d4[1] = reinterpret_cast<const uint4 *>(r)[1];
+                                if (P.out != nullptr) {
+                                    uint4 *d4 = reinterpret_cast<uint4 *>(P.out + o + 16 * q);
+                                    d4[0] = reinterpret_cast<const uint4 *>(r)[0];
+                                    d4[1] = reinterpret_cast<const uint4 *>(r)[1];
+                                }
+                                if (CG == 16 && P.head.y != nullptr) {
+                                    float h = __ldg(P.head.b);
+#pragma unroll
+                                    for (int j = 0; j < 8; ++j) {
+                                        const float2 f = __bfloat1622float2(r[j]);
+                                        h = fmaf(__ldg(P.head.w + 2 * j), f.x, h);
+                                        h = fmaf(__ldg(P.head.w + 2 * j + 1), f.y, h);
+                                    }
+                                    const size_t vox = o / 16;
+                                    P.head.y[vox] = __ldg(P.head.x + vox) + h;
+                                }
                             }
                         }
                         __syncwarp();
@@ -668,11 +693,11 @@ inline bool plan_shape(Params &P, int CG, int sm_count, int *grid, size_t *smem)
 }
 
 // out[v][N] = conv3(in1 (c1 channels) ++ in2 (c2 channels), w [N][27][c1+c2]) + bias, ReLU optional, zero where
-// `mask` (a tensor like out; nullptr: none) is not positive.
+// `mask` (a tensor like out; nullptr: none) is not positive; out may be nullptr where `head` takes the result.
 // Returns a message on a configuration this kernel does not cover (nullptr: launched).
 inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 *in2, int c2,
                           const __nv_bfloat16 *w, const float *bias, bool relu, const __nv_bfloat16 *mask,
-                          __nv_bfloat16 *out, int N, int D, int H, int W, int *status, int sm_count,
+                          const Head *head, __nv_bfloat16 *out, int N, int D, int H, int W, int *status, int sm_count,
                           cudaStream_t stream) {
     if (encoder() == nullptr) return "cuTensorMapEncodeTiled is not available";
     const int K = c1 + c2;
@@ -681,6 +706,7 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
     if (N % 16 != 0 || N < 16 || N > 256) return "output channels must be a multiple of 16 up to 256";
     if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(mask)) % 16 != 0)
         return "output or mask is not 16-byte aligned";
+    if (head != nullptr && N != 16) return "the output layer takes 16 channels";
     const int CG = channel_group(N);
     Params P{};
     P.nseg = K / kSeg;
@@ -699,6 +725,7 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
     P.relu = relu ? 1 : 0;
     P.mask = mask;
     P.out = out;
+    if (head != nullptr) P.head = *head;
     P.status = status;
     CUtensorMap ma0, ma1, mb, mb2;
     if (!encode_act(&ma0, in1, c1, D, H, W, P.pitch, P.BY + 2)) return "activation tensor map rejected";

@@ -21,6 +21,7 @@
 #include "kv_unet_kernels.cuh"
 #include "kv_wgrad_tc.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <random>
@@ -31,84 +32,192 @@ namespace {
 
 // ---------------------------------------------------------------- kernels
 
-__global__ void conv_first_fwd(const float *__restrict__ x, const float *__restrict__ w /*[16][27]*/,
-                               const float *__restrict__ b, bf16 *__restrict__ out, int D, int H, int W) {
-    const long long n = (long long)D * H * W;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const int xx = (int)(v % W);
-        const long long zy = v / W;
-        const int y = (int)(zy % H), z = (int)(zy / H);
-        float in[27];
+// Eight BF16 channels as one 16-byte access; every per-channel kernel below
+// moves them so (scalar BF16 accesses kept these passes at a third of the
+// memory rate).
+struct __align__(16) Bf8 {
+    __nv_bfloat162 v[4];
+};
+
+__device__ __forceinline__ Bf8 ld8(const bf16 *p) {
+    const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p));
+    return *reinterpret_cast<const Bf8 *>(&u);
+}
+
+__device__ __forceinline__ void st8(bf16 *p, const Bf8 &b) {
+    *reinterpret_cast<uint4 *>(p) = *reinterpret_cast<const uint4 *>(&b);
+}
+
+__device__ __forceinline__ void unpack8(const Bf8 &b, float (&f)[8]) {
 #pragma unroll
-        for (int tap = 0; tap < 27; ++tap) {
-            const int zz = z + tap / 9 - 1, yy = y + (tap / 3) % 3 - 1, x2 = xx + tap % 3 - 1;
-            const bool ok = (unsigned)zz < (unsigned)D && (unsigned)yy < (unsigned)H && (unsigned)x2 < (unsigned)W;
-            in[tap] = ok ? __ldg(x + ((long long)zz * H + yy) * W + x2) : 0.f;
+    for (int j = 0; j < 4; ++j) {
+        const float2 t = __bfloat1622float2(b.v[j]);
+        f[2 * j] = t.x;
+        f[2 * j + 1] = t.y;
+    }
+}
+
+__device__ __forceinline__ Bf8 pack8(const float (&f)[8]) {
+    Bf8 b;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b.v[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+    return b;
+}
+
+// First layer, 1 -> 16 channels in FP32.  432 multiply-adds a voxel bound it
+// (0.39 ms of FP32 issue at 128 x 512 x 512 voxels, 0.18 ms of memory), so a
+// thread computes kFirstRows voxels of consecutive y: the weights, in shared
+// memory, are read once for all of them, and their rows overlap.  One voxel a
+// thread with the weights in global memory took 2.19 ms, this takes 0.79
+// (0.94 with scalar fmaf).  Blocks of 128 x.
+constexpr int kFirstRows = 4;
+
+__global__ void __launch_bounds__(128) conv_first_fwd(const float *__restrict__ x, const float *__restrict__ w /*[16][27]*/,
+                                                      const float *__restrict__ b, bf16 *__restrict__ out, int D, int H,
+                                                      int W) {
+    __shared__ __align__(16) float ws[27][16];
+    __shared__ __align__(16) float bs[16];
+    for (int i = threadIdx.x; i < 432; i += blockDim.x) ws[i % 27][i / 27] = w[i];
+    if (threadIdx.x < 16) bs[threadIdx.x] = b[threadIdx.x];
+    __syncthreads();
+    const int xx = blockIdx.x * 128 + threadIdx.x;   // W % 128 == 0, H % 8 == 0
+    const int rows = H / kFirstRows;
+    for (long long zy = blockIdx.y; zy < (long long)D * rows; zy += gridDim.y) {
+        const int z = (int)(zy / rows), y0 = (int)(zy % rows) * kFirstRows;
+        // two channels a register pair: fma.rn.f32x2 rounds each half as fmaf does and takes one issue slot for both
+        unsigned long long acc[kFirstRows][8];
+#pragma unroll
+        for (int r = 0; r < kFirstRows; ++r)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) acc[r][c] = *reinterpret_cast<const unsigned long long *>(&bs[2 * c]);
+#pragma unroll
+        for (int dz = 0; dz < 3; ++dz) {
+            const int zz = z + dz - 1;
+            unsigned long long in[kFirstRows + 2][3];
+#pragma unroll
+            for (int r = 0; r < kFirstRows + 2; ++r)
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) {
+                    const int yy = y0 + r - 1, x2 = xx + dx - 1;
+                    const bool ok = (unsigned)zz < (unsigned)D && (unsigned)yy < (unsigned)H && (unsigned)x2 < (unsigned)W;
+                    const float f = ok ? __ldg(x + ((size_t)zz * H + yy) * W + x2) : 0.f;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(in[r][dx]) : "f"(f));
+                }
+#pragma unroll
+            for (int t = 0; t < 9; ++t) {
+                unsigned long long wv[8];
+#pragma unroll
+                for (int c = 0; c < 8; c += 2)
+                    *reinterpret_cast<ulonglong2 *>(wv + c) = *reinterpret_cast<const ulonglong2 *>(&ws[dz * 9 + t][2 * c]);
+#pragma unroll
+                for (int r = 0; r < kFirstRows; ++r)
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[r][c]) : "l"(wv[c]), "l"(in[r + t / 3][t % 3]));
+            }
         }
 #pragma unroll
-        for (int c = 0; c < 16; c += 2) {
-            float s0 = b[c], s1 = b[c + 1];
+        for (int r = 0; r < kFirstRows; ++r) {
+            bf16 *dst = out + (((size_t)z * H + y0 + r) * W + xx) * 16;
 #pragma unroll
-            for (int tap = 0; tap < 27; ++tap) {
-                s0 = fmaf(w[c * 27 + tap], in[tap], s0);
-                s1 = fmaf(w[(c + 1) * 27 + tap], in[tap], s1);
+            for (int h = 0; h < 2; ++h) {
+                float f[8];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(f[2 * c]), "=f"(f[2 * c + 1]) : "l"(acc[r][4 * h + c]));
+                    f[2 * c] = fmaxf(f[2 * c], 0.f);
+                    f[2 * c + 1] = fmaxf(f[2 * c + 1], 0.f);
+                }
+                st8(dst + 8 * h, pack8(f));
             }
-            *reinterpret_cast<__nv_bfloat162 *>(out + v * 16 + c) = __floats2bfloat162_rn(fmaxf(s0, 0.f), fmaxf(s1, 0.f));
         }
     }
 }
 
-// dW0[c][tap] += sum_v dpre[v][c] * x[v + tap]  (blockIdx.y = tap), and the
-// bias gradient when tap == 13 (the centre: every voxel contributes).
-__global__ void conv_first_wgrad(const float *__restrict__ x, const bf16 *__restrict__ dpre, float *__restrict__ dw,
-                                 float *__restrict__ db, int D, int H, int W) {
-    const int tap = blockIdx.y;
-    const long long n = (long long)D * H * W;
-    float acc[16], accb[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) acc[c] = accb[c] = 0.f;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const int xx = (int)(v % W);
-        const long long zy = v / W;
-        const int y = (int)(zy % H), z = (int)(zy / H);
-        const int zz = z + tap / 9 - 1, yy = y + (tap / 3) % 3 - 1, x2 = xx + tap % 3 - 1;
-        const bool ok = (unsigned)zz < (unsigned)D && (unsigned)yy < (unsigned)H && (unsigned)x2 < (unsigned)W;
-        const float xv = ok ? __ldg(x + ((long long)zz * H + yy) * W + x2) : 0.f;
-#pragma unroll
-        for (int c = 0; c < 16; c += 2) {
-            const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(dpre + v * 16 + c));
-            acc[c] = fmaf(g.x, xv, acc[c]);
-            acc[c + 1] = fmaf(g.y, xv, acc[c + 1]);
-            accb[c] += g.x;
-            accb[c + 1] += g.y;
-        }
+// Sums v over the block (blockDim.x threads, a multiple of 32, at most 512) and adds the total to *dst.
+__device__ __forceinline__ void block_add(float v, float *dst, float *sh /* [16] */) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.f;
+        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i];
+        atomicAdd(dst, t);
     }
+}
+
+// dW0[c][tap] += sum_v dpre[v][c] * x[v + tap], the nine taps of one dz (blockIdx.y) at once: 144 sums in registers
+// for one read of dpre (one tap a pass read it 27 times: 1.24 ms at 128 x 256 x 128 voxels).  The bias gradient comes
+// with dz = 1.
+__global__ void __launch_bounds__(256) conv_first_wgrad(const float *__restrict__ x, const bf16 *__restrict__ dpre,
+                                                        float *__restrict__ dw, float *__restrict__ db, int D, int H,
+                                                        int W) {
+    __shared__ float part[8][9][16];
+    const int dz = blockIdx.y;
+    const long long n = (long long)D * H * W;
+    float acc[9][16], accb[16];
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
-        float s = acc[c], sb = accb[c];
-        for (int o = 16; o > 0; o >>= 1) {
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-            sb += __shfl_xor_sync(0xffffffffu, sb, o);
+        accb[c] = 0.f;
+#pragma unroll
+        for (int t = 0; t < 9; ++t) acc[t][c] = 0.f;
+    }
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        const int xx = (int)(v % W);
+        const long long zy = v / W;
+        const int y = (int)(zy % H), zz = (int)(zy / H) + dz - 1;
+        float g[16], in[9];
+        float lo[8], hi[8];
+        unpack8(ld8(dpre + v * 16), lo);
+        unpack8(ld8(dpre + v * 16 + 8), hi);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            g[c] = lo[c];
+            g[8 + c] = hi[c];
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(dw + c * 27 + tap, s);
-            if (tap == 13) atomicAdd(db + c, sb);
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+            const int yy = y + t / 3 - 1, x2 = xx + t % 3 - 1;
+            const bool ok = (unsigned)zz < (unsigned)D && (unsigned)yy < (unsigned)H && (unsigned)x2 < (unsigned)W;
+            in[t] = ok ? __ldg(x + ((long long)zz * H + yy) * W + x2) : 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            if (dz == 1) accb[c] += g[c];
+#pragma unroll
+            for (int t = 0; t < 9; ++t) acc[t][c] = fmaf(g[c], in[t], acc[t][c]);
         }
     }
-}
-
-// y[v] = x[v] + b + sum_c w[c] h[v][c]
-__global__ void conv_out_fwd(const bf16 *__restrict__ h, const float *__restrict__ x, const float *__restrict__ w,
-                             const float *__restrict__ b, float *__restrict__ y, long long n) {
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        float s = b[0];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-        for (int c = 0; c < 16; c += 2) {
-            const float2 hv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(h + v * 16 + c));
-            s = fmaf(w[c], hv.x, s);
-            s = fmaf(w[c + 1], hv.y, s);
+    for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            float s = acc[t][c];
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) part[warp][t][c] = s;
         }
-        y[v] = x[v] + s;
+    __syncthreads();
+    if (threadIdx.x < 144) {
+        const int t = threadIdx.x / 16, c = threadIdx.x % 16;
+        float s = 0.f;
+        for (int i = 0; i < 8; ++i) s += part[i][t][c];
+        atomicAdd(dw + c * 27 + dz * 9 + t, s);
+    }
+    if (dz != 1) return;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        float s = accb[c];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) part[warp][0][c] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        float s = 0.f;
+        for (int i = 0; i < 8; ++i) s += part[i][0][threadIdx.x];
+        atomicAdd(db + threadIdx.x, s);
     }
 }
 
@@ -139,60 +248,74 @@ __global__ void mse_loss(const float *__restrict__ y, const float *__restrict__ 
     }
 }
 
-__global__ void sum_loss(const double *__restrict__ partials, int nb, long long n, float *__restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int i = 0; i < nb; ++i) s += partials[i];
-        out[0] = (float)(s / (double)n);
+__global__ void __launch_bounds__(256) sum_loss(const double *__restrict__ partials, int nb, long long n,
+                                                float *__restrict__ out) {
+    __shared__ double sh[256];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < nb; i += 256) s += partials[i];
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        __syncthreads();
     }
+    if (threadIdx.x == 0) out[0] = (float)(sh[0] / (double)n);
 }
 
-// backward of the output layer: dh[v][c] = w[c] dy[v]; dw[c] += sum dy h; db += sum dy
-__global__ void conv_out_bwd(const bf16 *__restrict__ h, const float *__restrict__ dy, const float *__restrict__ w,
-                             bf16 *__restrict__ dh, float *__restrict__ dw, float *__restrict__ db, long long n) {
-    float acc[16], accb = 0.f;
+// backward of the output layer: dh[v][c] = w[c] dy[v] where h > 0 (the ReLU of the layer before), else 0; dw[c] += sum
+// dy h; db += sum dy
+__global__ void __launch_bounds__(256) conv_out_bwd(const bf16 *__restrict__ h, const float *__restrict__ dy,
+                                                    const float *__restrict__ w, bf16 *__restrict__ dh,
+                                                    float *__restrict__ dw, float *__restrict__ db, long long n) {
+    __shared__ float sh[16];
+    float acc[16], wv[16], accb = 0.f;
 #pragma unroll
-    for (int c = 0; c < 16; ++c) acc[c] = 0.f;
+    for (int c = 0; c < 16; ++c) {
+        acc[c] = 0.f;
+        wv[c] = w[c];
+    }
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
         const float g = dy[v];
         accb += g;
 #pragma unroll
-        for (int c = 0; c < 16; c += 2) {
-            const float2 hv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(h + v * 16 + c));
-            acc[c] = fmaf(g, hv.x, acc[c]);
-            acc[c + 1] = fmaf(g, hv.y, acc[c + 1]);
-            *reinterpret_cast<__nv_bfloat162 *>(dh + v * 16 + c) = __floats2bfloat162_rn(w[c] * g, w[c + 1] * g);
+        for (int q = 0; q < 2; ++q) {
+            float hv[8], d[8];
+            unpack8(ld8(h + v * 16 + 8 * q), hv);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                acc[8 * q + c] = fmaf(g, hv[c], acc[8 * q + c]);
+                d[c] = hv[c] > 0.f ? wv[8 * q + c] * g : 0.f;
+            }
+            st8(dh + v * 16 + 8 * q, pack8(d));
         }
     }
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        float s = acc[c];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(dw + c, s);
-    }
-    for (int o = 16; o > 0; o >>= 1) accb += __shfl_xor_sync(0xffffffffu, accb, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(db, accb);
+    for (int c = 0; c < 16; ++c) block_add(acc[c], dw + c, sh);
+    block_add(accb, db, sh);
 }
 
 // 2x2x2 average pool (channels-last), out dims D/2 x H/2 x W/2
 __global__ void avgpool_fwd(const bf16 *__restrict__ in, bf16 *__restrict__ out, int D, int H, int W, int C) {
-    const int d2 = D / 2, h2 = H / 2, w2 = W / 2;
-    const long long n = (long long)d2 * h2 * w2 * (C / 2);
+    const int d2 = D / 2, h2 = H / 2, w2 = W / 2, c8 = C / 8;
+    const long long n = (long long)d2 * h2 * w2 * c8;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(e % (C / 2)) * 2;
-        const long long v = e / (C / 2);
+        const int c = (int)(e % c8) * 8;
+        const long long v = e / c8;
         const int x = (int)(v % w2);
         const long long zy = v / w2;
         const int y = (int)(zy % h2), z = (int)(zy / h2);
-        float s0 = 0.f, s1 = 0.f;
+        float s[8] = {};
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const long long src = ((long long)(2 * z + (k >> 2)) * H + (2 * y + ((k >> 1) & 1))) * W + 2 * x + (k & 1);
-            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(in + src * C + c));
-            s0 += f.x;
-            s1 += f.y;
+            float f[8];
+            unpack8(ld8(in + src * C + c), f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] += f[j];
         }
-        *reinterpret_cast<__nv_bfloat162 *>(out + v * C + c) = __floats2bfloat162_rn(0.125f * s0, 0.125f * s1);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] *= 0.125f;
+        st8(out + v * C + c, pack8(s));
     }
 }
 
@@ -200,31 +323,39 @@ __global__ void avgpool_fwd(const bf16 *__restrict__ in, bf16 *__restrict__ out,
 // e = relu(...) from its pool and its skip connection, already masked by e > 0
 __global__ void pool_bwd_skip_mask(const bf16 *__restrict__ dp, const bf16 *__restrict__ dcat, int ccat, int c_off,
                                    const bf16 *__restrict__ e, bf16 *__restrict__ de, int D, int H, int W, int C) {
-    const long long n = (long long)D * H * W * C;
+    const int c8 = C / 8;
+    const long long n = (long long)D * H * W * c8;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const long long v = i / C;
+        const int c = (int)(i % c8) * 8;
+        const long long v = i / c8;
         const int x = (int)(v % W);
         const long long zy = v / W;
         const int y = (int)(zy % H), z = (int)(zy / H);
         const long long pv = ((long long)(z / 2) * (H / 2) + y / 2) * (W / 2) + x / 2;
-        float g = 0.125f * __bfloat162float(dp[pv * C + c]) + __bfloat162float(dcat[v * ccat + c_off + c]);
-        if (!(__bfloat162float(e[i]) > 0.f)) g = 0.f;
-        de[i] = __float2bfloat16_rn(g);
+        float p[8], k[8], m[8];
+        unpack8(ld8(dp + pv * C + c), p);
+        unpack8(ld8(dcat + v * ccat + c_off + c), k);
+        unpack8(ld8(e + v * C + c), m);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) p[j] = m[j] > 0.f ? 0.125f * p[j] + k[j] : 0.f;
+        st8(de + v * C + c, pack8(p));
     }
 }
 
-// nearest x2 upsampling (channels-last): out D x H x W from in D/2 x H/2 x W/2
+// nearest x2 upsampling (channels-last): out D x H x W from in D/2 x H/2 x W/2; a thread writes the eight children
 __global__ void upsample_fwd(const bf16 *__restrict__ in, bf16 *__restrict__ out, int D, int H, int W, int C) {
-    const long long n = (long long)D * H * W * (C / 2);
+    const int c8 = C / 8, w2 = W / 2, h2 = H / 2;
+    const long long n = (long long)(D / 2) * h2 * W * c8;   // a thread: one x, the four (z, y) children
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(e % (C / 2)) * 2;
-        const long long v = e / (C / 2);
+        const int c = (int)(e % c8) * 8;
+        const long long v = e / c8;
         const int x = (int)(v % W);
         const long long zy = v / W;
-        const int y = (int)(zy % H), z = (int)(zy / H);
-        const long long pv = ((long long)(z / 2) * (H / 2) + y / 2) * (W / 2) + x / 2;
-        *reinterpret_cast<__nv_bfloat162 *>(out + v * C + c) = *reinterpret_cast<const __nv_bfloat162 *>(in + pv * C + c);
+        const int y = (int)(zy % h2), z = (int)(zy / h2);
+        const Bf8 val = ld8(in + (((long long)z * h2 + y) * w2 + x / 2) * C + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            st8(out + (((long long)(2 * z + (k >> 1)) * H + 2 * y + (k & 1)) * W + x) * C + c, val);
     }
 }
 
@@ -233,48 +364,71 @@ __global__ void upsample_fwd(const bf16 *__restrict__ in, bf16 *__restrict__ out
 __global__ void upsample_bwd_mask(const bf16 *__restrict__ dcat, int ccat, const bf16 *__restrict__ a,
                                   bf16 *__restrict__ dlow, int D, int H, int W, int C) {
     // D, H, W: the low (half) resolution
-    const long long n = (long long)D * H * W * C;
+    const int c8 = C / 8;
+    const long long n = (long long)D * H * W * c8;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const long long v = i / C;
+        const int c = (int)(i % c8) * 8;
+        const long long v = i / c8;
         const int x = (int)(v % W);
         const long long zy = v / W;
         const int y = (int)(zy % H), z = (int)(zy / H);
-        float s = 0.f;
+        float s[8] = {}, m[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const long long ch = ((long long)(2 * z + (k >> 2)) * (2 * H) + (2 * y + ((k >> 1) & 1))) * (2 * W) + 2 * x + (k & 1);
-            s += __bfloat162float(dcat[ch * ccat + c]);
+            float f[8];
+            unpack8(ld8(dcat + ch * ccat + c), f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] += f[j];
         }
-        if (!(__bfloat162float(a[i]) > 0.f)) s = 0.f;
-        dlow[i] = __float2bfloat16_rn(s);
+        unpack8(ld8(a + v * C + c), m);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (!(m[j] > 0.f)) s[j] = 0.f;
+        st8(dlow + v * C + c, pack8(s));
     }
 }
 
-// g *= (a > 0), in place
-__global__ void relu_mask(bf16 *__restrict__ g, const bf16 *__restrict__ a, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        if (!(__bfloat162float(a[i]) > 0.f)) g[i] = __float2bfloat16_rn(0.f);
+// db[c] += sum_v g[v][c].  A thread keeps eight channels (the stride is a multiple of C / 8) and sums them in
+// registers; C is 16, 32, 64 or 128.  Shared-memory atomics for every element took 0.96 ms over the thirteen layers
+// at 128 x 256 x 128 voxels.
+__global__ void __launch_bounds__(256) bias_grad(const bf16 *__restrict__ g, float *__restrict__ db, long long nvox, int C) {
+    __shared__ float sb[8][128];
+    const int c8 = C / 8;
+    const long long n = nvox * c8, stride = (long long)gridDim.x * blockDim.x;
+    float s[8] = {};
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+        float f[8];
+        unpack8(ld8(g + i * 8), f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += f[j];
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        for (int o = 16; o >= c8; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+        if (lane < c8) sb[warp][lane * 8 + j] = s[j];
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < C; c += blockDim.x) {
+        float t = 0.f;
+        for (int w = 0; w < 8; ++w) t += sb[w][c];
+        atomicAdd(db + c, t);
+    }
 }
 
-// db[c] += sum_v g[v][c]
-__global__ void bias_grad(const bf16 *__restrict__ g, float *__restrict__ db, long long nvox, int C) {
-    extern __shared__ float sb[];
-    for (int c = threadIdx.x; c < C; c += blockDim.x) sb[c] = 0.f;
-    __syncthreads();
-    const long long n = nvox * C;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        atomicAdd(&sb[i % C], __bfloat162float(g[i]));
-    __syncthreads();
-    for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(db + c, sb[c]);
-}
+// Wt[ci][26 - tap][co] = W[co][tap][ci]: backward-data weights of every layer in one launch (blockIdx.y: layer)
+struct FlipTable {
+    int w[13], cout[13], cin[13];
+};
 
-// Wt[ci][26 - tap][co] = W[co][tap][ci]: backward-data weights
-__global__ void flip_transpose(const bf16 *__restrict__ w, bf16 *__restrict__ wt, int cout, int cin) {
-    const int n = cout * 27 * cin;
+__global__ void flip_transpose(const bf16 *__restrict__ pw, bf16 *__restrict__ pwt, FlipTable T) {
+    const int l = blockIdx.y, cout = T.cout[l], cin = T.cin[l], n = cout * 27 * cin;
+    const bf16 *w = pw + T.w[l];
+    bf16 *wt = pwt + T.w[l];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int ci = i % cin, tap = (i / cin) % 27, co = i / (27 * cin);
-        wt[((size_t)ci * 27 + (26 - tap)) * cout + co] = w[i];
+        const int co = i % cout, t = (i / cout) % 27, ci = i / (27 * cout);
+        wt[i] = w[((size_t)co * 27 + (26 - t)) * cin + ci];
     }
 }
 
@@ -402,19 +556,19 @@ kv_status ensure_workspace(kv_unet *u, int D, int H, int W, bool grads) {
 
 // forward or backward-data convolution of one layer
 kv_status conv3(kv_unet *u, int layer, const bf16 *in1, const bf16 *in2, bf16 *out, int lvl, bool weights_t,
-                int c_in_override = -1) {
+                const bf16 *mask = nullptr, const convtc::Head *head = nullptr) {
     const kv_unet::Conv &L = u->conv[layer];
     kv_ctx *ctx = u->ctx;
     const int D = u->D >> lvl, H = u->H >> lvl, W = u->W >> lvl;
     // forward: in1 (c1) ++ in2 (c2) -> cout with W; backward-data: in1 = dPre (cout) -> c1 + c2 with Wt
     const int c1 = weights_t ? L.cout : L.c1, c2 = weights_t ? 0 : L.c2;
-    const int cout = weights_t ? (c_in_override > 0 ? c_in_override : L.c1 + L.c2) : L.cout;
+    const int cout = weights_t ? L.c1 + L.c2 : L.cout;
     const bf16 *w = weights_t ? u->wt + L.w : u->pb + L.w;
     const float *bias = weights_t ? nullptr : u->p + L.b;
     LaunchTimer lt(ctx, weights_t ? "unet_conv_dgrad" : "unet_conv_fwd");
     // tcgen05 / TMA implicit GEMM (kv_conv_tc.cuh); covers every level of every volume the network takes
-    const char *why = convtc::launch(in1, c1, in2, c2, w, bias, !weights_t, nullptr, out, cout, D, H, W, u->tc_status,
-                                     ctx->sm_count, ctx->stream);
+    const char *why = convtc::launch(in1, c1, in2, c2, w, bias, !weights_t, mask, head, out, cout, D, H, W,
+                                     u->tc_status, ctx->sm_count, ctx->stream);
     if (why != nullptr) return kv_fail(ctx, KV_ERR_UNSUPPORTED, "tensor-core convolution: %s", why);
     KV_CHECK_LAUNCH(ctx, "unet conv3 (tcgen05)");
     return KV_OK;
@@ -433,55 +587,53 @@ kv_status wgrad(kv_unet *u, int layer, const bf16 *dpre, const bf16 *in1, const 
     }
     {
         LaunchTimer lb(ctx, "unet_bias_grad");
-        bias_grad<<<grid_n(ctx, nvox * L.cout), 256, L.cout * sizeof(float), ctx->stream>>>(dpre, u->g + L.b, nvox, L.cout);
+        bias_grad<<<std::min(grid_n(ctx, nvox * (L.cout / 8)), 4 * ctx->sm_count), 256, 0, ctx->stream>>>(dpre, u->g + L.b, nvox, L.cout);
     }
     KV_CHECK_LAUNCH(ctx, "unet wgrad");
     return KV_OK;
 }
 
-kv_status forward(kv_unet *u) {
+kv_status forward(kv_unet *u, bool keep) {
     kv_ctx *ctx = u->ctx;
     const int D = u->D, H = u->H, W = u->W;
     const long long n0 = (long long)D * H * W;
     bf16 **a = u->act;
     {
         LaunchTimer lt(ctx, "unet_conv_first");
-        conv_first_fwd<<<grid_n(ctx, n0), 256, 0, ctx->stream>>>(u->x, u->p + u->w_first, u->p + u->b_first, a[A0], D, H, W);
+        conv_first_fwd<<<dim3(W / 128, (unsigned)std::min<long long>((long long)D * (H / kFirstRows), 65535)), 128, 0, ctx->stream>>>(u->x, u->p + u->w_first, u->p + u->b_first, a[A0], D, H, W);
     }
     KV_TRY(conv3(u, 0, a[A0], nullptr, a[E1], 0, false));
-    avgpool_fwd<<<grid_n(ctx, (n0 >> 3) * 8), 256, 0, ctx->stream>>>(a[E1], a[P1], D, H, W, 16);
+    avgpool_fwd<<<grid_n(ctx, (n0 >> 3) * 2), 256, 0, ctx->stream>>>(a[E1], a[P1], D, H, W, 16);
     KV_TRY(conv3(u, 1, a[P1], nullptr, a[A2], 1, false));
     KV_TRY(conv3(u, 2, a[A2], nullptr, a[E2], 1, false));
-    avgpool_fwd<<<grid_n(ctx, (n0 >> 6) * 16), 256, 0, ctx->stream>>>(a[E2], a[P2], D >> 1, H >> 1, W >> 1, 32);
+    avgpool_fwd<<<grid_n(ctx, (n0 >> 6) * 4), 256, 0, ctx->stream>>>(a[E2], a[P2], D >> 1, H >> 1, W >> 1, 32);
     KV_TRY(conv3(u, 3, a[P2], nullptr, a[A4], 2, false));
     KV_TRY(conv3(u, 4, a[A4], nullptr, a[E3], 2, false));
-    avgpool_fwd<<<grid_n(ctx, (n0 >> 9) * 32), 256, 0, ctx->stream>>>(a[E3], a[P3], D >> 2, H >> 2, W >> 2, 64);
+    avgpool_fwd<<<grid_n(ctx, (n0 >> 9) * 8), 256, 0, ctx->stream>>>(a[E3], a[P3], D >> 2, H >> 2, W >> 2, 64);
     KV_TRY(conv3(u, 5, a[P3], nullptr, a[A6], 3, false));
     KV_TRY(conv3(u, 6, a[A6], nullptr, a[B], 3, false));
-    upsample_fwd<<<grid_n(ctx, (n0 >> 6) * 64), 256, 0, ctx->stream>>>(a[B], a[U3], D >> 2, H >> 2, W >> 2, 128);
+    upsample_fwd<<<grid_n(ctx, (n0 >> 8) * 16), 256, 0, ctx->stream>>>(a[B], a[U3], D >> 2, H >> 2, W >> 2, 128);
     KV_TRY(conv3(u, 7, a[U3], a[E3], a[A8], 2, false));
     KV_TRY(conv3(u, 8, a[A8], nullptr, a[D3], 2, false));
-    upsample_fwd<<<grid_n(ctx, (n0 >> 3) * 32), 256, 0, ctx->stream>>>(a[D3], a[U2], D >> 1, H >> 1, W >> 1, 64);
+    upsample_fwd<<<grid_n(ctx, (n0 >> 5) * 8), 256, 0, ctx->stream>>>(a[D3], a[U2], D >> 1, H >> 1, W >> 1, 64);
     KV_TRY(conv3(u, 9, a[U2], a[E2], a[A10], 1, false));
     KV_TRY(conv3(u, 10, a[A10], nullptr, a[D2], 1, false));
-    upsample_fwd<<<grid_n(ctx, n0 * 16), 256, 0, ctx->stream>>>(a[D2], a[U1], D, H, W, 32);
+    upsample_fwd<<<grid_n(ctx, (n0 >> 2) * 4), 256, 0, ctx->stream>>>(a[D2], a[U1], D, H, W, 32);
     KV_TRY(conv3(u, 11, a[U1], a[E1], a[A12], 0, false));
-    KV_TRY(conv3(u, 12, a[A12], nullptr, a[D1], 0, false));
-    {
-        LaunchTimer lt(ctx, "unet_conv_out");
-        conv_out_fwd<<<grid_n(ctx, n0), 256, 0, ctx->stream>>>(a[D1], u->x, u->p + u->w_out, u->p + u->b_out, u->y, n0);
-    }
+    // the output layer reads the last layer's voxels where they are computed; D1 itself is kept for the backward pass
+    const convtc::Head head{u->p + u->w_out, u->p + u->b_out, u->x, u->y};
+    KV_TRY(conv3(u, 12, a[A12], nullptr, keep ? a[D1] : nullptr, 0, false, nullptr, &head));
     KV_CHECK_LAUNCH(ctx, "unet forward");
     return KV_OK;
 }
 
 // backward of a conv + relu layer whose output gradient (already masked by
 // the layer's relu) is dpre: weight / bias gradients and the input gradient
-// into dx (unmasked; c_dx channels)
-kv_status conv_backward(kv_unet *u, int layer, const bf16 *dpre, const bf16 *in1, const bf16 *in2, bf16 *dx, int lvl) {
+// into dx, zero where `mask` (the relu output it is the gradient of, when in1 is one) is not positive
+kv_status conv_backward(kv_unet *u, int layer, const bf16 *dpre, const bf16 *in1, const bf16 *in2, bf16 *dx, int lvl,
+                        const bf16 *mask = nullptr) {
     KV_TRY(wgrad(u, layer, dpre, in1, in2, lvl));
-    if (dx != nullptr) KV_TRY(conv3(u, layer, dpre, nullptr, dx, lvl, true));
-    return KV_OK;
+    return conv3(u, layer, dpre, nullptr, dx, lvl, true, mask);
 }
 
 kv_status backward(kv_unet *u) {
@@ -490,53 +642,46 @@ kv_status backward(kv_unet *u) {
     const long long n0 = (long long)D * H * W;
     bf16 **a = u->act, **g = u->grad;
     // weights for the backward-data convolutions
-    for (int l = 0; l < 14; ++l) {
-        const kv_unet::Conv &L = u->conv[l];
-        if (L.cout == 0) continue;
-        const int n = L.cout * 27 * (L.c1 + L.c2);
-        flip_transpose<<<(n + 255) / 256, 256, 0, ctx->stream>>>(u->pb + L.w, u->wt + L.w, L.cout, L.c1 + L.c2);
+    FlipTable flip;
+    for (int l = 0; l < 13; ++l) {
+        flip.w[l] = (int)u->conv[l].w;
+        flip.cout[l] = u->conv[l].cout;
+        flip.cin[l] = u->conv[l].c1 + u->conv[l].c2;
     }
+    flip_transpose<<<dim3(4 * ctx->sm_count / 13 + 1, 13), 256, 0, ctx->stream>>>(u->pb, u->wt, flip);
     // output layer
-    conv_out_bwd<<<grid_n(ctx, n0), 256, 0, ctx->stream>>>(a[D1], u->dy, u->p + u->w_out, g[D1], u->g + u->w_out,
+    conv_out_bwd<<<std::min(grid_n(ctx, n0), 4 * ctx->sm_count), 256, 0, ctx->stream>>>(a[D1], u->dy, u->p + u->w_out, g[D1], u->g + u->w_out,
                                                            u->g + u->b_out, n0);
-    relu_mask<<<grid_n(ctx, n0 * 16), 256, 0, ctx->stream>>>(g[D1], a[D1], n0 * 16);
     // level 0 decoder
-    KV_TRY(conv_backward(u, 12, g[D1], a[A12], nullptr, g[A12], 0));
-    relu_mask<<<grid_n(ctx, n0 * 16), 256, 0, ctx->stream>>>(g[A12], a[A12], n0 * 16);
+    KV_TRY(conv_backward(u, 12, g[D1], a[A12], nullptr, g[A12], 0, a[A12]));
     KV_TRY(conv_backward(u, 11, g[A12], a[U1], a[E1], g[CAT1], 0));      // 48 ch: up(d2) 32 ++ e1 16
-    upsample_bwd_mask<<<grid_n(ctx, (n0 >> 3) * 32), 256, 0, ctx->stream>>>(g[CAT1], 48, a[D2], g[D2], D >> 1, H >> 1, W >> 1, 32);
+    upsample_bwd_mask<<<grid_n(ctx, (n0 >> 3) * 4), 256, 0, ctx->stream>>>(g[CAT1], 48, a[D2], g[D2], D >> 1, H >> 1, W >> 1, 32);
     // level 1 decoder
-    KV_TRY(conv_backward(u, 10, g[D2], a[A10], nullptr, g[A10], 1));
-    relu_mask<<<grid_n(ctx, (n0 >> 3) * 32), 256, 0, ctx->stream>>>(g[A10], a[A10], (n0 >> 3) * 32);
+    KV_TRY(conv_backward(u, 10, g[D2], a[A10], nullptr, g[A10], 1, a[A10]));
     KV_TRY(conv_backward(u, 9, g[A10], a[U2], a[E2], g[CAT2], 1));       // 96 ch: up(d3) 64 ++ e2 32
-    upsample_bwd_mask<<<grid_n(ctx, (n0 >> 6) * 64), 256, 0, ctx->stream>>>(g[CAT2], 96, a[D3], g[D3], D >> 2, H >> 2, W >> 2, 64);
+    upsample_bwd_mask<<<grid_n(ctx, (n0 >> 6) * 8), 256, 0, ctx->stream>>>(g[CAT2], 96, a[D3], g[D3], D >> 2, H >> 2, W >> 2, 64);
     // level 2 decoder
-    KV_TRY(conv_backward(u, 8, g[D3], a[A8], nullptr, g[A8], 2));
-    relu_mask<<<grid_n(ctx, (n0 >> 6) * 64), 256, 0, ctx->stream>>>(g[A8], a[A8], (n0 >> 6) * 64);
+    KV_TRY(conv_backward(u, 8, g[D3], a[A8], nullptr, g[A8], 2, a[A8]));
     KV_TRY(conv_backward(u, 7, g[A8], a[U3], a[E3], g[CAT3], 2));        // 192 ch: up(b) 128 ++ e3 64
-    upsample_bwd_mask<<<grid_n(ctx, (n0 >> 9) * 128), 256, 0, ctx->stream>>>(g[CAT3], 192, a[B], g[B], D >> 3, H >> 3, W >> 3, 128);
+    upsample_bwd_mask<<<grid_n(ctx, (n0 >> 9) * 16), 256, 0, ctx->stream>>>(g[CAT3], 192, a[B], g[B], D >> 3, H >> 3, W >> 3, 128);
     // bottleneck
-    KV_TRY(conv_backward(u, 6, g[B], a[A6], nullptr, g[A6], 3));
-    relu_mask<<<grid_n(ctx, (n0 >> 9) * 128), 256, 0, ctx->stream>>>(g[A6], a[A6], (n0 >> 9) * 128);
+    KV_TRY(conv_backward(u, 6, g[B], a[A6], nullptr, g[A6], 3, a[A6]));
     KV_TRY(conv_backward(u, 5, g[A6], a[P3], nullptr, g[P3], 3));
-    pool_bwd_skip_mask<<<grid_n(ctx, (n0 >> 6) * 64), 256, 0, ctx->stream>>>(g[P3], g[CAT3], 192, 128, a[E3], g[E3],
+    pool_bwd_skip_mask<<<grid_n(ctx, (n0 >> 6) * 8), 256, 0, ctx->stream>>>(g[P3], g[CAT3], 192, 128, a[E3], g[E3],
                                                                              D >> 2, H >> 2, W >> 2, 64);
     // level 2 encoder
-    KV_TRY(conv_backward(u, 4, g[E3], a[A4], nullptr, g[A4], 2));
-    relu_mask<<<grid_n(ctx, (n0 >> 6) * 64), 256, 0, ctx->stream>>>(g[A4], a[A4], (n0 >> 6) * 64);
+    KV_TRY(conv_backward(u, 4, g[E3], a[A4], nullptr, g[A4], 2, a[A4]));
     KV_TRY(conv_backward(u, 3, g[A4], a[P2], nullptr, g[P2], 2));
-    pool_bwd_skip_mask<<<grid_n(ctx, (n0 >> 3) * 32), 256, 0, ctx->stream>>>(g[P2], g[CAT2], 96, 64, a[E2], g[E2],
+    pool_bwd_skip_mask<<<grid_n(ctx, (n0 >> 3) * 4), 256, 0, ctx->stream>>>(g[P2], g[CAT2], 96, 64, a[E2], g[E2],
                                                                              D >> 1, H >> 1, W >> 1, 32);
     // level 1 encoder
-    KV_TRY(conv_backward(u, 2, g[E2], a[A2], nullptr, g[A2], 1));
-    relu_mask<<<grid_n(ctx, (n0 >> 3) * 32), 256, 0, ctx->stream>>>(g[A2], a[A2], (n0 >> 3) * 32);
+    KV_TRY(conv_backward(u, 2, g[E2], a[A2], nullptr, g[A2], 1, a[A2]));
     KV_TRY(conv_backward(u, 1, g[A2], a[P1], nullptr, g[P1], 1));
-    pool_bwd_skip_mask<<<grid_n(ctx, n0 * 16), 256, 0, ctx->stream>>>(g[P1], g[CAT1], 48, 32, a[E1], g[E1], D, H, W, 16);
+    pool_bwd_skip_mask<<<grid_n(ctx, n0 * 2), 256, 0, ctx->stream>>>(g[P1], g[CAT1], 48, 32, a[E1], g[E1], D, H, W, 16);
     // level 0 encoder
-    KV_TRY(conv_backward(u, 0, g[E1], a[A0], nullptr, g[A0], 0));
-    relu_mask<<<grid_n(ctx, n0 * 16), 256, 0, ctx->stream>>>(g[A0], a[A0], n0 * 16);
+    KV_TRY(conv_backward(u, 0, g[E1], a[A0], nullptr, g[A0], 0, a[A0]));
     {
-        dim3 grid(grid_n(ctx, n0) > 1024 ? 1024 : grid_n(ctx, n0), 27);
+        dim3 grid(std::min(grid_n(ctx, n0), ctx->sm_count), 3);
         conv_first_wgrad<<<grid, 256, 0, ctx->stream>>>(u->x, g[A0], u->g + u->w_first, u->g + u->b_first, D, H, W);
     }
     KV_CHECK_LAUNCH(ctx, "unet backward");
@@ -548,14 +693,14 @@ kv_status loss_and_grad(kv_unet *u) {
     const long long n0 = (long long)u->D * u->H * u->W;
     const int nb = grid_n(ctx, n0) > 4096 ? 4096 : grid_n(ctx, n0);
     mse_loss<<<nb, 256, 0, ctx->stream>>>(u->y, u->t, u->dy, n0, u->partials);
-    sum_loss<<<1, 32, 0, ctx->stream>>>(u->partials, nb, n0, u->loss);
+    sum_loss<<<1, 256, 0, ctx->stream>>>(u->partials, nb, n0, u->loss);
     KV_CHECK_LAUNCH(ctx, "unet loss");
     return KV_OK;
 }
 
 kv_status train_body(kv_unet *u, float lr, bool apply) {
     kv_ctx *ctx = u->ctx;
-    KV_TRY(forward(u));
+    KV_TRY(forward(u, true));
     KV_TRY(loss_and_grad(u));
     KV_CHECK_CUDA(ctx, cudaMemsetAsync(u->g, 0, u->nparams * sizeof(float), ctx->stream));
     KV_TRY(backward(u));
@@ -692,7 +837,7 @@ extern "C" kv_status kv_unet_forward(kv_unet *u, const float *in, float *out, in
     KV_TRY(ensure_workspace(u, D, H, W, false));
     const size_t n = (size_t)D * H * W;
     KV_TRY(copy_in(u, u->x, in, n, mem));
-    KV_TRY(forward(u));
+    KV_TRY(forward(u, false));
     KV_CHECK_CUDA(ctx, cudaMemcpyAsync(out, u->y, n * sizeof(float),
                                        mem == KV_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, ctx->stream));
     return tc_check(u);
@@ -815,7 +960,7 @@ extern "C" kv_status kv_conv3_bf16(kv_ctx *ctx, const uint16_t *in1, int32_t c1,
     // volumes that are not whole tiles take the tensor-core kernel too where it covers the call, else mma.sync; the
     // two sum in the same order, with equal bits
     if (kernel != 2) {
-        const char *why = convtc::launch(a, c1, c2 ? b : nullptr, c2, wb, bias, relu != 0, nullptr, o, cout, D, H, W,
+        const char *why = convtc::launch(a, c1, c2 ? b : nullptr, c2, wb, bias, relu != 0, nullptr, nullptr, o, cout, D, H, W,
                                          ctx->d_status, ctx->sm_count, ctx->stream);
         if (why == nullptr) {
             KV_CHECK_LAUNCH(ctx, "kv_conv3_bf16 (tcgen05)");
