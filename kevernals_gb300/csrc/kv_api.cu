@@ -478,8 +478,12 @@ extern "C" kv_status kv_plan_create(kv_ctx *ctx, const kv_geometry *g, kv_family
             cudaMalloc((void **)&plan->d_org, bytes) != cudaSuccess) {
             s = kv_fail(ctx, KV_ERR_OOM, "plan tables");
         } else {
-            cudaMemcpy(plan->d_src, plan->src.data(), bytes, cudaMemcpyHostToDevice);
-            cudaMemcpy(plan->d_org, plan->det.data(), bytes, cudaMemcpyHostToDevice);
+            // every stream that uses the plan later finds the tables done
+            cudaMemcpyAsync(plan->d_src, plan->src.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
+            cudaMemcpyAsync(plan->d_org, plan->det.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
+            s = rc_build_tables(plan);
+            if (cudaStreamSynchronize(ctx->stream) != cudaSuccess && s == KV_OK)
+                s = kv_fail(ctx, KV_ERR_CUDA, "plan tables");
         }
     }
     if (s != KV_OK) {
@@ -497,6 +501,7 @@ extern "C" kv_status kv_plan_destroy(kv_plan *plan) {
     exact_free_tables(&plan->ex);
     cudaFree(plan->d_src);
     cudaFree(plan->d_org);
+    cudaFree(plan->d_rctab);
     cudaFree(plan->d_vol);
     cudaFree(plan->d_proj);
     cudaFree(plan->d_ratio);

@@ -118,6 +118,7 @@ struct kv_plan {
     BackStageCfg bstage;             // staged backprojector (R == 0: not used)
     float *d_src = nullptr;          // RC family: [P][3] sources (float3 layout)
     float *d_org = nullptr;          // RC family: [P][3] detector origins
+    float *d_rctab = nullptr;        // RC family: ray components of detector columns and rows (rc_build_tables)
 
     // workspace (allocated on demand, kept for the plan's lifetime)
     void *d_vol = nullptr;           // volume in storage type
@@ -258,6 +259,8 @@ kv_status exact_back_slab_launch(kv_plan *plan, BackMode mode, const BackArgs &a
 kv_status exact_sensitivity_launch(kv_plan *plan, double *sens);
 kv_status exact_prescale_launch(kv_plan *plan, const float *y, void *yp);
 
+// the backprojector's tables from d_src / d_org (on the context stream)
+kv_status rc_build_tables(kv_plan *plan);
 kv_status rc_forward_launch(kv_plan *plan, const float *d_src, const float *d_org, int n_views,
                             int mode, const float *vol, const float *meas, float *out,
                             float relax);

@@ -113,6 +113,23 @@ def test_rc_random_geometries_match_oracle(ctx):
         assert np.array_equal(plan.back(f), O.rc_back(g, f))
 
 
+@pytest.mark.parametrize("geom", [
+    (37, 21, 5, 1.0, 1.0, 2.0, 3, 90, 70, 0.1, 0.1, 20.0),      # a voxel covers more pixels than the window
+    (40, 33, 6, 0.2, 0.3, 0.5, 4, 30, 30, 0.9, 0.7, 12.0),      # pixels wider than voxels
+    (20, 18, 3, 0.5, 0.5, 1.0, 67, 24, 22, 0.6, 0.6, 25.0),     # more views than a block holds at a time
+    (16, 16, 40, 0.5, 0.5, 4.0, 5, 40, 300, 0.2, 0.1, 35.0),    # thick, steep
+])
+def test_rc_back_window_cut_matches_oracle(ctx, geom):
+    """The backprojector's cut window against the oracle's full one, bit for bit."""
+    g = linear_sweep(*geom)
+    rng = np.random.default_rng(12)
+    plan = engine.Plan(ctx, g, "rc")
+    p = rng.random(g.proj_shape, dtype=np.float32)
+    assert np.array_equal(plan.back(p), O.rc_back(g, p))
+    vol = rng.random(g.volume_shape, dtype=np.float32)
+    assert np.array_equal(plan.forward(vol), O.rc_forward(g, vol))
+
+
 # ------------------------------------------------------------- EXACT family
 
 @pytest.mark.parametrize("gi", [0, 1, 2])
