@@ -46,31 +46,61 @@ __global__ void __launch_bounds__(256) saa_kernel(int nu, int nv, int nz, int P,
 }
 
 // The same sums with each view's rows staged in shared memory.  A block
-// covers 32 detector columns x kSaaRows rows x kSaaSlices slices; for every
+// covers 32 detector columns x kSaaRows rows x KS slices; for every
 // view one thread loads, by TMA, the band of that view's rows the block's
 // shifted rows reach (kSaaRows + the largest spread of the block's shifts;
 // rows outside the detector read zeros, which is the reference's zero
 // padding) into a ring of shared-memory stages, and every thread adds its
-// kSaaRows / 8 x kSaaSlices outputs' rows from the band.  Views are added in
+// kSaaRows / 8 x KS outputs' rows from the band.  Views are added in
 // the same order with the same TwoSum as saa_kernel, and a row outside the
 // detector adds an exact zero, so the two kernels agree bit for bit.
-constexpr int kSaaRows = 32, kSaaSlices = 4, kSaaStages = 3;
+//
+// Seven FP32 additions per row and slice bound it (60 views of 2048 x 2048
+// into 128 slices: 2.3e11, 6.0 ms of the FP32 pipes).  Two rows a step in
+// packed additions (each half rounds as the scalar one) halve the issue slots,
+// one check of the band per slice and eight slices per staged band the rest:
+// 18.4 -> 11.7 ms there.  Where eight slices' spread does not fit, four.
+constexpr int kSaaRows = 32, kSaaStages = 4;
 constexpr uint32_t kSaaWaitPolls = 1u << 22;
 
-__global__ void __launch_bounds__(256) saa_band_kernel(const __grid_constant__ CUtensorMap pmap, int nu, int nv,
-                                                       int nz, int P, const int32_t *__restrict__ shift,
-                                                       float *__restrict__ out, int nb, uint32_t stage_stride,
-                                                       int *status) {
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long r, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a - b as b * -1 + a, rounded once: the packed multiply-add is native, the packed subtraction was not (10 instead of 5
+// instructions a row and slice)
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+    return r;
+}
+
+template <int KS>
+__global__ void __launch_bounds__(256, 2) saa_band_kernel(const __grid_constant__ CUtensorMap pmap, int nu, int nv,
+                                                          int nz, int P, const int32_t *__restrict__ shift,
+                                                          float *__restrict__ out, int nb, uint32_t stage_stride,
+                                                          int wide, int *status) {
+    constexpr int kPairs = kSaaRows / 16;   // a half warp a row, two columns a lane
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full[kSaaStages];
     __shared__ int bstart[kSaaStages];
     unsigned char *base = smem + ((128u - (kvtma::smem_u32(smem) & 127u)) & 127u);
     float *bands = reinterpret_cast<float *>(base);
-    int *sh = reinterpret_cast<int *>(base + kSaaStages * stage_stride);     // [kSaaSlices][P]
+    int *sh = reinterpret_cast<int *>(base + kSaaStages * stage_stride);     // [P][KS]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int u0 = blockIdx.x * 32, v0 = blockIdx.y * kSaaRows, k0 = blockIdx.z * kSaaSlices;
-    const int kn = min(kSaaSlices, nz - k0);
-    for (int t = threadIdx.x; t < kn * P; t += blockDim.x) sh[t] = shift[(size_t)k0 * P + t];
+    const int u0 = blockIdx.x * 32, v0 = blockIdx.y * kSaaRows, k0 = blockIdx.z * KS;
+    const int kn = min(KS, nz - k0);
+    for (int t = threadIdx.x; t < KS * P; t += blockDim.x)   // slices past the last repeat it
+        sh[t] = shift[(size_t)(k0 + min(t % KS, kn - 1)) * P + t / KS];
     if (threadIdx.x == 0) {
         for (int s = 0; s < kSaaStages; ++s) kvtma::mbar_init(&full[s], 1);
         kvtma::fence_mbar_init();
@@ -78,8 +108,8 @@ __global__ void __launch_bounds__(256) saa_band_kernel(const __grid_constant__ C
     __syncthreads();
     const uint32_t band_bytes = 32u * (uint32_t)nb * 4u;
     auto issue = [&](int i, int st) {
-        int tmin = sh[i];
-        for (int kk = 1; kk < kn; ++kk) tmin = min(tmin, sh[kk * P + i]);
+        int tmin = sh[i * KS];
+        for (int kk = 1; kk < KS; ++kk) tmin = min(tmin, sh[i * KS + kk]);
         const int bs = v0 + tmin;
         bstart[st] = bs;
         kvtma::fence_proxy_async_smem();
@@ -89,40 +119,55 @@ __global__ void __launch_bounds__(256) saa_band_kernel(const __grid_constant__ C
     if (threadIdx.x == 0)
         for (int i = 0; i < kSaaStages && i < P; ++i) issue(i, i);
     __syncthreads();
-    float hi[kSaaRows / 8][kSaaSlices], lo[kSaaRows / 8][kSaaSlices];
+    const int row0 = 2 * warp + (lane >> 4), col0 = 2 * (lane & 15);
+    unsigned long long hi[kPairs][KS], lo[kPairs][KS];   // rows 16 m + row0, columns col0 and col0 + 1
 #pragma unroll
-    for (int m = 0; m < kSaaRows / 8; ++m)
+    for (int m = 0; m < kPairs; ++m)
 #pragma unroll
-        for (int kk = 0; kk < kSaaSlices; ++kk) hi[m][kk] = lo[m][kk] = 0.f;
+        for (int kk = 0; kk < KS; ++kk) hi[m][kk] = lo[m][kk] = 0ull;
     int err = 0, i = 0;
-    for (; i < P; ++i) {
+    // one view's rows into sums a -> b: two register sets, so that the new sums need no move into the old ones' place
+    auto add_view = [&](int view, int st, unsigned long long (&a)[kPairs][KS], unsigned long long (&b)[kPairs][KS]) {
+        const float *band = bands + (size_t)st * (stage_stride / 4) + col0;
+        const int rel = v0 + row0 - bstart[st];
+#pragma unroll
+        for (int kk = 0; kk < KS; ++kk) {
+            const int r0 = rel + sh[view * KS + kk];
+            const bool in = (unsigned)r0 <= (unsigned)(nb - kSaaRows + 15);
+            if (!in) err |= 4;                                          // rows outside the band: never expected
+            const float *row = band + (in ? r0 : 0) * 32;
+#pragma unroll
+            for (int m = 0; m < kPairs; ++m) {
+                const unsigned long long x = *reinterpret_cast<const unsigned long long *>(row + 16 * m * 32);
+                b[m][kk] = add2(a[m][kk], x);                           // TwoSum(a, x)
+                const unsigned long long bp = sub2(b[m][kk], a[m][kk]);
+                const unsigned long long e = add2(sub2(a[m][kk], sub2(b[m][kk], bp)), sub2(x, bp));
+                lo[m][kk] = add2(lo[m][kk], e);
+            }
+        }
+    };
+    for (; i < P; i += 2) {   // two views a barrier
         const int st = i % kSaaStages;
+        const bool two = i + 1 < P;
         if (!kvtma::mbar_wait_bounded(&full[st], (uint32_t)(i / kSaaStages) & 1u, kSaaWaitPolls)) err |= 1;
+        if (two && !kvtma::mbar_wait_bounded(&full[st + 1], (uint32_t)(i / kSaaStages) & 1u, kSaaWaitPolls)) err |= 1;
         if (err == 0) {
-            const float *band = bands + (size_t)st * (stage_stride / 4);
-            const int rel = v0 + warp - bstart[st];
+            unsigned long long mid[kPairs][KS];
+            add_view(i, st, hi, mid);
+            if (two) {
+                add_view(i + 1, st + 1, mid, hi);
+            } else {
 #pragma unroll
-            for (int kk = 0; kk < kSaaSlices; ++kk) {
-                if (kk >= kn) break;
-                const int r0 = rel + sh[kk * P + i];
+                for (int m = 0; m < kPairs; ++m)
 #pragma unroll
-                for (int m = 0; m < kSaaRows / 8; ++m) {
-                    const int r = r0 + 8 * m;
-                    if ((unsigned)r >= (unsigned)nb) {   // outside the band: never expected
-                        err |= 4;
-                        continue;
-                    }
-                    const float x = band[r * 32 + lane];
-                    const float sm = hi[m][kk] + x;                 // TwoSum(hi, x)
-                    const float bp = sm - hi[m][kk];
-                    const float e = (hi[m][kk] - (sm - bp)) + (x - bp);
-                    hi[m][kk] = sm;
-                    lo[m][kk] += e;
-                }
+                    for (int kk = 0; kk < KS; ++kk) hi[m][kk] = mid[m][kk];
             }
         }
         if (__syncthreads_or(err)) break;
-        if (threadIdx.x == 0 && i + kSaaStages < P) issue(i + kSaaStages, st);
+        if (threadIdx.x == 0) {
+            if (i + kSaaStages < P) issue(i + kSaaStages, st);
+            if (i + 1 + kSaaStages < P) issue(i + 1 + kSaaStages, st + 1);
+        }
     }
     if (i < P) {   // failed: record, let the loads in flight land, leave
         if (err) atomicOr(status, err);
@@ -131,16 +176,27 @@ __global__ void __launch_bounds__(256) saa_band_kernel(const __grid_constant__ C
                 kvtma::mbar_wait_bounded(&full[j % kSaaStages], (uint32_t)(j / kSaaStages) & 1u, kSaaWaitPolls);
         return;
     }
-    const int u = u0 + lane;
+    const int u = u0 + col0;   // nu is a multiple of 4 here
     if (u >= nu) return;
     const double w = 1.0 / (double)P;
 #pragma unroll
-    for (int kk = 0; kk < kSaaSlices; ++kk) {
+    for (int kk = 0; kk < KS; ++kk) {
         if (kk >= kn) break;
 #pragma unroll
-        for (int m = 0; m < kSaaRows / 8; ++m) {
-            const int v = v0 + warp + 8 * m;
-            if (v < nv) out[((size_t)(k0 + kk) * nv + v) * nu + u] = (float)(((double)hi[m][kk] + (double)lo[m][kk]) * w);
+        for (int m = 0; m < kPairs; ++m) {
+            const int v = v0 + row0 + 16 * m;
+            if (v >= nv) continue;
+            float h[2], l[2];
+            unpack2(hi[m][kk], h[0], h[1]);
+            unpack2(lo[m][kk], l[0], l[1]);
+            const float2 o = make_float2((float)(((double)h[0] + (double)l[0]) * w), (float)(((double)h[1] + (double)l[1]) * w));
+            float *dst = out + ((size_t)(k0 + kk) * nv + v) * nu + u;
+            if (wide) {
+                *reinterpret_cast<float2 *>(dst) = o;
+            } else {
+                dst[0] = o.x;
+                dst[1] = o.y;
+            }
         }
     }
 }
@@ -395,13 +451,13 @@ kv_status ramp_filter_launch(kv_plan *plan, const float *in, float *out, int hal
 namespace {
 
 // Rows of the band a block of the staged kernel needs: kSaaRows + the
-// largest spread of one block's shifts over its slices, for any view.
-int saa_band_rows(const kv_geometry &g, const int32_t *sh) {
+// largest spread of one block's shifts over its ks slices, for any view.
+int saa_band_rows(const kv_geometry &g, const int32_t *sh, int ks) {
     int span = 0;
-    for (int k0 = 0; k0 < g.nz; k0 += kSaaSlices)
+    for (int k0 = 0; k0 < g.nz; k0 += ks)
         for (int i = 0; i < g.n_views; ++i) {
             int lo = sh[(size_t)k0 * g.n_views + i], hi = lo;
-            for (int k = k0 + 1; k < std::min(g.nz, k0 + kSaaSlices); ++k) {
+            for (int k = k0 + 1; k < std::min(g.nz, k0 + ks); ++k) {
                 lo = std::min(lo, sh[(size_t)k * g.n_views + i]);
                 hi = std::max(hi, sh[(size_t)k * g.n_views + i]);
             }
@@ -410,33 +466,49 @@ int saa_band_rows(const kv_geometry &g, const int32_t *sh) {
     return kSaaRows + span;
 }
 
+// The staged kernel with KS slices a block; false where its band does not fit.
+template <int KS>
+bool saa_band_launch(kv_plan *plan, const int32_t *d_shift, const int32_t *h_shift, const float *proj, float *out,
+                     size_t smem_limit, kv_status *status) {
+    const kv_geometry &g = plan->g;
+    kv_ctx *ctx = plan->ctx;
+    const int nb = saa_band_rows(g, h_shift, KS);
+    const uint32_t stride = (uint32_t)((32u * nb * 4u + 127u) / 128u * 128u);
+    const size_t smem = (size_t)kSaaStages * stride + (size_t)KS * g.n_views * sizeof(int32_t) + 128;
+    if (nb > 256 || smem > smem_limit) return false;
+    CUtensorMap map;
+    cuuint64_t dims[3] = {(cuuint64_t)g.nu, (cuuint64_t)g.nv, (cuuint64_t)g.n_views};
+    cuuint64_t strides[2] = {(cuuint64_t)g.nu * 4, (cuuint64_t)g.nu * g.nv * 4};
+    cuuint32_t box[3] = {32, (cuuint32_t)nb, 1};
+    cuuint32_t es[3] = {1, 1, 1};
+    if (kvtma::encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(proj), dims, strides, box, es,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    *status = [&]() -> kv_status {
+        KV_CHECK_CUDA(ctx, cudaFuncSetAttribute(saa_band_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        dim3 grid((g.nu + 31) / 32, (g.nv + kSaaRows - 1) / kSaaRows, (g.nz + KS - 1) / KS);
+        LaunchTimer lt(ctx, "saa");
+        saa_band_kernel<KS><<<grid, 256, smem, ctx->stream>>>(map, g.nu, g.nv, g.nz, g.n_views, d_shift, out, nb, stride,
+                                                              reinterpret_cast<uintptr_t>(out) % 8 == 0, ctx->d_status);
+        KV_CHECK_LAUNCH(ctx, "saa_band_kernel");
+        return KV_OK;
+    }();
+    return true;
+}
+
 }  // namespace
 
 kv_status saa_launch(kv_plan *plan, const int32_t *d_shift, const int32_t *h_shift, const float *proj, float *out) {
     const kv_geometry &g = plan->g;
     kv_ctx *ctx = plan->ctx;
-    // the staged kernel where its band fits and TMA can address the stack
-    const int nb = saa_band_rows(g, h_shift);
-    const uint32_t stride = (uint32_t)((32u * nb * 4u + 127u) / 128u * 128u);
-    const size_t smem = (size_t)kSaaStages * stride + (size_t)kSaaSlices * g.n_views * sizeof(int32_t) + 128;
-    if (nb <= 256 && smem <= 160 * 1024 && (g.nu * 4) % 16 == 0 && reinterpret_cast<uintptr_t>(proj) % 16 == 0 &&
-        kvtma::encoder() != nullptr) {
-        CUtensorMap map;
-        cuuint64_t dims[3] = {(cuuint64_t)g.nu, (cuuint64_t)g.nv, (cuuint64_t)g.n_views};
-        cuuint64_t strides[2] = {(cuuint64_t)g.nu * 4, (cuuint64_t)g.nu * g.nv * 4};
-        cuuint32_t box[3] = {32, (cuuint32_t)nb, 1};
-        cuuint32_t es[3] = {1, 1, 1};
-        if (kvtma::encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(proj), dims, strides, box,
-                             es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS) {
-            KV_CHECK_CUDA(ctx, cudaFuncSetAttribute(saa_band_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            dim3 grid((g.nu + 31) / 32, (g.nv + kSaaRows - 1) / kSaaRows, (g.nz + kSaaSlices - 1) / kSaaSlices);
-            LaunchTimer lt(ctx, "saa");
-            saa_band_kernel<<<grid, 256, smem, ctx->stream>>>(map, g.nu, g.nv, g.nz, g.n_views, d_shift, out, nb,
-                                                              stride, ctx->d_status);
-            KV_CHECK_LAUNCH(ctx, "saa_band_kernel");
-            return KV_OK;
-        }
+    // the staged kernel where its band fits and TMA can address the stack; eight slices a block where two blocks
+    // stay resident
+    if ((g.nu * 4) % 16 == 0 && reinterpret_cast<uintptr_t>(proj) % 16 == 0 && kvtma::encoder() != nullptr) {
+        kv_status s = KV_OK;
+        if (saa_band_launch<8>(plan, d_shift, h_shift, proj, out, 100 * 1024, &s) ||
+            saa_band_launch<4>(plan, d_shift, h_shift, proj, out, 160 * 1024, &s))
+            return s;
     }
     const int kb = 8;
     dim3 block(32, 8), grid((g.nu + 31) / 32, (g.nv + 7) / 8, (g.nz + kb - 1) / kb);

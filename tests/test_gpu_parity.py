@@ -270,6 +270,23 @@ def test_shift_and_add_staged_equals_direct(ctx):
         assert np.abs(staged - ref).max() <= 1e-6 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("geom", [
+    (16, 16, 16, 0.5, 0.5, 8.0, 5, 32, 300, 0.1, 0.1, 35.0),    # eight slices spread over 188 rows: four a block
+    (16, 16, 24, 0.5, 0.5, 6.0, 6, 32, 300, 0.1, 0.1, 35.0),    # the same with an even number of views
+    (16, 16, 13, 0.5, 0.5, 4.0, 3, 36, 90, 0.1, 0.1, 35.0),     # slices, rows and columns left over in the last blocks
+])
+def test_shift_and_add_block_shapes_equal_direct(ctx, geom):
+    """Block shapes of the staged kernel against the direct kernel (a detector that is not whole 16-byte units): the
+    same sums in the same order."""
+    g = linear_sweep(*geom)
+    rng = np.random.default_rng(3)
+    p = rng.standard_normal(g.proj_shape, dtype=np.float32)
+    gw = Geometry(g.nx, g.ny, g.nz, g.dx, g.dy, g.dz, g.nu + 1, g.nv, g.du, g.dv, g.src, g.det_origin, g.fulcrum_z)
+    pw = np.concatenate([p, np.ones((g.n_views, g.nv, 1), np.float32)], axis=2)
+    assert np.array_equal(engine.Plan(ctx, g, "exact").shift_and_add(p),
+                          engine.Plan(ctx, gw, "exact").shift_and_add(pw)[:, :, :g.nu])
+
+
 # ---------------------------------------------------------------- edges
 
 def test_device_buffers_match_host(ctx):
