@@ -643,12 +643,7 @@ extern "C" kv_status kv_fbp(kv_plan *plan, const float *proj, float *volume, int
     KV_TRY(stage_in(plan, volume, mem, &plan->d_vol32, plan->nvox, false, &vd));
     KV_TRY(ensure_sens(plan));
     KV_TRY(ensure(plan->ctx, &plan->d_ratio, plan->nproj * sizeof(float)));
-    float *filtered = nullptr;
-    KV_CHECK_CUDA(plan->ctx, cudaMallocAsync((void **)&filtered, plan->nproj * sizeof(float), plan->ctx->stream));
-    kv_status st = ramp_filter_launch(plan, pd, filtered, half_taps);
-    if (st == KV_OK) st = exact_prescale_launch(plan, filtered, plan->d_ratio);
-    cudaFreeAsync(filtered, plan->ctx->stream);
-    KV_TRY(st);
+    KV_TRY(ramp_filter_launch(plan, pd, static_cast<float *>(plan->d_ratio), half_taps));
     // volume = 0 + 1 * A^T(y) / A^T 1: the SART-mode update epilogue from zero
     KV_TRY(fill_launch(plan->ctx, vd, plan->nvox, 0.f));
     KV_TRY(exact_back_launch(plan, BACK_SART, BackArgs{plan->d_ratio, vd, plan->d_sens, 1.f}));

@@ -270,6 +270,7 @@ kv_status rc_back_slab_launch(kv_plan *plan, int mode, const float *proj, float 
 
 // shift-and-add; h_shift: the host copy of the [nz][P] shift table in d_shift
 kv_status saa_launch(kv_plan *plan, const int32_t *d_shift, const int32_t *h_shift, const float *proj, float *out);
+// ramp-filters the projections along v and scales them by the ray factor (EXACT tables of the plan)
 kv_status ramp_filter_launch(kv_plan *plan, const float *in, float *out, int half_taps);
 kv_status fill_launch(kv_ctx *ctx, float *p, size_t n, float v);
 kv_status convert_launch(kv_ctx *ctx, const float *in, void *out, size_t n, kv_storage s);

@@ -189,6 +189,19 @@ def test_exact_fbp_vs_fp64_oracle(ctx, gi, half_taps):
         plan.fbp(p, 257)
 
 
+@pytest.mark.parametrize("nu,nv,half_taps", [(37, 41, 1), (48, 65, 7), (48, 64, 8), (50, 130, 9), (36, 90, 256)])
+def test_fbp_tap_and_tile_edges(ctx, nu, nv, half_taps):
+    """Tap counts around the eight a thread takes at once, detectors of whole and broken 16-byte rows and of rows left
+    over in a block: the ramp in FP64 followed by the engine's own backprojection and sensitivity (a ray in the plane
+    between two voxel columns, as in the first geometry, goes to the other column in the oracle), at the bound of
+    test_exact_fbp_vs_fp64_oracle."""
+    g = linear_sweep(24, 20, 6, 0.7, 0.7, 1.3, 4, nu, nv, 0.5, 0.4, 18.0)
+    p = np.random.default_rng(8).random(g.proj_shape, dtype=np.float32)
+    plan = engine.Plan(ctx, g, "exact")
+    b, s = plan.back(O.ramp_filter_v(p, half_taps).astype(np.float32)), plan.sensitivity()
+    assert rel_l2(plan.fbp(p, half_taps), np.where(s > 0, b / np.where(s > 0, s, 1.0), 0.0)) < 1e-5
+
+
 def test_exact_sensitivity_vs_oracle(ctx):
     g = small_geoms()[0]
     plan = engine.Plan(ctx, g, "exact")
