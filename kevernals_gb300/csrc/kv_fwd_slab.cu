@@ -213,9 +213,12 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
         s_yt[threadIdx.x] = T.yt[(size_t)p * G.nv + v];
         s_yi[threadIdx.x] = T.yi[(size_t)p * G.nv + v];
     }
+    __shared__ int s_range[2];   // first and last slab whose box meets the volume
     if (threadIdx.x == 0) {
         for (int s = 0; s < A.stages; ++s) kvtma::mbar_init(&full[s], 1);
         kvtma::fence_mbar_init();
+        s_range[0] = A.nslab;
+        s_range[1] = -1;
     }
     __syncthreads();
 
@@ -233,9 +236,17 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
             box_origin(Xa, ia, Xb, ibb, s_yt[0], s_yi[0], s_yt[vb_local], s_yi[vb_local], s_hr[ks], s_hr[ke],
                        A.align, x0, y0, nxn, nyn);
             org[s] = make_int2(x0, y0);
+            if (x0 < G.nx && x0 + A.BX > 0 && y0 < G.ny && y0 + A.BY > 0) {
+                atomicMin(&s_range[0], s);
+                atomicMax(&s_range[1], s);
+            }
         }
     }
     __syncthreads();
+    // the slabs before and after read zeros only and add exact zeros: the rays
+    // of a detector wider than the volume's shadow skip them (256 x 256 x 64
+    // voxels under 15 views of 512 x 512: 324 -> 204 us)
+    const int s_begin = s_range[0], s_end = s_range[1] + 1;
     // thread 0: load the box of slab s into stage st
     auto issue = [&](int s, int st) {
         kvtma::fence_proxy_async_smem();
@@ -284,10 +295,10 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
     };
 
     if (threadIdx.x == 0)
-        for (int s = 0; s < A.stages && s < A.nslab; ++s) issue(s, s);
+        for (int s = 0; s < A.stages && s_begin + s < s_end; ++s) issue(s_begin + s, s);
     __syncthreads();
     int err = 0;
-    if (threadIdx.x < A.S * TV) err |= make_desc(0, 0);
+    if (s_begin < s_end && threadIdx.x < A.S * TV) err |= make_desc(s_begin, 0);
     __syncthreads();
 
     // ---- this lane's detector column
@@ -310,13 +321,13 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
 #pragma unroll
     for (int q = 0; q < R; ++q) acc[q][0] = acc[q][1] = wsum[q] = 0.f;
 
-    int s = 0;
-    for (; s < A.nslab; ++s) {
-        const int st = s % A.stages;
-        if (!kvtma::mbar_wait_bounded(&full[st], (uint32_t)(s / A.stages) & 1u, kWaitPolls)) err |= 1;
+    int s = s_begin;
+    for (; s < s_end; ++s) {
+        const int n = s - s_begin, st = n % A.stages;
+        if (!kvtma::mbar_wait_bounded(&full[st], (uint32_t)(n / A.stages) & 1u, kWaitPolls)) err |= 1;
         if (err == 0) {
             const unsigned char *box = reinterpret_cast<const unsigned char *>(boxes + (size_t)st * A.stage_elems);
-            const YDesc *dsc = desc + (s & 1) * A.S * TV;
+            const YDesc *dsc = desc + (n & 1) * A.S * TV;
             const int xoff = ib - org[s].x;
             const int kend = min(A.S, G.nz - s * A.S);
             for (int kk = 0; kk < kend; ++kk) {
@@ -351,16 +362,17 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
                 }
             }
         }
-        if (s + 1 < A.nslab && threadIdx.x < A.S * TV) err |= make_desc(s + 1, (s + 1) & 1);
+        if (s + 1 < s_end && threadIdx.x < A.S * TV) err |= make_desc(s + 1, (n + 1) & 1);
         if (__syncthreads_or(err)) break;
-        if (threadIdx.x == 0 && s + A.stages < A.nslab) issue(s + A.stages, st);
+        if (threadIdx.x == 0 && s + A.stages < s_end) issue(s + A.stages, st);
     }
-    if (s < A.nslab) {
+    if (s < s_end) {
         // failed: record, let the loads still in flight land, and leave
         if (err) atomicOr(A.status, err);
         if (threadIdx.x == 0)
-            for (int j = s; j < min(A.nslab, s + A.stages); ++j)
-                kvtma::mbar_wait_bounded(&full[j % A.stages], (uint32_t)(j / A.stages) & 1u, kWaitPolls);
+            for (int j = s; j < min(s_end, s + A.stages); ++j)
+                kvtma::mbar_wait_bounded(&full[(j - s_begin) % A.stages], (uint32_t)((j - s_begin) / A.stages) & 1u,
+                                         kWaitPolls);
         return;
     }
 
