@@ -326,6 +326,11 @@ void ctx_free(kv_ctx *ctx) {
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     for (cudaEvent_t e : ctx->copy_events) cudaEventDestroy(e);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+    for (cudaStream_t s : ctx->side_streams) {
+        cudaStreamSynchronize(s);
+        cudaStreamDestroy(s);
+    }
+    for (cudaEvent_t e : ctx->side_events) cudaEventDestroy(e);
     cudaFree(ctx->d_red);
     cudaFree(ctx->d_status);
     cudaStreamDestroy(ctx->own_stream);
@@ -427,6 +432,48 @@ extern "C" kv_status kv_ctx_timing_read(kv_ctx *ctx, char *buf, size_t buflen) {
 // Plans
 // ---------------------------------------------------------------------------
 
+namespace {
+// Launch shapes of a new plan's kernels (kv_plan_autotune can pick others).
+//
+// Slab forward: the shapes that fit, by the number of rounds of resident CTAs
+// times what a round takes (two CTAs of R = 8, three of R = 4 or 2 a SM;
+// rounds measured 1 : 0.78 : 0.54 on a full GPU).  Large detectors take R = 8
+// (512 x 512 x 15 views: 321 us, R = 4: 336); 96 x 128 x 30 views R = 4 (20.6
+// us, R = 8: 24.4), 56 x 64 x 7 views R = 2 (12.8, R = 8: 18.1).
+//
+// Backprojector: few blocks leave every warp a chain of all views at ~2.4 us a
+// view, so the views are split over the warps of a block (back_vs).  With 8
+// rows a thread and no split, 8 x 128 x 64 voxels, 49 views (32 blocks): 121
+// -> 24 us at 8 groups; 16 x 64 x 96, 30 views (48): 74 -> 25; 24 x 128 x 128,
+// 15 views (192): 41 -> 35 at 4; 41 x 187 x 213 (861) would lose, 112 -> 154
+// at 2, as warps on different views share no detector rows in L1.
+void default_shapes(kv_plan *plan) {
+    const kv_geometry &g = plan->g;
+    const int sms = plan->ctx->sm_count > 0 ? plan->ctx->sm_count : 1;
+    // (R, S, stages), rounds' cost
+    static const struct {
+        int R, S, stages, per_sm;
+        double round;
+    } shapes[] = {{8, 4, 2, 2, 1.0}, {4, 4, 3, 3, 0.78}, {4, 2, 3, 3, 0.95}, {2, 4, 3, 3, 0.54}, {2, 2, 2, 3, 0.8}};
+    double best = 1e300;
+    const bool padded = (size_t)g.nx * kv_storage_bytes(plan->storage) % 16 != 0;
+    FwdSlabCfg pick;
+    for (const auto &sh : shapes) {
+        const double ctas = (double)((g.nu + 31) / 32) * ((g.nv + 8 * sh.R - 1) / (8 * sh.R)) * g.n_views;
+        const double cost = std::ceil(ctas / (sms * sh.per_sm)) * sh.round;
+        FwdSlabCfg c;
+        if (cost >= best ||
+            !fwd_slab_fit(plan, sh.R, sh.S, sh.stages, fwd_slab_default_group(g.n_views), &c, nullptr, padded))
+            continue;
+        best = cost;
+        pick = c;
+    }
+    (padded ? plan->fpad : plan->fslab) = pick;
+    const long long blocks = (long long)g.nz * ((g.ny + 63) / 64) * ((g.nx + 31) / 32);
+    plan->back_vs = blocks * 2 <= sms ? 8 : (2 * blocks <= 3 * sms ? 4 : 1);
+}
+}  // namespace
+
 extern "C" kv_status kv_plan_create(kv_ctx *ctx, const kv_geometry *g, kv_family family,
                                     kv_storage storage, kv_plan **out) {
     if (ctx == nullptr || g == nullptr || out == nullptr) return KV_ERR_INVALID_ARG;
@@ -461,17 +508,7 @@ extern "C" kv_status kv_plan_create(kv_ctx *ctx, const kv_geometry *g, kv_family
     kv_status s = KV_OK;
     if (family == KV_FAMILY_EXACT) {
         s = exact_build_tables(plan, plan->src.data(), plan->det.data(), g->n_views, &plan->ex, &plan->hx);
-        // the slab-staged forward projector where the geometry suits it: the
-        // first shape of this list that fits (measured fastest first at the
-        // chest-DT geometry; kv_plan_autotune can pick another)
-        static const int shapes[][3] = {{8, 4, 2}, {4, 4, 3}, {4, 2, 3}, {2, 4, 3}, {2, 2, 2}};
-        for (const auto &sh : shapes) {
-            FwdSlabCfg c;
-            if (s == KV_OK && fwd_slab_fit(plan, sh[0], sh[1], sh[2], fwd_slab_default_group(g->n_views), &c, nullptr)) {
-                plan->fslab = c;
-                break;
-            }
-        }
+        if (s == KV_OK) default_shapes(plan);
     } else {
         size_t bytes = 3 * sizeof(float) * g->n_views;
         if (cudaMalloc((void **)&plan->d_src, bytes) != cudaSuccess ||
@@ -507,6 +544,8 @@ extern "C" kv_status kv_plan_destroy(kv_plan *plan) {
     cudaFree(plan->d_ratio);
     cudaFree(plan->d_vol32);
     cudaFree(plan->d_proj32);
+    cudaFree(plan->d_pad);
+    cudaFree(plan->d_rows);
     cudaFree(plan->d_sens);
     cudaFree(plan->d_shift);
     if (plan->graph_exec) cudaGraphExecDestroy(plan->graph_exec);
@@ -746,6 +785,34 @@ namespace {
 kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem,
                   kv_iter_cb cb, void *user);
 
+// The padded-row volume of a plan whose iterations use it; where it cannot be
+// had (memory, or a capture that began before the first solve) the plan takes
+// the one-thread-per-ray kernel.
+void ensure_pad(kv_plan *plan) {
+    if (plan->fpad.R == 0 || plan->d_pad != nullptr) return;
+    const size_t bytes = (size_t)plan->fpad.pitch * plan->g.ny * plan->g.nz * kv_storage_bytes(plan->storage);
+    if (stream_capturing(plan->ctx) || cudaMalloc(&plan->d_pad, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        plan->d_pad = nullptr;
+    }
+}
+
+// SART's row sums A 1 depend on the geometry alone: the first forward pass of
+// a plan's first SART solve stores them and later passes read them (a quarter
+// of the pass was their in-volume test).  Returns the mode of the next pass.
+FwdMode sart_mode(kv_plan *plan, FwdArgs &a) {
+    a.rows = plan->d_rows;
+    return plan->d_rows != nullptr && plan->rows_valid ? FWD_SART_ROWS : FWD_SART;
+}
+
+void ensure_rows(kv_plan *plan) {
+    if (plan->d_rows == nullptr &&
+        (stream_capturing(plan->ctx) || cudaMalloc((void **)&plan->d_rows, plan->nproj * sizeof(float)) != cudaSuccess)) {
+        cudaGetLastError();
+        plan->d_rows = nullptr;   // every pass forms them again
+    }
+}
+
 // Without a callback (and without tracing) the iteration loop is captured once
 // as a CUDA graph on the context's own stream and launched on the call's
 // stream; the executable graph is kept and relaunched while the buffers and
@@ -759,10 +826,12 @@ kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float 
     const bool same = plan->graph_exec != nullptr && plan->graph_p == p && plan->graph_x == x &&
                       plan->graph_iters == iters && plan->graph_mlem == (int)mlem && plan->graph_relax == relax &&
                       plan->graph_fb == plan->fwd_by && plan->graph_bb == plan->back_by &&
-                      plan->graph_slab == slab_key(plan->fslab) && plan->graph_br == plan->back_rows &&
-                      plan->graph_bs == plan->back_slices &&
+                      plan->graph_slab == slab_key(plan->fslab) + (slab_key(plan->fpad) << 1) && plan->graph_br == plan->back_rows &&
+                      plan->graph_bs == plan->back_slices && plan->graph_vs == plan->back_vs &&
+                      plan->graph_rows == (int)(!mlem && plan->rows_valid) &&
                       plan->graph_bst == plan->bstage.R * 16 + plan->bstage.stages;
     if (!same) {
+        const bool had_rows = plan->rows_valid;
         if (plan->graph_exec != nullptr) {
             KV_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             cudaGraphExecDestroy(plan->graph_exec);
@@ -793,12 +862,15 @@ kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float 
         plan->graph_relax = relax;
         plan->graph_fb = plan->fwd_by;
         plan->graph_bb = plan->back_by;
-        plan->graph_slab = slab_key(plan->fslab);
+        plan->graph_slab = slab_key(plan->fslab) + (slab_key(plan->fpad) << 1);
         plan->graph_br = plan->back_rows;
         plan->graph_bs = plan->back_slices;
+        plan->graph_vs = plan->back_vs;
+        plan->graph_rows = (int)(!mlem && had_rows);
         plan->graph_bst = plan->bstage.R * 16 + plan->bstage.stages;
     }
     KV_CHECK_CUDA(ctx, cudaGraphLaunch(plan->graph_exec, ctx->stream));
+    if (!mlem && plan->family == KV_FAMILY_EXACT && plan->d_rows != nullptr) plan->rows_valid = true;
     return KV_OK;
 }
 
@@ -807,15 +879,22 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
     kv_ctx *ctx = plan->ctx;
     const size_t es = kv_storage_bytes(plan->storage);
     KV_TRY(ensure(ctx, &plan->d_ratio, plan->nproj * es));
-    if (plan->family == KV_FAMILY_EXACT) KV_TRY(ensure_sens(plan));
+    if (plan->family == KV_FAMILY_EXACT) {
+        KV_TRY(ensure_sens(plan));
+        ensure_pad(plan);
+        if (!mlem) ensure_rows(plan);
+    }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(ctx->stream, &cs);
     if (cb == nullptr && !ctx->timing && iters >= 2 && cs == cudaStreamCaptureStatusNone)
         return iterate_graph(plan, p, x, iters, relax, mlem);
+    const bool had_rows = plan->rows_valid;
     for (int it = 0; it < iters; ++it) {
         if (plan->family == KV_FAMILY_EXACT) {
             FwdArgs fa{x, p, plan->d_ratio, cb ? ctx->d_red : nullptr, relax};
-            KV_TRY(exact_forward_launch(plan, plan->ex, plan->g.n_views, mlem ? FWD_MLEM : FWD_SART, fa));
+            fa.pad = plan->d_pad;
+            KV_TRY(exact_forward_launch(plan, plan->ex, plan->g.n_views, mlem ? FWD_MLEM : sart_mode(plan, fa), fa));
+            if (!mlem && plan->d_rows != nullptr) plan->rows_valid = true;
         } else if (cb) {
             KV_TRY(rc_forward_launch(plan, plan->d_src, plan->d_org, plan->g.n_views, RC_PLAIN, (const float *)x,
                                      nullptr, (float *)plan->d_ratio, relax));
@@ -838,6 +917,7 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
             KV_TRY(rc_back_launch(plan, mlem ? RC_MLEM : RC_ART, (const float *)plan->d_ratio, (float *)x));
         }
     }
+    if (cs != cudaStreamCaptureStatusNone) plan->rows_valid = had_rows;   // captured, not run
     return KV_OK;
 }
 
@@ -854,9 +934,14 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
 // ratio) and on slices [z0, z0 + n) (backprojection + update).
 kv_status update_forward_views(kv_plan *plan, bool mlem, const float *pd, const float *xd, float relax, int v0,
                                int n) {
-    if (plan->family == KV_FAMILY_EXACT)
-        return exact_forward_views_launch(plan, v0, n, mlem ? FWD_MLEM : FWD_SART,
-                                          FwdArgs{xd, pd, plan->d_ratio, nullptr, relax});
+    if (plan->family == KV_FAMILY_EXACT) {
+        FwdArgs fa{xd, pd, plan->d_ratio, nullptr, relax};
+        fa.pad = plan->d_pad;
+        fa.pad_ready = v0 > 0;   // view chunks of one volume, the first from view 0
+        KV_TRY(exact_forward_views_launch(plan, v0, n, mlem ? FWD_MLEM : sart_mode(plan, fa), fa));
+        if (!mlem && plan->d_rows != nullptr && v0 + n == plan->g.n_views) plan->rows_valid = true;   // chunks in order
+        return KV_OK;
+    }
     const size_t off = (size_t)v0 * plan->g.nu * plan->g.nv;
     return rc_forward_launch(plan, plan->d_src + 3 * (size_t)v0, plan->d_org + 3 * (size_t)v0, n,
                              mlem ? RC_MLEM : RC_ART, xd, pd + off, (float *)plan->d_ratio + off, relax);
@@ -903,7 +988,11 @@ kv_status driver_overlapped(kv_plan *plan, const float *proj, float *volume, int
     KV_TRY(ensure(ctx, &plan->d_proj32, plan->nproj * sizeof(float)));
     KV_TRY(ensure(ctx, &plan->d_vol32, plan->nvox * sizeof(float)));
     KV_TRY(ensure(ctx, &plan->d_ratio, plan->nproj * sizeof(float)));
-    if (plan->family == KV_FAMILY_EXACT) KV_TRY(ensure_sens(plan));
+    if (plan->family == KV_FAMILY_EXACT) {
+        KV_TRY(ensure_sens(plan));
+        ensure_pad(plan);
+        if (!mlem) ensure_rows(plan);
+    }
     KV_TRY(ensure_copy_stream(ctx));
     return sync_both(ctx, overlapped_body(plan, proj, volume, iters, relax, mlem));
 }
@@ -994,20 +1083,20 @@ extern "C" kv_status kv_batch_mlem(kv_ctx *ctx, int n, kv_plan *const *plans, co
         if (pl->family != KV_FAMILY_EXACT || pl->storage != KV_STORAGE_F32)
             return kv_fail(ctx, KV_ERR_UNSUPPORTED, "kv_batch_mlem: EXACT / FP32 plans only (plan %d)", i);
     }
-    const int by = plans[0]->fwd_by, bb = plans[0]->back_by;
     std::vector<const float *> pd(n);
     std::vector<float *> xd(n);
     for (int i = 0; i < n; ++i) {
         kv_plan *pl = plans[i];
         KV_TRY(ensure(ctx, &pl->d_ratio, pl->nproj * sizeof(float)));
         KV_TRY(ensure_sens(pl));
+        ensure_pad(pl);
         float *a, *b;
         KV_TRY(stage_in(pl, projections[i], mem, &pl->d_proj32, pl->nproj, true, &a));
         KV_TRY(stage_in(pl, volumes[i], mem, &pl->d_vol32, pl->nvox, true, &b));
         pd[i] = a;
         xd[i] = b;
     }
-    if (iterations > 0) KV_TRY(exact_batch_mlem_launch(ctx, n, plans, pd.data(), xd.data(), iterations, relax, by, bb));
+    if (iterations > 0) KV_TRY(exact_batch_mlem_launch(ctx, n, plans, pd.data(), xd.data(), iterations, relax));
     for (int i = 0; i < n; ++i) KV_TRY(stage_out(plans[i], volumes[i], mem, xd[i], plans[i]->nvox));
     return KV_OK;
 }
@@ -1051,7 +1140,7 @@ extern "C" kv_status kv_plan_set_slab(kv_plan *plan, int rays_per_thread, int sl
     if (plan->family != KV_FAMILY_EXACT)
         return kv_fail(plan->ctx, KV_ERR_UNSUPPORTED, "the slab forward projector is an EXACT-family kernel");
     if (rays_per_thread == 0) {
-        plan->fslab = FwdSlabCfg{};
+        plan->fslab = plan->fpad = FwdSlabCfg{};
         return KV_OK;
     }
     FwdSlabCfg c;
@@ -1106,6 +1195,7 @@ extern "C" kv_status kv_plan_set_back_shape(kv_plan *plan, int rows_per_thread, 
         return kv_fail(plan->ctx, KV_ERR_INVALID_ARG,
                        "gather backprojector shape must be rows 0, (1, 1), (2, 1), (2, 2), (4, 1), (4, 2) or (8, 1)");
     if (rows_per_thread == 0) slices_per_thread = 1;
+    plan->back_vs = 1;   // a shape asked for is the plain one
     plan->back_rows = rows_per_thread;
     plan->back_slices = slices_per_thread;
     return KV_OK;

@@ -34,6 +34,7 @@ struct StageArgs {
     uint32_t stage_bytes;               // bytes one box load delivers: BU * BV * 4
     uint32_t org_off;                   // byte offset of the per-view patch origins
     int *status;                        // error bits (0: fine)
+    int vs;                          // view groups of the sums
 };
 
 // The candidate detector indices along one axis of the voxels lo .. hi of a
@@ -142,12 +143,24 @@ __global__ void __launch_bounds__(kThreads) exact_back_stage_kernel(const __grid
     if (threadIdx.x == 0)
         for (int p = 0; p < A.stages && p < G.n_views; ++p) issue(p, p);
 
-    float acc[R];
+    // sums by view groups, added in order, where the plan's gather kernel forms them so (A.vs groups; 1: one sum)
+    float acc[R], total[R];
 #pragma unroll
-    for (int q = 0; q < R; ++q) acc[q] = 0.f;
+    for (int q = 0; q < R; ++q) acc[q] = total[q] = 0.f;
     int err = 0;
-    int p = 0;
+    int p = 0, group = 0;
+    auto fold = [&] {
+        while (group < A.vs && p == (group + 1) * G.n_views / A.vs) {
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                total[q] = group == 0 ? acc[q] : total[q] + acc[q];
+                acc[q] = 0.f;
+            }
+            ++group;
+        }
+    };
     for (; p < G.n_views; ++p) {
+        fold();
         const int st = p % A.stages;
         if (!kvtma::mbar_wait_bounded(&full[st], (uint32_t)(p / A.stages) & 1u, kWaitPolls)) err |= 8;
         const int4 o = org[p];
@@ -230,6 +243,7 @@ __global__ void __launch_bounds__(kThreads) exact_back_stage_kernel(const __grid
                 kvtma::mbar_wait_bounded(&full[j % A.stages], (uint32_t)(j / A.stages) & 1u, kWaitPolls);
         return;
     }
+    fold();
     if (!live_i) return;
     float *vol = static_cast<float *>(a.vol);
 #pragma unroll
@@ -237,7 +251,7 @@ __global__ void __launch_bounds__(kThreads) exact_back_stage_kernel(const __grid
         const int j = jw + 8 * q;
         if (j >= G.ny) continue;
         const size_t idx = ((size_t)k * G.ny + j) * G.nx + i;
-        const float b = acc[q];
+        const float b = total[q];
         if (mode == BACK_PLAIN) {
             vol[idx] = b;
         } else if (mode == BACK_MLEM) {
@@ -335,6 +349,7 @@ kv_status back_stage_launch(kv_plan *plan, BackMode mode, const BackArgs &a, int
     A.stage_bytes = (uint32_t)c.BU * c.BV * sizeof(float);
     A.org_off = L.org_off;
     A.status = plan->ctx->d_status;
+    A.vs = plan->back_rows == 8 ? plan->back_vs : 1;
     const ExGeom G{g.nx, g.ny, g.nz, g.nu, g.nv, n_views};
     dim3 grid(nzs, (g.ny + 8 * c.R - 1) / (8 * c.R), (g.nx + 31) / 32);
     const void *fn = c.R == 8 ? (const void *)exact_back_stage_kernel<8> : (const void *)exact_back_stage_kernel<4>;

@@ -394,8 +394,9 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
         } else if (MODE == FWD_MLEM) {
             const float r = qv > 0.f ? a.relax * pm / qv : 0.f;
             Store<ProjT>::st(out + ray, r * ls);
-        } else if (MODE == FWD_SART) {
-            const float rows = wsum[q] * ls;
+        } else if (MODE == FWD_SART || MODE == FWD_SART_ROWS) {
+            const float rows = MODE == FWD_SART ? wsum[q] * ls : __ldg(a.rows + ray);
+            if (MODE == FWD_SART && a.rows != nullptr) a.rows[ray] = rows;
             const float r = rows > 0.f ? (pm - qv) / rows : 0.f;
             Store<ProjT>::st(out + ray, r * ls);
         }
@@ -431,6 +432,18 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
             partials[3 * (size_t)blockIdx.x + 2] = r2;
         }
     }
+}
+
+// dst[z][y][0 .. nx) = src[z][y][..], rows `pitch` elements apart (what lies between is never read: the tensor map
+// ends the row at nx)
+template <typename T>
+__global__ void __launch_bounds__(256) pad_rows_kernel(const T *__restrict__ src, T *__restrict__ dst, int nx, int ny,
+                                                       int nz, int pitch) {
+    for (int z = blockIdx.y; z < nz; z += gridDim.y)
+        for (int y = blockIdx.x * 8 + threadIdx.y; y < ny; y += gridDim.x * 8) {
+            const size_t row = (size_t)z * ny + y;
+            for (int x = threadIdx.x; x < nx; x += 32) dst[row * pitch + x] = src[row * nx + x];
+        }
 }
 
 // Dynamic shared memory layout of one CTA (byte offsets from the first
@@ -470,6 +483,7 @@ kv_status slab_launch_r(kv_plan *plan, const CUtensorMap &map, const ExGeom &G, 
     case FWD_MLEM: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_MLEM, R>; break;
     case FWD_SART: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_SART, R>; break;
     case FWD_RESID: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_RESID, R>; break;
+    case FWD_SART_ROWS: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_SART_ROWS, R>; break;
     }
     KV_CHECK_CUDA(plan->ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     LaunchTimer lt(plan->ctx, "exact_fwd");
@@ -478,6 +492,7 @@ kv_status slab_launch_r(kv_plan *plan, const CUtensorMap &map, const ExGeom &G, 
     case FWD_MLEM: fwd_slab_kernel<VolT, ProjT, FWD_MLEM, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
     case FWD_SART: fwd_slab_kernel<VolT, ProjT, FWD_SART, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
     case FWD_RESID: fwd_slab_kernel<VolT, ProjT, FWD_RESID, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
+    case FWD_SART_ROWS: fwd_slab_kernel<VolT, ProjT, FWD_SART_ROWS, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
     }
     KV_CHECK_LAUNCH(plan->ctx, "fwd_slab_kernel");
     return KV_OK;
@@ -489,7 +504,8 @@ kv_status slab_launch_r(kv_plan *plan, const CUtensorMap &map, const ExGeom &G, 
 // Host side
 // ---------------------------------------------------------------------------
 
-bool fwd_slab_fit(const kv_plan *plan, int R, int S, int stages, int group, FwdSlabCfg *out, std::string *why) {
+bool fwd_slab_fit(const kv_plan *plan, int R, int S, int stages, int group, FwdSlabCfg *out, std::string *why,
+                  bool padded) {
     const kv_geometry &g = plan->g;
     const ExactHostTables &H = plan->hx;
     const int es = (int)kv_storage_bytes(plan->storage);
@@ -503,7 +519,7 @@ bool fwd_slab_fit(const kv_plan *plan, int R, int S, int stages, int group, FwdS
     if (stages < 2 || stages > kMaxStages) return no("stage count out of range");
     if (group < 1) return no("view group must be positive");
     if (kvtma::encoder() == nullptr) return no("cuTensorMapEncodeTiled is not available");
-    if (((size_t)g.nx * es) % 16 != 0) return no("volume rows are not a whole number of 16-byte units");
+    if (!padded && ((size_t)g.nx * es) % 16 != 0) return no("volume rows are not a whole number of 16-byte units");
     if (H.xt.size() != (size_t)g.n_views * g.nu || H.yt.size() != (size_t)g.n_views * g.nv)
         return no("host tables missing");
     for (const float4 &x : H.xt)
@@ -546,6 +562,7 @@ bool fwd_slab_fit(const kv_plan *plan, int R, int S, int stages, int group, FwdS
     c.BX = bx;
     c.BY = by;
     c.smem = L.total;
+    c.pitch = (g.nx + align - 1) / align * align;
     *out = c;
     return true;
 }
@@ -555,17 +572,27 @@ int fwd_slab_default_group(int n_views) {
     return (n_views + groups - 1) / groups;
 }
 
-size_t fwd_slab_blocks(const kv_plan *plan, int n_views) {
-    const FwdSlabCfg &c = plan->fslab;
+size_t fwd_slab_blocks(const kv_plan *plan, const FwdSlabCfg &c, int n_views) {
     const int TV = 8 * c.R;
     return (size_t)((plan->g.nu + 31) / 32) * ((plan->g.nv + TV - 1) / TV) * n_views;
 }
 
-kv_status fwd_slab_launch(kv_plan *plan, const ExactTables &t, int P, FwdMode mode, const FwdArgs &a,
-                          double *partials) {
-    const FwdSlabCfg &c = plan->fslab;
+kv_status fwd_slab_launch(kv_plan *plan, const FwdSlabCfg &c, const ExactTables &t, int P, FwdMode mode,
+                          const FwdArgs &args, double *partials) {
     const kv_geometry &g = plan->g;
     const int es = (int)kv_storage_bytes(plan->storage);
+    FwdArgs a = args;
+    if (c.pitch != g.nx) {
+        // volume rows that are not whole 16-byte units: TMA reads a copy with padded rows
+        if (!a.pad_ready) {
+            LaunchTimer lt(plan->ctx, "pad_rows");
+            const dim3 block(32, 8), grid((unsigned)std::min(g.ny, 65535) / 8 + 1, (unsigned)std::min(g.nz, 65535));
+            if (es == 4) pad_rows_kernel<<<grid, block, 0, plan->ctx->stream>>>(static_cast<const uint32_t *>(a.vol), static_cast<uint32_t *>(a.pad), g.nx, g.ny, g.nz, c.pitch);
+            else pad_rows_kernel<<<grid, block, 0, plan->ctx->stream>>>(static_cast<const uint16_t *>(a.vol), static_cast<uint16_t *>(a.pad), g.nx, g.ny, g.nz, c.pitch);
+            KV_CHECK_LAUNCH(plan->ctx, "pad_rows_kernel");
+        }
+        a.vol = a.pad;
+    }
     if (reinterpret_cast<uintptr_t>(a.vol) % 16 != 0)
         return kv_fail(plan->ctx, KV_ERR_INVALID_ARG, "volume buffer is not 16-byte aligned");
     CUtensorMap map;
@@ -573,7 +600,7 @@ kv_status fwd_slab_launch(kv_plan *plan, const ExactTables &t, int P, FwdMode mo
                                    : plan->storage == KV_STORAGE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                                      : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     cuuint64_t dims[3] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
-    cuuint64_t strides[2] = {(cuuint64_t)g.nx * es, (cuuint64_t)g.nx * g.ny * es};
+    cuuint64_t strides[2] = {(cuuint64_t)c.pitch * es, (cuuint64_t)c.pitch * g.ny * es};
     cuuint32_t box[3] = {(cuuint32_t)c.BX, (cuuint32_t)c.BY, (cuuint32_t)c.S};
     cuuint32_t estr[3] = {1, 1, 1};
     if (kvtma::encoder()(&map, dt, 3, const_cast<void *>(a.vol), dims, strides, box, estr,

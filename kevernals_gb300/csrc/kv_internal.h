@@ -41,6 +41,9 @@ struct kv_ctx {
     // the last backprojection (created on first use)
     cudaStream_t copy_stream = nullptr;
     std::vector<cudaEvent_t> copy_events;
+    // batched solves: side streams and their join events (created on first use)
+    std::vector<cudaStream_t> side_streams;
+    std::vector<cudaEvent_t> side_events;
 };
 
 // Brackets one kernel launch with CUDA events on the context stream when the
@@ -92,6 +95,7 @@ struct FwdSlabCfg {
     int group = 0;      // consecutive views launched together (L2 reuse)
     int BX = 0, BY = 0; // box extent in voxels
     size_t smem = 0;    // dynamic shared memory per CTA
+    int pitch = 0;      // elements from one volume row to the next (nx rounded up to 16 bytes)
 };
 
 // Shape of the TMA-staged EXACT backprojector (kv_back_stage.cu, FP32
@@ -115,6 +119,8 @@ struct kv_plan {
     ExactTables ex;                  // EXACT family
     ExactHostTables hx;              // host copies of ex
     FwdSlabCfg fslab;                // slab forward projector (R == 0: not used)
+    FwdSlabCfg fpad;                 // the same on a copy of the volume with padded rows, in the iterative drivers,
+                                     // where the volume's own rows are not whole 16-byte units (R == 0: not used)
     BackStageCfg bstage;             // staged backprojector (R == 0: not used)
     float *d_src = nullptr;          // RC family: [P][3] sources (float3 layout)
     float *d_org = nullptr;          // RC family: [P][3] detector origins
@@ -126,6 +132,9 @@ struct kv_plan {
     void *d_ratio = nullptr;         // forward output / ratio in storage type
     float *d_vol32 = nullptr;        // float32 staging for host I/O
     float *d_proj32 = nullptr;
+    void *d_pad = nullptr;           // volume with padded rows (fpad)
+    float *d_rows = nullptr;         // A 1, SART's row sums (EXACT)
+    bool rows_valid = false;
     double *d_sens = nullptr;        // A^T 1 in FP64 (EXACT)
     bool sens_valid = false;
     int32_t *d_shift = nullptr;      // shift-and-add table [nz][P]
@@ -135,6 +144,7 @@ struct kv_plan {
     int back_by = 8;                 // backprojector block = 32 x back_by voxels (one voxel per thread)
     int back_rows = 8;               // voxel rows per thread of the gather backprojector (0: one voxel per thread)
     int back_slices = 1;             // slices per thread of the gather backprojector
+    int back_vs = 1;                 // view groups of a block (with 8 rows, 1 slice; chosen by the plan only)
 
     // captured iteration loop (kv_mlem / kv_sart without callback), reused
     // while the buffers and parameters are the same
@@ -143,7 +153,7 @@ struct kv_plan {
     const void *graph_x = nullptr;
     int graph_iters = 0, graph_mlem = 0, graph_fb = 0, graph_bb = 0;
     long long graph_slab = 0;
-    int graph_br = 0, graph_bs = 0, graph_bst = 0;
+    int graph_br = 0, graph_bs = 0, graph_bst = 0, graph_vs = 0, graph_rows = 0;
     float graph_relax = 0.f;
 };
 
@@ -152,7 +162,7 @@ struct kv_plan {
 void kv_ctx_release_ref(kv_ctx *ctx);
 
 kv_status exact_batch_mlem_launch(kv_ctx *ctx, int n, kv_plan *const *plans, const float *const *p,
-                                  float *const *x, int iters, float relax, int by, int bb);
+                                  float *const *x, int iters, float relax);
 kv_status exact_autotune(kv_plan *plan);
 
 // ---------------------------------------------------------------------------
@@ -221,7 +231,8 @@ enum FwdMode : int {
     FWD_PLAIN = 0,    // out = A x
     FWD_MLEM = 1,     // out = Ls * (q > 0 ? relax * p / q : 0)      (pre-scaled ratio)
     FWD_SART = 2,     // out = Ls * (rowsum > 0 ? (p - q) / rowsum : 0)
-    FWD_RESID = 3     // no output; FP64 residual / log-likelihood only
+    FWD_RESID = 3,    // no output; FP64 residual / log-likelihood only
+    FWD_SART_ROWS = 4 // FWD_SART with the row sums read from `rows`
 };
 // Epilogue modes of the EXACT backprojector.
 enum BackMode : int {
@@ -236,6 +247,9 @@ struct FwdArgs {
     void *out;             // ProjT [P][nv][nu]
     double *red;           // FP64 reductions {sum (q-p)^2, sum p^2, sum p log q - q} or null
     float relax;
+    float *rows = nullptr;    // [P][nv][nu] row sums: stored by FWD_SART (null: not), read by FWD_SART_ROWS
+    void *pad = nullptr;   // the plan's d_pad where the caller owns the plan's workspaces, else null: no padded slab
+    bool pad_ready = false;   // d_pad already holds vol
 };
 struct BackArgs {
     const void *yp;        // ProjT [P][nv][nu], scaled by the ray factor Ls
@@ -283,11 +297,12 @@ kv_status phantom_launch(kv_ctx *ctx, int nx, int ny, int nz, float dx, float dy
 // ray and slice, boxes within 256 voxels and the shared-memory budget) and
 // sizes its boxes for (R, S, stages, group); fwd_slab_launch runs it for
 // views [0, n_views) of the tables `t` (the plan's own, possibly offset).
-bool fwd_slab_fit(const kv_plan *plan, int R, int S, int stages, int group, FwdSlabCfg *out, std::string *why);
+bool fwd_slab_fit(const kv_plan *plan, int R, int S, int stages, int group, FwdSlabCfg *out, std::string *why,
+                  bool padded = false);
 int fwd_slab_default_group(int n_views);
-size_t fwd_slab_blocks(const kv_plan *plan, int n_views);
-kv_status fwd_slab_launch(kv_plan *plan, const ExactTables &t, int n_views, FwdMode mode, const FwdArgs &a,
-                          double *partials);
+size_t fwd_slab_blocks(const kv_plan *plan, const FwdSlabCfg &c, int n_views);
+kv_status fwd_slab_launch(kv_plan *plan, const FwdSlabCfg &c, const ExactTables &t, int n_views, FwdMode mode,
+                          const FwdArgs &a, double *partials);
 
 // TMA-staged EXACT backprojector (kv_back_stage.cu): back_stage_fit checks
 // that the plan suits it (FP32 storage, 16-byte detector rows, every

@@ -225,6 +225,59 @@ def test_exact_mlem_sart_vs_fp64_oracle(ctx):
     assert rel_l2(x, xo) < 1e-5
 
 
+@pytest.mark.parametrize("storage", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("nx", [33, 34, 36, 39])
+def test_padded_rows_match_the_ray_kernel(ctx, storage, nx):
+    """Iterations on volumes whose rows are not whole 16-byte units (the slab projector on a padded copy) against the
+    same iterations with the one-thread-per-ray kernel: the same lengths summed in another order, so FP32 iterates
+    agree to a few roundings and 16-bit ones to a few ulps of their storage."""
+    g = linear_sweep(nx, 29, 7, 0.7, 0.45, 1.3, 4, 37, 41, 0.55, 0.35, 22.0)
+    p = O.exact_forward(g, phantom_for(g).astype(np.float64)).astype(np.float32)
+    tol = {"f32": 1e-6, "bf16": 2 ** -7, "f16": 2 ** -10}[storage]
+    for sart in (False, True):
+        xs = []
+        for ray in (False, True):
+            plan = engine.Plan(ctx, g, "exact", storage)
+            if ray:
+                plan.set_slab(0)
+            x = np.full(g.volume_shape, 0.0 if sart else 1.0, np.float32)
+            (plan.sart if sart else plan.mlem)(p, x, 3)
+            xs.append(x)
+        assert rel_l2(xs[0], xs[1]) < tol
+
+
+@pytest.mark.parametrize("geom", [
+    (24, 20, 6, 0.5, 0.5, 1.0, 3, 40, 36, 0.4, 0.4, 15.0),      # fewer views than groups
+    (33, 9, 3, 0.5, 0.5, 1.0, 8, 40, 36, 0.4, 0.4, 15.0),       # one view a group, one row left over
+    (64, 65, 40, 0.5, 0.5, 1.0, 13, 96, 96, 0.4, 0.4, 15.0),    # four groups
+])
+def test_back_view_groups(ctx, geom):
+    """A small plan's backprojector, whose warps share the views, against the plain shape: the same terms in groups."""
+    g = linear_sweep(*geom)
+    y = np.random.default_rng(6).random(g.proj_shape, dtype=np.float32)
+    plain = engine.Plan(ctx, g, "exact")
+    plain.set_back_shape(8, 1)
+    assert rel_l2(engine.Plan(ctx, g, "exact").back(y), plain.back(y)) < 1e-6
+
+
+def test_sart_row_sums_are_kept(ctx):
+    """The second solve of a plan reads the row sums that the first stored: the same iterates, bit for bit, on device
+    and host buffers, and equal to a fresh plan's."""
+    torch = pytest.importorskip("torch")
+    for g in small_geoms():
+        p = O.exact_forward(g, phantom_for(g).astype(np.float64)).astype(np.float32)
+        plan, pd, xs = engine.Plan(ctx, g, "exact"), torch.from_numpy(p).cuda(), []
+        for n in (1, 3, 3, 1):
+            x = torch.zeros(g.volume_shape, device="cuda")
+            plan.sart(pd, x, n, 0.5)
+            h = np.zeros(g.volume_shape, np.float32)
+            engine.Plan(ctx, g, "exact").sart(p, h, n, 0.5)
+            assert np.array_equal(x.cpu().numpy(), h)
+            h2 = np.zeros(g.volume_shape, np.float32)
+            plan.sart(p, h2, n, 0.5)
+            assert np.array_equal(h2, h)
+
+
 def test_exact_residual_matches_numpy(ctx):
     g = small_geoms()[1]
     truth = phantom_for(g)
