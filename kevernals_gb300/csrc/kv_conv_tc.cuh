@@ -37,17 +37,16 @@
 // Measured on a GB300, against a kernel that loaded one tile per tap and
 // issued one N = Cout MMA per tap and 16 channels: 32+16 -> 16 channels at
 // 128 x 256 x 128 voxels 1434 -> 176 us (990 TFLOP/s); the thirteen layers of
-// the U-Net at 128 x 512 x 512 voxels 31.9 -> 5.4 ms, forward and
-// backward-data at 128 x 256 x 128 8.1 -> 1.9 ms.
+// the U-Net at 128 x 512 x 512 voxels 31.9 -> 4.6 ms, forward and
+// backward-data at 128 x 256 x 128 8.1 -> 1.7 ms.
 //
-// Warp roles (352 threads): warp 0 issues the TMA loads of the planes and of
-// streamed weights, warps 1 and 10 issue the MMAs of the even and
-// the odd sub-tiles (an MMA takes ~45 cycles and a sub-tile's waits, commit and
-// address set-up ~240: two issuers keep the tensor pipe fed; one took 284 us
-// where two take 203 on the layer below; warp 1 owns the TMEM allocation),
-// warps 2-9 drain the accumulators (each warp
-// its 32 TMEM lanes = 32 voxels; two sets of four warps take the sub-tiles in
-// turn), add the bias, apply ReLU or the caller's mask, convert to BF16 and
+// Warp roles: warp 0 issues the TMA loads of the planes and of streamed
+// weights; two or four warps issue the MMAs, each its sub-tiles in turn (an MMA
+// takes ~45 cycles and a sub-tile's waits, commit and address set-up ~240, so
+// one issuer cannot keep the tensor pipe fed; warp 1 owns the TMEM allocation);
+// two or four sets of four warps drain the accumulators (each warp its 32 TMEM
+// lanes = 32 voxels; the sets take the sub-tiles in turn), add the bias, apply
+// ReLU or the caller's mask, convert to BF16 and
 // store.  The CTA is persistent over its share of (column, plane) units.
 // Every wait on an mbarrier is bounded: on timeout the thread records an
 // error code, raises the CTA's abort flag and every role winds down, so a
@@ -64,9 +63,16 @@
 
 namespace convtc {
 
-constexpr int kThreads = 352;
-constexpr int kIssuers = 2;       // warps that issue MMAs
-constexpr int kEpilogueSets = 2;  // sets of four warps that drain accumulators
+// Warps by channel group: MMA issuers and sets of four warps that drain
+// accumulators.  With 16 channels a sub-tile's nine MMAs take ~400 cycles and
+// draining it ~1400, so four sets (16 -> 16 channels at 64 x 512 x 512 voxels:
+// two sets and four sub-tiles 318 us, four sets and eight sub-tiles 278);
+// streamed weights of 32 channels want an issuer a sub-tile (96 -> 32 at 64 x 256 x 256: two 1020, four 840
+// us); with 64 channels the MMAs are long and registers are short.
+__host__ __device__ constexpr int issuers(int cg) { return cg == 32 ? 4 : 2; }
+__host__ __device__ constexpr int drain_sets(int cg) { return cg <= 16 ? 4 : 2; }
+__host__ __device__ constexpr int threads(int cg) { return (1 + issuers(cg) + 4 * drain_sets(cg)) * 32; }
+constexpr int kMaxIssuers = 4;
 constexpr int kTileM = 128;
 constexpr int kSeg = 16;          // channels per segment: one K step, one 32-byte row per voxel
 constexpr int kRow = kSeg * 2;    // bytes of a row
@@ -221,13 +227,14 @@ __device__ __forceinline__ void issue_taps(uint32_t t0, uint32_t t1, uint32_t a,
 }
 
 template <int CG>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(threads(CG), 1)
     conv3_march_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
                        const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b2,
                        const __grid_constant__ Params P) {
+    constexpr int kIssuers = issuers(CG), kSets = drain_sets(CG);
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_full[kMaxT], acc_empty[kMaxT],
-        b_full[kMaxChunks], b_empty[kMaxChunks], drain_bar[kIssuers];
+        b_full[kMaxChunks], b_empty[kMaxChunks], drain_bar[kMaxIssuers];
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_flag;
     __shared__ unsigned long long issued_sh, b_issued_sh;   // planes / pieces of weights loaded by TMA
@@ -265,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_sh;
-    if (warp >= 2 && warp < 6) {   // every accumulator starts at zero
+    if (warp > kIssuers && warp <= kIssuers + 4) {   // every accumulator starts at zero
         for (uint32_t c = 0; c < P.tmem_cols; c += 16) tc_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c);
         tc_wait_st();
         tc_fence_before();
@@ -329,9 +336,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 u += ze - zs;
             }
         }
-    } else if (warp == 1 || warp == 10) {
+    } else if (warp <= kIssuers) {
         // ---------------------------------------------------------- MMA issuers
-        const int issuer = warp == 1 ? 0 : 1;
+        const int issuer = warp - 1;
         // The whole warp runs this role converged (every wait's outcome is agreed on by a vote) and one elected
         // thread issues: the operands of tcgen05.mma live in uniform registers, and values computed in a
         // one-thread branch would have to be moved there MMA by MMA.
@@ -442,9 +449,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         volatile int never = 0;
         mbar_wait(&drain_bar[issuer], 0, &never, P.status, 6);
     } else {
-        // ---------------------------------------------------------- epilogue (warps 2-9)
+        // ---------------------------------------------------------- epilogue
         const int quarter = warp & 3;                  // TMEM lanes 32*quarter .. +31
-        const int set = (warp - 2) >> 2;
+        const int set = (warp - 1 - kIssuers) >> 2;
+        float hw[CG == 16 ? 17 : 1];                   // the output layer's weights and bias
+        if (CG == 16 && P.head.y != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 17; ++j) hw[j] = __ldg(j < 16 ? P.head.w + j : P.head.b);
+        }
         uint32_t plane_phase = 0;
         bool ok = true;
         for (long long u = u_begin; u < u_end && ok;) {
@@ -452,7 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int ze = (int)(u_end - u < P.D - zs ? zs + (u_end - u) : P.D);
             const int x0 = (col % P.tiles_x) * P.BW, y0 = (col / P.tiles_x) * P.BY;
             for (int z = max(zs - 1, 0); z <= min(ze, P.D - 1) && ok; ++z) {
-                for (int t = set; t < P.T; t += kEpilogueSets) {
+                for (int t = set; t < P.T; t += kSets) {
                     const bool got = mbar_wait(&acc_full[t], plane_phase, &abort_flag, P.status, 4);
                     if (!__all_sync(0xffffffffu, got)) { ok = false; break; }   // warp-uniform: tcgen05.ld is .sync.aligned
                     tc_fence_after();
@@ -506,12 +518,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                                     d4[1] = reinterpret_cast<const uint4 *>(r)[1];
                                 }
                                 if (CG == 16 && P.head.y != nullptr) {
-                                    float h = __ldg(P.head.b);
+                                    float h = hw[16];
 #pragma unroll
                                     for (int j = 0; j < 8; ++j) {
                                         const float2 f = __bfloat1622float2(r[j]);
-                                        h = fmaf(__ldg(P.head.w + 2 * j), f.x, h);
-                                        h = fmaf(__ldg(P.head.w + 2 * j + 1), f.y, h);
+                                        h = fmaf(hw[2 * j], f.x, h);
+                                        h = fmaf(hw[2 * j + 1], f.y, h);
                                     }
                                     const size_t vox = o / 16;
                                     P.head.y[vox] = __ldg(P.head.x + vox) + h;
@@ -607,9 +619,11 @@ inline int channel_group(int N) {
 // dz groups takes max(shared-memory reads of A and B at 128 B a cycle, n * CG /
 // 2 cycles of arithmetic), measured 46 cycles at CG = 16, n = 3; loads come at
 // about 32 B a cycle and SM out of L2; waits, commits and address set-up cost
-// about 300 cycles a sub-tile (resident weights) or a piece of weights, shared
-// by two issuers; draining a sub-tile takes about 300 + 10 CG cycles a set of
-// warps.  A single plane buffer exposes its load.
+// about 300 cycles a sub-tile (resident weights) or a piece of weights;
+// draining a sub-tile takes about 1200 + 10 CG cycles from its last MMA to the
+// next plane's first, so few sub-tiles leave the pipe idle (16 -> 16 channels
+// at 64 x 512 x 512 voxels: four 318 us, eight 278).  A single plane buffer
+// exposes its load.
 inline bool plan_shape(Params &P, int CG, int sm_count, int *grid, size_t *smem) {
     const uint32_t budget = 224u * 1024u;
     const int max_t = std::min(kMaxT, 512 / (3 * CG));
@@ -653,15 +667,18 @@ inline bool plan_shape(Params &P, int CG, int sm_count, int *grid, size_t *smem)
                         b_bytes = align1k(chunks * piece);
                     }
                     if (bufs * plane_bytes + b_bytes > budget) continue;
-                    const int tiles = (T + kIssuers - 1) / kIssuers;   // of one issuer
+                    const int tiles = (T + issuers(CG) - 1) / issuers(CG);   // of one issuer
                     const int pieces = mode < 2 ? tiles : 9 * ((P.nseg + kChunkSegs - 1) / kChunkSegs);
                     const double compute = 9.0 * T * P.nseg * (mode == 0 ? whole : split) + 150.0 * pieces;
                     const double load_a = (double)P.nseg * (BY + 2) * pitch * kRow / 32.0;
                     const double load_b = mode < 2 ? 0.0 : 27.0 * P.nseg * CG * kRow / 32.0;
-                    const double drain = (T + kEpilogueSets - 1) / kEpilogueSets * (300.0 + 10.0 * CG);
+                    const double drain = 1200.0 + 10.0 * CG, drains = (T + drain_sets(CG) - 1) / drain_sets(CG) * 0.6 * drain;
+                    // a sub-tile's next plane waits for its drain: its own MMAs (those of the issuers side by side),
+                    // then the drain; streamed weights finish every sub-tile at the plane's end
+                    const double chain = compute / T * (mode == 2 ? T : std::min(T, issuers(CG))) + drain;
                     double plane = bufs == 1 ? std::max(compute, load_b) + load_a + 1500.0
                                              : std::max(compute, load_a + load_b) + (bufs == 2 ? 200.0 : 0.0);
-                    plane = std::max(plane, drain) + (mode == 2 || T <= 2 ? drain : 0.0);
+                    plane = std::max(plane, std::max(drains, chain));
                     const long long per = (units + parts - 1) / parts;
                     const double cols = 1.0 + (double)per / P.D;
                     const double total = plane * (per + 0.8 * 2 * cols) + (mode < 2 ? b_bytes / 32.0 : 0.0);
@@ -737,7 +754,7 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
     auto go = [&](auto kernel) -> const char * {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return "shared memory request rejected";
-        kernel<<<(unsigned)grid, kThreads, smem, stream>>>(ma0, ma1, mb, mb2, P);
+        kernel<<<(unsigned)grid, threads(CG), smem, stream>>>(ma0, ma1, mb, mb2, P);
         return nullptr;
     };
     switch (CG) {
