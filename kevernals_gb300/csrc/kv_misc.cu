@@ -57,10 +57,11 @@ __global__ void __launch_bounds__(256) saa_kernel(int nu, int nv, int nz, int P,
 // detector adds an exact zero, so the two kernels agree bit for bit.
 //
 // Seven FP32 additions per row and slice bound it (60 views of 2048 x 2048
-// into 128 slices: 2.3e11, 6.0 ms of the FP32 pipes).  Two rows a step in
-// packed additions (each half rounds as the scalar one) halve the issue slots,
-// one check of the band per slice and eight slices per staged band the rest:
-// 18.4 -> 11.7 ms there.  Where eight slices' spread does not fit, four.
+// into 128 slices: 2.3e11, 6.0 ms of the FP32 pipes).  Two columns a lane in
+// packed additions (each half rounds as the scalar one), eight slices a staged
+// band, two views a barrier and the slices' places in the band computed before
+// the loop: 18.4 -> 10.2 ms there.  Where eight slices' spread does not fit,
+// four.
 constexpr int kSaaRows = 32, kSaaStages = 4;
 constexpr uint32_t kSaaWaitPolls = 1u << 22;
 
@@ -93,29 +94,43 @@ __global__ void __launch_bounds__(256, 2) saa_band_kernel(const __grid_constant_
     constexpr int kPairs = kSaaRows / 16;   // a half warp a row, two columns a lane
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full[kSaaStages];
-    __shared__ int bstart[kSaaStages];
     unsigned char *base = smem + ((128u - (kvtma::smem_u32(smem) & 127u)) & 127u);
-    float *bands = reinterpret_cast<float *>(base);
-    int *sh = reinterpret_cast<int *>(base + kSaaStages * stage_stride);     // [P][KS]
+    int *off = reinterpret_cast<int *>(base + kSaaStages * stage_stride);    // [P][KS]: bytes into the band
+    int *first = off + KS * P;                                               // [P]: the band's first row
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int u0 = blockIdx.x * 32, v0 = blockIdx.y * kSaaRows, k0 = blockIdx.z * KS;
     const int kn = min(KS, nz - k0);
-    for (int t = threadIdx.x; t < KS * P; t += blockDim.x)   // slices past the last repeat it
-        sh[t] = shift[(size_t)(k0 + min(t % KS, kn - 1)) * P + t / KS];
+    // Where in its band each (view, slice) starts, once: in the loop a slice costs an address and its seven additions
+    // (shifts, band checks and addresses there were half its instructions).  A start outside the band is never
+    // expected; it is recorded and the block ends.
+    int err = 0;
+    for (int p = threadIdx.x; p < P; p += blockDim.x) {
+        int t[KS], tmin = shift[(size_t)k0 * P + p];
+#pragma unroll
+        for (int kk = 0; kk < KS; ++kk) {
+            t[kk] = shift[(size_t)(k0 + min(kk, kn - 1)) * P + p];   // slices past the last repeat it
+            tmin = min(tmin, t[kk]);
+        }
+        first[p] = v0 + tmin;
+#pragma unroll
+        for (int kk = 0; kk < KS; ++kk) {
+            off[p * KS + kk] = (t[kk] - tmin) * 128;
+            if (t[kk] - tmin > nb - kSaaRows) err = 4;
+        }
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kSaaStages; ++s) kvtma::mbar_init(&full[s], 1);
         kvtma::fence_mbar_init();
     }
-    __syncthreads();
+    if (__syncthreads_or(err)) {
+        if (err) atomicOr(status, err);
+        return;
+    }
     const uint32_t band_bytes = 32u * (uint32_t)nb * 4u;
     auto issue = [&](int i, int st) {
-        int tmin = sh[i * KS];
-        for (int kk = 1; kk < KS; ++kk) tmin = min(tmin, sh[i * KS + kk]);
-        const int bs = v0 + tmin;
-        bstart[st] = bs;
         kvtma::fence_proxy_async_smem();
         kvtma::mbar_arrive_expect_tx(&full[st], band_bytes);
-        kvtma::tma_load_3d(kvtma::smem_u32(base + (size_t)st * stage_stride), &pmap, &full[st], u0, bs, i);
+        kvtma::tma_load_3d(kvtma::smem_u32(base + (size_t)st * stage_stride), &pmap, &full[st], u0, first[i], i);
     };
     if (threadIdx.x == 0)
         for (int i = 0; i < kSaaStages && i < P; ++i) issue(i, i);
@@ -126,20 +141,25 @@ __global__ void __launch_bounds__(256, 2) saa_band_kernel(const __grid_constant_
     for (int m = 0; m < kPairs; ++m)
 #pragma unroll
         for (int kk = 0; kk < KS; ++kk) hi[m][kk] = lo[m][kk] = 0ull;
-    int err = 0, i = 0;
+    int i = 0;
     // one view's rows into sums a -> b: two register sets, so that the new sums need no move into the old ones' place
     auto add_view = [&](int view, int st, unsigned long long (&a)[kPairs][KS], unsigned long long (&b)[kPairs][KS]) {
-        const float *band = bands + (size_t)st * (stage_stride / 4) + col0;
-        const int rel = v0 + row0 - bstart[st];
+        const unsigned char *band = base + (size_t)st * stage_stride + (row0 * 32 + col0) * 4;
+        int o[KS];
+#pragma unroll
+        for (int kk = 0; kk < KS; kk += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(off + view * KS + kk);
+            o[kk] = v.x;
+            o[kk + 1] = v.y;
+            o[kk + 2] = v.z;
+            o[kk + 3] = v.w;
+        }
 #pragma unroll
         for (int kk = 0; kk < KS; ++kk) {
-            const int r0 = rel + sh[view * KS + kk];
-            const bool in = (unsigned)r0 <= (unsigned)(nb - kSaaRows + 15);
-            if (!in) err |= 4;                                          // rows outside the band: never expected
-            const float *row = band + (in ? r0 : 0) * 32;
+            const unsigned char *row = band + o[kk];
 #pragma unroll
             for (int m = 0; m < kPairs; ++m) {
-                const unsigned long long x = *reinterpret_cast<const unsigned long long *>(row + 16 * m * 32);
+                const unsigned long long x = *reinterpret_cast<const unsigned long long *>(row + 16 * m * 128);
                 b[m][kk] = add2(a[m][kk], x);                           // TwoSum(a, x)
                 const unsigned long long bp = sub2(b[m][kk], a[m][kk]);
                 const unsigned long long e = add2(sub2(a[m][kk], sub2(b[m][kk], bp)), sub2(x, bp));
@@ -553,7 +573,7 @@ bool saa_band_launch(kv_plan *plan, const int32_t *d_shift, const int32_t *h_shi
     kv_ctx *ctx = plan->ctx;
     const int nb = saa_band_rows(g, h_shift, KS);
     const uint32_t stride = (uint32_t)((32u * nb * 4u + 127u) / 128u * 128u);
-    const size_t smem = (size_t)kSaaStages * stride + (size_t)KS * g.n_views * sizeof(int32_t) + 128;
+    const size_t smem = (size_t)kSaaStages * stride + (size_t)(KS + 1) * g.n_views * sizeof(int32_t) + 128;
     if (nb > 256 || smem > smem_limit) return false;
     CUtensorMap map;
     cuuint64_t dims[3] = {(cuuint64_t)g.nu, (cuuint64_t)g.nv, (cuuint64_t)g.n_views};
