@@ -436,8 +436,8 @@ namespace {
 // Launch shapes of a new plan's kernels (kv_plan_autotune can pick others).
 //
 // Slab forward: the shapes that fit, by the number of rounds of resident CTAs
-// times what a round takes (two CTAs of R = 8, three of R = 4 or 2 a SM;
-// rounds measured 1 : 0.78 : 0.54 on a full GPU).  Large detectors take R = 8
+// times what a round takes (two CTAs of R = 8, three of R = 4 or 2 a SM where
+// shared memory allows; rounds measured 1 : 0.78 : 0.54 on a full GPU).  Large detectors take R = 8
 // (512 x 512 x 15 views: 321 us, R = 4: 336); 96 x 128 x 30 views R = 4 (20.6
 // us, R = 8: 24.4), 56 x 64 x 7 views R = 2 (12.8, R = 8: 18.1).
 //
@@ -454,17 +454,20 @@ void default_shapes(kv_plan *plan) {
     static const struct {
         int R, S, stages, per_sm;
         double round;
-    } shapes[] = {{8, 4, 2, 2, 1.0}, {4, 4, 3, 3, 0.78}, {4, 2, 3, 3, 0.95}, {2, 4, 3, 3, 0.54}, {2, 2, 2, 3, 0.8}};
+    } shapes[] = {{8, 4, 2, 2, 1.0}, {4, 4, 2, 3, 0.78}, {4, 2, 3, 3, 0.95}, {2, 4, 3, 3, 0.54}, {2, 2, 2, 3, 0.8}};
     double best = 1e300;
     const bool padded = (size_t)g.nx * kv_storage_bytes(plan->storage) % 16 != 0;
     FwdSlabCfg pick;
     for (const auto &sh : shapes) {
         const double ctas = (double)((g.nu + 31) / 32) * ((g.nv + 8 * sh.R - 1) / (8 * sh.R)) * g.n_views;
-        const double cost = std::ceil(ctas / (sms * sh.per_sm)) * sh.round;
         FwdSlabCfg c;
-        if (cost >= best ||
+        if (std::ceil(ctas / (sms * sh.per_sm)) * sh.round >= best ||
             !fwd_slab_fit(plan, sh.R, sh.S, sh.stages, fwd_slab_default_group(g.n_views), &c, nullptr, padded))
             continue;
+        // registers allow per_sm CTAs, shared memory (227 KB, 1 KB a CTA reserved) maybe fewer
+        const int fit = std::max(1, std::min(sh.per_sm, (int)(227 * 1024 / (c.smem + 1024))));
+        const double cost = std::ceil(ctas / (sms * fit)) * sh.round * fit / sh.per_sm;
+        if (cost >= best) continue;
         best = cost;
         pick = c;
     }

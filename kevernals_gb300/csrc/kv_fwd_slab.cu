@@ -83,8 +83,10 @@ __host__ __device__ __forceinline__ void span2(float4 A, int ia, float4 B, int i
 
 // Box origin of slab s for the tile whose corner rays are (Xa, Xb) in x and
 // (Ya, Yb) in y: three columns of margin (a ray's start column and the two
-// after it stay inside), two rows (the rows a ray meets are exactly those
-// between its end planes).  x is rounded down to the TMA's 16-byte grid.
+// after it stay inside), kMaxRows - 1 rows (the rows a ray meets are exactly
+// those between its end planes; in lockstep with longer rays its address runs
+// on by up to that many, at zero length).  x is rounded down to the TMA's
+// 16-byte grid.
 __host__ __device__ __forceinline__ void box_origin(float4 Xa, int ia, float4 Xb, int ibb, float4 Ya, int ja,
                                                     float4 Yb, int jbb, float h0, float h1, int align, int &x0,
                                                     int &y0, int &need_x, int &need_y) {
@@ -92,9 +94,9 @@ __host__ __device__ __forceinline__ void box_origin(float4 Xa, int ia, float4 Xb
     span2(Xa, ia, Xb, ibb, h0, h1, cmin, cmax);
     span2(Ya, ja, Yb, jbb, h0, h1, rmin, rmax);
     x0 = floor_to(cmin - 3, align);
-    y0 = rmin - 2;
+    y0 = rmin - (kMaxRows - 1);
     need_x = cmax + 3 - x0 + 1;
-    need_y = rmax + 2 - y0 + 1;
+    need_y = rmax + kMaxRows - 1 - y0 + 1;
 }
 
 template <typename T> __device__ __forceinline__ float sld(const T *p);
@@ -111,8 +113,10 @@ __device__ __forceinline__ bool in_volume(int col, int row, int nx, int ny) {
 
 // The rays q0 .. q0+NQ-1 of this thread (same detector column, rows 8 apart)
 // in one slice, their rows in lockstep: rows past a ray's own count have
-// lo = hi = 1 (the crossings are clamped to 1) and weigh nothing, and its
-// row address stops advancing there, so every read stays inside the box.
+// lo = hi = 1 (the crossings are clamped to 1) and weigh nothing, and the
+// box's margin holds the addresses they run on to (stopping each ray's address
+// at its own count took a compare and a predicate a row: 60 views of 2048 x
+// 2048, 128 slices, 48.4 -> 45.2 ms with the first row's clamps gone too).
 // Lengths in clamp form: with a1 = min(max(X1, lo), hi) and a2 likewise, the
 // ray spends a1 - lo in its first column, a2 - a1 in the second and hi - a2
 // in the third.  Where min(hi, X_{c+1}) - max(lo, X_c) is positive these are
@@ -148,13 +152,14 @@ __device__ __forceinline__ void slice_rays(const unsigned char *box, const YDesc
             if (r > 0) {
                 lo[q] = hi[q];
                 hi[q] = r == 1 ? yc[q].y : (r == 2 ? yc[q].z : (r == 3 ? yc[q].w : 1.f));
-                if (r < nr[q]) off[q] += step[q];
+                off[q] += step[q];
             }
-            const float a1 = fminf(fmaxf(X1, lo[q]), hi[q]);
-            const float w0 = __fsub_rn(a1, lo[q]);
+            // the first row starts at 0 and the crossings are not negative: no clamp from below, nothing to subtract
+            const float a1 = r == 0 ? fminf(X1, hi[q]) : fminf(fmaxf(X1, lo[q]), hi[q]);
+            const float w0 = r == 0 ? a1 : __fsub_rn(a1, lo[q]);
             float w1, w2 = 0.f;
             if (NC3) {
-                const float a2 = fminf(fmaxf(X2, lo[q]), hi[q]);
+                const float a2 = r == 0 ? fminf(X2, hi[q]) : fminf(fmaxf(X2, lo[q]), hi[q]);
                 w1 = __fsub_rn(a2, a1);
                 w2 = __fsub_rn(hi[q], a2);
             } else {
