@@ -109,6 +109,7 @@ struct Params {
     int relu;
     const __nv_bfloat16 *mask;    // nullptr: none; else outputs where mask <= 0 become 0
     __nv_bfloat16 *out;           // [voxels][N]; nullptr: not stored
+    int out32;                    // out is 32-byte aligned
     Head head;                    // y == nullptr: none (N = 16 only)
     int *status;                  // 0 ok; set on a failed wait
 };
@@ -179,6 +180,13 @@ __device__ __forceinline__ void tc_zero16(uint32_t taddr) {
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
         "r"(0u)
         : "memory");
+}
+
+// 32 bytes as one store (32-byte aligned): two 16-byte stores a lane write every sector in two parts
+__device__ __forceinline__ void st32(void *p, const uint4 &a, const uint4 &b) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major operand tile of 32-byte rows
@@ -514,8 +522,13 @@ __global__ void __launch_bounds__(threads(CG), 1)
                                 }
                                 if (P.out != nullptr) {
                                     uint4 *d4 = reinterpret_cast<uint4 *>(P.out + o + 16 * q);
-                                    d4[0] = reinterpret_cast<const uint4 *>(r)[0];
-                                    d4[1] = reinterpret_cast<const uint4 *>(r)[1];
+                                    const uint4 *r4 = reinterpret_cast<const uint4 *>(r);
+                                    if (P.out32) {
+                                        st32(d4, r4[0], r4[1]);
+                                    } else {
+                                        d4[0] = r4[0];
+                                        d4[1] = r4[1];
+                                    }
                                 }
                                 if (CG == 16 && P.head.y != nullptr) {
                                     float h = hw[16];
@@ -742,6 +755,7 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
     P.relu = relu ? 1 : 0;
     P.mask = mask;
     P.out = out;
+    P.out32 = reinterpret_cast<uintptr_t>(out) % 32 == 0;
     if (head != nullptr) P.head = *head;
     P.status = status;
     CUtensorMap ma0, ma1, mb, mb2;

@@ -66,11 +66,12 @@ __device__ __forceinline__ Bf8 pack8(const float (&f)[8]) {
 
 // First layer, 1 -> 16 channels in FP32.  432 multiply-adds a voxel bound it
 // (0.39 ms of FP32 issue at 128 x 512 x 512 voxels, 0.18 ms of memory), so a
-// thread computes kFirstRows voxels of consecutive y: the weights, in shared
-// memory, are read once for all of them, and their rows overlap.  One voxel a
-// thread with the weights in global memory took 2.19 ms, this takes 0.79
-// (0.94 with scalar fmaf).  Blocks of 128 x.
-constexpr int kFirstRows = 4;
+// thread computes kFirstRows voxels of consecutive y in packed arithmetic: the
+// weights, in shared memory, are read once for all of them, and their rows
+// overlap.  One voxel a thread with the weights in global memory took 2.19 ms;
+// four rows 0.79 (0.94 with scalar fmaf), two rows, which leave registers for
+// more warps, and 32-byte stores 0.75.  Blocks of 128 x.
+constexpr int kFirstRows = 2;
 
 __global__ void __launch_bounds__(128) conv_first_fwd(const float *__restrict__ x, const float *__restrict__ w /*[16][27]*/,
                                                       const float *__restrict__ b, bf16 *__restrict__ out, int D, int H,
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(128) conv_first_fwd(const float *__restrict__ 
 #pragma unroll
         for (int r = 0; r < kFirstRows; ++r) {
             bf16 *dst = out + (((size_t)z * H + y0 + r) * W + xx) * 16;
+            Bf8 o[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 float f[8];
@@ -128,8 +130,9 @@ __global__ void __launch_bounds__(128) conv_first_fwd(const float *__restrict__ 
                     f[2 * c] = fmaxf(f[2 * c], 0.f);
                     f[2 * c + 1] = fmaxf(f[2 * c + 1], 0.f);
                 }
-                st8(dst + 8 * h, pack8(f));
+                o[h] = pack8(f);
             }
+            convtc::st32(dst, *reinterpret_cast<const uint4 *>(&o[0]), *reinterpret_cast<const uint4 *>(&o[1]));
         }
     }
 }
@@ -147,77 +150,99 @@ __device__ __forceinline__ void block_add(float v, float *dst, float *sh /* [16]
     }
 }
 
-// dW0[c][tap] += sum_v dpre[v][c] * x[v + tap], the nine taps of one dz (blockIdx.y) at once: 144 sums in registers
-// for one read of dpre (one tap a pass read it 27 times: 1.24 ms at 128 x 256 x 128 voxels).  The bias gradient comes
-// with dz = 1.
-__global__ void __launch_bounds__(256) conv_first_wgrad(const float *__restrict__ x, const bf16 *__restrict__ dpre,
-                                                        float *__restrict__ dw, float *__restrict__ db, int D, int H,
-                                                        int W) {
-    __shared__ float part[8][9][16];
-    const int dz = blockIdx.y;
-    const long long n = (long long)D * H * W;
-    float acc[9][16], accb[16];
+// dW0[c][tap] += sum_v dpre[v][c] * x[v + tap] for the nine taps of one dz (blockIdx.y) and eight channels
+// (blockIdx.z): 72 sums a thread in packed FP32, over four voxels of consecutive y at a time, whose 18 x values and
+// four 16-byte gradients are all in flight together.  All 16 channels of one voxel a thread (250 registers, one block
+// a SM, a load latency a voxel) took 341 us at 128 x 256 x 128 voxels, one tap a pass 1244; this takes 167.  The bias
+// gradient comes with dz = 1.
+__global__ void __launch_bounds__(256, 2) conv_first_wgrad(const float *__restrict__ x, const bf16 *__restrict__ dpre,
+                                                           float *__restrict__ dw, float *__restrict__ db, int D, int H,
+                                                           int W) {
+    __shared__ float part[8][9][8];
+    const int dz = blockIdx.y, c0 = 8 * blockIdx.z, h4 = H / 4;   // H % 8 == 0
+    const long long n = (long long)D * h4 * W;
+    unsigned long long acc[9][4];
+    float accb[8];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        accb[c] = 0.f;
-#pragma unroll
-        for (int t = 0; t < 9; ++t) acc[t][c] = 0.f;
-    }
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const int xx = (int)(v % W);
-        const long long zy = v / W;
-        const int y = (int)(zy % H), zz = (int)(zy / H) + dz - 1;
-        float g[16], in[9];
-        float lo[8], hi[8];
-        unpack8(ld8(dpre + v * 16), lo);
-        unpack8(ld8(dpre + v * 16 + 8), hi);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            g[c] = lo[c];
-            g[8 + c] = hi[c];
-        }
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            const int yy = y + t / 3 - 1, x2 = xx + t % 3 - 1;
-            const bool ok = (unsigned)zz < (unsigned)D && (unsigned)yy < (unsigned)H && (unsigned)x2 < (unsigned)W;
-            in[t] = ok ? __ldg(x + ((long long)zz * H + yy) * W + x2) : 0.f;
-        }
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            if (dz == 1) accb[c] += g[c];
-#pragma unroll
-            for (int t = 0; t < 9; ++t) acc[t][c] = fmaf(g[c], in[t], acc[t][c]);
-        }
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int c = 0; c < 8; ++c) accb[c] = 0.f;
 #pragma unroll
     for (int t = 0; t < 9; ++t)
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            float s = acc[t][c];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) part[warp][t][c] = s;
+        for (int c = 0; c < 4; ++c) acc[t][c] = 0ull;
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        const int xx = (int)(v % W);
+        const long long zy = v / W;
+        const int y0 = (int)(zy % h4) * 4, z = (int)(zy / h4), zz = z + dz - 1;
+        Bf8 g[4];
+        float in[6][3];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) g[r] = ld8(dpre + (((size_t)z * H + y0 + r) * W + xx) * 16 + c0);
+#pragma unroll
+        for (int r = 0; r < 6; ++r)
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                const int yy = y0 + r - 1, x2 = xx + dx - 1;
+                const bool ok = (unsigned)zz < (unsigned)D && (unsigned)yy < (unsigned)H && (unsigned)x2 < (unsigned)W;
+                in[r][dx] = ok ? __ldg(x + ((size_t)zz * H + yy) * W + x2) : 0.f;
+            }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            unsigned long long gp[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float2 f = __bfloat1622float2(g[r].v[c]);
+                if (dz == 1) {
+                    accb[2 * c] += f.x;
+                    accb[2 * c + 1] += f.y;
+                }
+                asm("mov.b64 %0, {%1, %2};" : "=l"(gp[c]) : "f"(f.x), "f"(f.y));
+            }
+#pragma unroll
+            for (int t = 0; t < 9; ++t) {
+                unsigned long long xv;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(xv) : "f"(in[r + t / 3][t % 3]));
+#pragma unroll
+                for (int c = 0; c < 4; ++c) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][c]) : "l"(gp[c]), "l"(xv));
+            }
+        }
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto warp_sum = [](float f) {
+        for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+        return f;
+    };
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            float a, b;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(acc[t][c]));
+            a = warp_sum(a);
+            b = warp_sum(b);
+            if (lane == 0) {
+                part[warp][t][2 * c] = a;
+                part[warp][t][2 * c + 1] = b;
+            }
         }
     __syncthreads();
-    if (threadIdx.x < 144) {
-        const int t = threadIdx.x / 16, c = threadIdx.x % 16;
-        float s = 0.f;
-        for (int i = 0; i < 8; ++i) s += part[i][t][c];
-        atomicAdd(dw + c * 27 + dz * 9 + t, s);
+    if (threadIdx.x < 72) {
+        const int t = threadIdx.x / 8, c = threadIdx.x % 8;
+        float f = 0.f;
+        for (int i = 0; i < 8; ++i) f += part[i][t][c];
+        atomicAdd(dw + (c0 + c) * 27 + dz * 9 + t, f);
     }
     if (dz != 1) return;
     __syncthreads();
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        float s = accb[c];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) part[warp][0][c] = s;
+    for (int c = 0; c < 8; ++c) {
+        const float f = warp_sum(accb[c]);
+        if (lane == 0) part[warp][0][c] = f;
     }
     __syncthreads();
-    if (threadIdx.x < 16) {
-        float s = 0.f;
-        for (int i = 0; i < 8; ++i) s += part[i][0][threadIdx.x];
-        atomicAdd(db + threadIdx.x, s);
+    if (threadIdx.x < 8) {
+        float f = 0.f;
+        for (int i = 0; i < 8; ++i) f += part[i][0][threadIdx.x];
+        atomicAdd(db + c0 + threadIdx.x, f);
     }
 }
 
@@ -277,6 +302,7 @@ __global__ void __launch_bounds__(256) conv_out_bwd(const bf16 *__restrict__ h, 
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
         const float g = dy[v];
         accb += g;
+        Bf8 o[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             float hv[8], d[8];
@@ -286,8 +312,9 @@ __global__ void __launch_bounds__(256) conv_out_bwd(const bf16 *__restrict__ h, 
                 acc[8 * q + c] = fmaf(g, hv[c], acc[8 * q + c]);
                 d[c] = hv[c] > 0.f ? wv[8 * q + c] * g : 0.f;
             }
-            st8(dh + v * 16 + 8 * q, pack8(d));
+            o[q] = pack8(d);
         }
+        convtc::st32(dh + v * 16, *reinterpret_cast<const uint4 *>(&o[0]), *reinterpret_cast<const uint4 *>(&o[1]));
     }
 #pragma unroll
     for (int c = 0; c < 16; ++c) block_add(acc[c], dw + c, sh);
@@ -681,7 +708,8 @@ kv_status backward(kv_unet *u) {
     // level 0 encoder
     KV_TRY(conv_backward(u, 0, g[E1], a[A0], nullptr, g[A0], 0, a[A0]));
     {
-        dim3 grid(std::min(grid_n(ctx, n0), ctx->sm_count), 3);
+        // one round of resident blocks over the six (dz, channel half) passes
+        dim3 grid(std::min(grid_n(ctx, n0 / 4), std::max(1, ctx->sm_count / 3)), 3, 2);
         conv_first_wgrad<<<grid, 256, 0, ctx->stream>>>(u->x, g[A0], u->g + u->w_first, u->g + u->b_first, D, H, W);
     }
     KV_CHECK_LAUNCH(ctx, "unet backward");
