@@ -197,10 +197,9 @@ kv_status kv_mlem(kv_plan *plan, const float *projections, float *volume_inout, 
 kv_status kv_sart(kv_plan *plan, const float *projections, float *volume_inout, int iterations,
                   float relax, kv_mem mem, kv_iter_cb cb, void *user);
 /* Batched MLEM: n independent EXACT/FP32 reconstructions of uneven volume,
- * detector and view counts, all created on `ctx`, run together.  Each
- * iteration is one persistent forward launch and one persistent
- * backprojection launch over the tiles of every problem; the whole
- * `iterations` loop is captured as one CUDA graph.  Results are identical to
+ * detector and view counts, all created on `ctx`, run side by side: each goes
+ * through its own plan's kernels on one of the context's side streams, which
+ * fork from and join the context's stream.  Results are identical to
  * calling kv_mlem on each plan.  No reference counterpart (the reference
  * reconstructs one case per call).  projections[i] / volumes[i] are host or
  * device buffers according to `mem`; volumes are updated in place. */
@@ -271,8 +270,8 @@ kv_status kv_plan_set_back_staging(kv_plan *plan, int rows_per_thread, int stage
  * (may be NULL when c2 = 0) c2 channels concatenated after them, out cout
  * channels; w is [cout][27][c1 + c2] BF16 (taps z, y, x), bias cout floats
  * or NULL; FP32 accumulation.  kernel: 0 = tcgen05 / TMA implicit GEMM where
- * the volume is a whole number of 128-voxel tiles, else mma.sync; 1 =
- * tcgen05 only; 2 = mma.sync only.  Channel counts: multiples of 16 (the
+ * it covers the call, else mma.sync (equal bits); 1 = tcgen05 only, for
+ * volumes of whole 128-voxel tiles; 2 = mma.sync only.  Channel counts: multiples of 16 (the
  * tcgen05 kernel: 16, 32, 64 or 128 per input, cout <= 256).  Stream-ordered
  * on the context's stream; a tensor-core pipeline wait that gives up is
  * reported by the next kv_sync. */

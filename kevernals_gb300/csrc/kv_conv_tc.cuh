@@ -734,6 +734,11 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
     auto ok_c = [](int c) { return c == 16 || c == 32 || c == 64 || c == 128; };
     if (!ok_c(c1) || (c2 != 0 && !ok_c(c2))) return "input channels must be 16, 32, 64 or 128";
     if (N % 16 != 0 || N < 16 || N > 256) return "output channels must be a multiple of 16 up to 256";
+    // the operator's limits: four segments of one width, and 128 + N rows of every segment twice in 200 KB
+    const int kseg = std::min(std::min(c1, 64), c2 != 0 ? c2 : 64), segs = K / kseg;
+    if (segs > 4) return "too many input channel segments";
+    if (2 * (size_t)segs * (align1k(kTileM * kseg * 2) + align1k(N * kseg * 2)) > 200 * 1024)
+        return "stage does not fit in shared memory";
     if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(mask)) % 16 != 0)
         return "output or mask is not 16-byte aligned";
     if (head != nullptr && N != 16) return "the output layer takes 16 channels";

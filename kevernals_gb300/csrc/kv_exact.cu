@@ -44,9 +44,8 @@ __device__ __forceinline__ void lateral_slices(float pos0, float slope, int n, i
     khi = fmaxf(a, b);
 }
 
-// One tile of 32 x blockDim.y rays of view p (tile coordinates bx, by) --
-// the body of the forward kernel, shared by the per-plan launch and the
-// batched persistent kernel.  blin: linear tile index for the partial sums.
+// One tile of 32 x blockDim.y rays of view p (tile coordinates bx, by), the
+// body of the forward kernel.  blin: linear tile index for the partial sums.
 template <typename VolT, typename ProjT, int MODE>
 __device__ __forceinline__ void fwd_tile(const ExGeom &G, const ExactTables &T, const FwdArgs &a,
                                          double *partials, int bx, int by, int p, size_t blin) {

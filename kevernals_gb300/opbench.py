@@ -155,8 +155,8 @@ def main(argv=None):
             net.close()
         elif op == "batch_small":
             # many small problems: 256 seeded uneven cases at a quarter of the
-            # batched workload's sizes, 30 MLEM iterations, one persistent
-            # launch per phase (kv_batch_mlem) against solving one by one
+            # batched workload's sizes, 30 MLEM iterations side by side
+            # (kv_batch_mlem) against solving one by one
             from .geometry import uneven_cases
             cases = uneven_cases(256, 20261203 + 3000, scale=4)
             bplans, data = [], []

@@ -106,7 +106,7 @@ def test_conv_layer_tcgen05_vs_mma_sync_and_fp64(ctx, shape):
 COLUMNS = [
     (1, 1, 128, 16, 0, 16), (3, 11, 128, 16, 0, 16), (37, 23, 128, 32, 16, 16), (5, 3, 256, 16, 0, 48),
     (7, 14, 64, 64, 32, 32), (3, 6, 64, 32, 0, 96), (2, 20, 32, 128, 64, 64), (4, 24, 16, 128, 0, 128),
-    (2, 5, 192, 32, 0, 32), (3, 7, 48, 64, 0, 64), (1, 2, 16, 64, 0, 192), (9, 1, 384, 16, 128, 80),
+    (2, 5, 192, 32, 0, 32), (3, 7, 48, 64, 0, 64), (1, 2, 16, 64, 0, 192), (9, 1, 384, 64, 128, 80),
 ]
 
 
@@ -122,3 +122,17 @@ def test_conv_columns_equal_mma_sync(ctx, shape):
     bias = (rng.standard_normal(cout) * 0.1).astype(np.float32)
     got = _conv(ctx, a, c1, b, c2, w, bias, True, cout, (D, H, W), 0)
     assert np.array_equal(got, _conv(ctx, a, c1, b, c2, w, bias, True, cout, (D, H, W), 2))
+
+
+@pytest.mark.parametrize("c1,c2,cout", [(128, 16, 16), (16, 128, 32), (128, 128, 256), (48, 0, 16)])
+def test_conv_limits_are_refused(ctx, c1, c2, cout):
+    """Channel counts outside the operator's limits on a volume of whole tiles: an error, nothing run."""
+    torch = pytest.importorskip("torch")
+    from kevernals_gb300 import _lib
+    t = torch.zeros(2 * 128 * 256 * 27, dtype=torch.int16, device="cuda")
+    f = torch.zeros(256, device="cuda")
+    p = C.c_void_p(t.data_ptr())
+    for kernel in (0, 1):
+        st = _lib.lib().kv_conv3_bf16(ctx.handle, p, c1, p if c2 else None, c2, p, C.c_void_p(f.data_ptr()), 1, p,
+                                      cout, 1, 2, 128, kernel)
+        assert _lib.STATUS_NAMES[st] == "KV_ERR_UNSUPPORTED"
