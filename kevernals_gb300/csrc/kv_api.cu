@@ -549,6 +549,7 @@ extern "C" kv_status kv_plan_destroy(kv_plan *plan) {
     cudaFree(plan->d_proj32);
     cudaFree(plan->d_pad);
     cudaFree(plan->d_rows);
+    if (plan->rows_event) cudaEventDestroy(plan->rows_event);
     cudaFree(plan->d_sens);
     cudaFree(plan->d_shift);
     if (plan->graph_exec) cudaGraphExecDestroy(plan->graph_exec);
@@ -808,7 +809,24 @@ FwdMode sart_mode(kv_plan *plan, FwdArgs &a) {
     return plan->d_rows != nullptr && plan->rows_valid ? FWD_SART_ROWS : FWD_SART;
 }
 
+// The row sums are stored by what was launched last on the context's stream;
+// a solve on another stream waits for them (wait_rows).
+void mark_rows(kv_plan *plan) {
+    if (plan->d_rows == nullptr || plan->rows_valid) return;
+    plan->rows_valid = true;
+    if (stream_capturing(plan->ctx)) return;   // the caller records behind the launch
+    if (plan->rows_event == nullptr) cudaEventCreateWithFlags(&plan->rows_event, cudaEventDisableTiming);
+    if (plan->rows_event == nullptr || cudaEventRecord(plan->rows_event, plan->ctx->stream) != cudaSuccess)
+        cudaStreamSynchronize(plan->ctx->stream);
+}
+
+void wait_rows(kv_plan *plan) {
+    if (plan->rows_valid && plan->rows_event != nullptr && !stream_capturing(plan->ctx))
+        cudaStreamWaitEvent(plan->ctx->stream, plan->rows_event, 0);
+}
+
 void ensure_rows(kv_plan *plan) {
+    wait_rows(plan);
     if (plan->d_rows == nullptr &&
         (stream_capturing(plan->ctx) || cudaMalloc((void **)&plan->d_rows, plan->nproj * sizeof(float)) != cudaSuccess)) {
         cudaGetLastError();
@@ -873,7 +891,7 @@ kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float 
         plan->graph_bst = plan->bstage.R * 16 + plan->bstage.stages;
     }
     KV_CHECK_CUDA(ctx, cudaGraphLaunch(plan->graph_exec, ctx->stream));
-    if (!mlem && plan->family == KV_FAMILY_EXACT && plan->d_rows != nullptr) plan->rows_valid = true;
+    if (!mlem && plan->family == KV_FAMILY_EXACT) mark_rows(plan);
     return KV_OK;
 }
 
@@ -897,7 +915,7 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
             FwdArgs fa{x, p, plan->d_ratio, cb ? ctx->d_red : nullptr, relax};
             fa.pad = plan->d_pad;
             KV_TRY(exact_forward_launch(plan, plan->ex, plan->g.n_views, mlem ? FWD_MLEM : sart_mode(plan, fa), fa));
-            if (!mlem && plan->d_rows != nullptr) plan->rows_valid = true;
+            if (!mlem) mark_rows(plan);
         } else if (cb) {
             KV_TRY(rc_forward_launch(plan, plan->d_src, plan->d_org, plan->g.n_views, RC_PLAIN, (const float *)x,
                                      nullptr, (float *)plan->d_ratio, relax));
@@ -942,7 +960,7 @@ kv_status update_forward_views(kv_plan *plan, bool mlem, const float *pd, const 
         fa.pad = plan->d_pad;
         fa.pad_ready = v0 > 0;   // view chunks of one volume, the first from view 0
         KV_TRY(exact_forward_views_launch(plan, v0, n, mlem ? FWD_MLEM : sart_mode(plan, fa), fa));
-        if (!mlem && plan->d_rows != nullptr && v0 + n == plan->g.n_views) plan->rows_valid = true;   // chunks in order
+        if (!mlem && v0 + n == plan->g.n_views) mark_rows(plan);   // chunks in order
         return KV_OK;
     }
     const size_t off = (size_t)v0 * plan->g.nu * plan->g.nv;

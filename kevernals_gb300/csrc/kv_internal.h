@@ -135,6 +135,7 @@ struct kv_plan {
     void *d_pad = nullptr;           // volume with padded rows (fpad)
     float *d_rows = nullptr;         // A 1, SART's row sums (EXACT)
     bool rows_valid = false;
+    cudaEvent_t rows_event = nullptr;   // recorded behind the pass that stored d_rows
     double *d_sens = nullptr;        // A^T 1 in FP64 (EXACT)
     bool sens_valid = false;
     int32_t *d_shift = nullptr;      // shift-and-add table [nz][P]
