@@ -49,9 +49,10 @@ constexpr uint32_t kWaitPolls = 1u << 22;
 struct YDesc {
     float4 yc;      // min(1, Y1 .. Y4)
     int rowoff;     // byte offset of (slice, first row) within the stage
-    int rowstep;    // +-BX elements, in bytes: next row in the direction of travel
+    int rowstep;    // +-BX elements, in bytes: next row in the direction of travel (0: no second row)
     int nr;         // rows met in this slice (0: no ray)
-    int row0;       // volume row of the first row (SART row sums count in-volume voxels only)
+    int row0;       // SART row sums (they count in-volume voxels only): volume row of the first row; else the step to
+                    // the third row (0: none)
 };
 
 struct SlabArgs {
@@ -83,10 +84,8 @@ __host__ __device__ __forceinline__ void span2(float4 A, int ia, float4 B, int i
 
 // Box origin of slab s for the tile whose corner rays are (Xa, Xb) in x and
 // (Ya, Yb) in y: three columns of margin (a ray's start column and the two
-// after it stay inside), kMaxRows - 1 rows (the rows a ray meets are exactly
-// those between its end planes; in lockstep with longer rays its address runs
-// on by up to that many, at zero length).  x is rounded down to the TMA's
-// 16-byte grid.
+// after it stay inside), two rows (the rows a ray meets are exactly those
+// between its end planes).  x is rounded down to the TMA's 16-byte grid.
 __host__ __device__ __forceinline__ void box_origin(float4 Xa, int ia, float4 Xb, int ibb, float4 Ya, int ja,
                                                     float4 Yb, int jbb, float h0, float h1, int align, int &x0,
                                                     int &y0, int &need_x, int &need_y) {
@@ -94,9 +93,9 @@ __host__ __device__ __forceinline__ void box_origin(float4 Xa, int ia, float4 Xb
     span2(Xa, ia, Xb, ibb, h0, h1, cmin, cmax);
     span2(Ya, ja, Yb, jbb, h0, h1, rmin, rmax);
     x0 = floor_to(cmin - 3, align);
-    y0 = rmin - (kMaxRows - 1);
+    y0 = rmin - 2;
     need_x = cmax + 3 - x0 + 1;
-    need_y = rmax + kMaxRows - 1 - y0 + 1;
+    need_y = rmax + 2 - y0 + 1;
 }
 
 template <typename T> __device__ __forceinline__ float sld(const T *p);
@@ -113,10 +112,13 @@ __device__ __forceinline__ bool in_volume(int col, int row, int nx, int ny) {
 
 // The rays q0 .. q0+NQ-1 of this thread (same detector column, rows 8 apart)
 // in one slice, their rows in lockstep: rows past a ray's own count have
-// lo = hi = 1 (the crossings are clamped to 1) and weigh nothing, and the
-// box's margin holds the addresses they run on to (stopping each ray's address
-// at its own count took a compare and a predicate a row: 60 views of 2048 x
-// 2048, 128 slices, 48.4 -> 45.2 ms with the first row's clamps gone too).
+// lo = hi = 1 (the crossings are clamped to 1) and weigh nothing, and its
+// address stops at its last row: it stays in the box, and a voxel that is not
+// finite reaches no ray of another row (0 x inf).  The steps to the second
+// and third row are zero where there is none (make_desc), so only the rows
+// beyond compare with the ray's count (compared at every row, 60 views of 2048
+// x 2048 and 128 slices take 48.4 ms; from the third on 46.4; from the fourth,
+// as here, 45.6; never, 45.2).
 // Lengths in clamp form: with a1 = min(max(X1, lo), hi) and a2 likewise, the
 // ray spends a1 - lo in its first column, a2 - a1 in the second and hi - a2
 // in the third.  Where min(hi, X_{c+1}) - max(lo, X_c) is positive these are
@@ -152,7 +154,9 @@ __device__ __forceinline__ void slice_rays(const unsigned char *box, const YDesc
             if (r > 0) {
                 lo[q] = hi[q];
                 hi[q] = r == 1 ? yc[q].y : (r == 2 ? yc[q].z : (r == 3 ? yc[q].w : 1.f));
-                off[q] += step[q];
+                if (r == 1) off[q] += step[q];
+                else if (r == 2 && !SART) off[q] += row0[q];
+                else if (r < nr[q]) off[q] += step[q];
             }
             // the first row starts at 0 and the crossings are not negative: no clamp from below, nothing to subtract
             const float a1 = r == 0 ? fminf(X1, hi[q]) : fminf(fmaxf(X1, lo[q]), hi[q]);
@@ -290,9 +294,9 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
             } else {
                 d.yc = make_float4(fminf(1.f, y1), fminf(1.f, y2), fminf(1.f, y3), fminf(1.f, y4));
                 d.rowoff = (kk * A.BY + js) * A.BX * (int)sizeof(VolT);
-                d.rowstep = (negy ? -A.BX : A.BX) * (int)sizeof(VolT);
+                d.rowstep = nr == 1 ? 0 : (negy ? -A.BX : A.BX) * (int)sizeof(VolT);
                 d.nr = nr;
-                d.row0 = j0;
+                d.row0 = SART ? j0 : (nr <= 2 ? 0 : d.rowstep);
             }
         }
         desc[(buf * A.S + kk) * TV + vl] = d;
