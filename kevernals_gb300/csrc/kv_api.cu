@@ -38,6 +38,7 @@ kv_status device_status(kv_ctx *ctx) {
     KV_CHECK_CUDA(ctx, cudaMemcpyAsync(&h, ctx->d_status, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     KV_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (h == 0) return KV_OK;
+    ctx->status_gen += 1;
     KV_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
     return kv_fail(ctx, (h & 9) ? KV_ERR_TIMEOUT : KV_ERR_CUDA,
                    "a projector kernel stopped early (status bits 0x%x: 1 = a staged load did not arrive, "
@@ -801,58 +802,87 @@ void ensure_pad(kv_plan *plan) {
     }
 }
 
-// SART's row sums A 1 depend on the geometry alone: the first forward pass of
-// a plan's first SART solve stores them and later passes read them (a quarter
-// of the pass was their in-volume test).  Returns the mode of the next pass.
-FwdMode sart_mode(kv_plan *plan, FwdArgs &a) {
-    a.rows = plan->d_rows;
-    return plan->d_rows != nullptr && plan->rows_valid ? FWD_SART_ROWS : FWD_SART;
-}
-
-// The row sums are stored by what was launched last on the context's stream;
-// a solve on another stream waits for them (wait_rows).
-void mark_rows(kv_plan *plan) {
-    if (plan->d_rows == nullptr || plan->rows_valid) return;
-    plan->rows_valid = true;
-    if (stream_capturing(plan->ctx)) return;   // the caller records behind the launch
-    if (plan->rows_event == nullptr) cudaEventCreateWithFlags(&plan->rows_event, cudaEventDisableTiming);
-    if (plan->rows_event == nullptr || cudaEventRecord(plan->rows_event, plan->ctx->stream) != cudaSuccess)
-        cudaStreamSynchronize(plan->ctx->stream);
-}
-
-void wait_rows(kv_plan *plan) {
-    if (plan->rows_valid && plan->rows_event != nullptr && !stream_capturing(plan->ctx))
-        cudaStreamWaitEvent(plan->ctx->stream, plan->rows_event, 0);
-}
-
-void ensure_rows(kv_plan *plan) {
-    wait_rows(plan);
-    if (plan->d_rows == nullptr &&
-        (stream_capturing(plan->ctx) || cudaMalloc((void **)&plan->d_rows, plan->nproj * sizeof(float)) != cudaSuccess)) {
-        cudaGetLastError();
-        plan->d_rows = nullptr;   // every pass forms them again
+// SART's row sums A 1 depend on the geometry alone: a plan's first SART pass
+// stores them in d_rows and later passes read them (a quarter of the pass was
+// their in-volume test).  They count as stored only while no kernel of the
+// context has reported an error since (status_gen): a pass that gave up
+// leaves some unwritten.  ready_rows: whether a solve may read them from its
+// first pass on.  A caller's capture never does: its graph stores its own.
+bool ready_rows(kv_plan *plan) {
+    kv_ctx *ctx = plan->ctx;
+    if (stream_capturing(ctx)) return false;
+    if (plan->d_rows == nullptr) {
+        if (cudaMalloc((void **)&plan->d_rows, plan->nproj * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            plan->d_rows = nullptr;   // every pass forms them again
+        }
+        return false;
     }
+    if (plan->rows_gen != ctx->status_gen) return false;
+    // the pass that stored them may have run on another stream
+    if (cudaStreamWaitEvent(ctx->stream, plan->rows_event, 0) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// The pass launched last on the context's stream has stored the row sums.
+void keep_rows(kv_plan *plan) {
+    kv_ctx *ctx = plan->ctx;
+    if (stream_capturing(ctx)) return;   // recorded, not run
+    if (plan->rows_event == nullptr &&
+        cudaEventCreateWithFlags(&plan->rows_event, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        plan->rows_event = nullptr;
+        return;
+    }
+    if (cudaEventRecord(plan->rows_event, ctx->stream) == cudaSuccess) plan->rows_gen = ctx->status_gen;
+    else cudaGetLastError();
+}
+
+// One fused EXACT forward pass of a solve on views [v0, v0 + n).  `rows`: the
+// solve's passes read stored row sums; set once its own first pass, whole or
+// in chunks of views in order, has stored them.
+kv_status update_forward(kv_plan *plan, bool mlem, const void *p, const void *x, double *red, float relax, int v0,
+                         int n, bool *rows) {
+    FwdArgs fa{x, p, plan->d_ratio, red, relax};
+    fa.pad = plan->d_pad;
+    fa.pad_ready = v0 > 0;   // view chunks of one volume, the first from view 0
+    if (!mlem) fa.rows = plan->d_rows;
+    const FwdMode mode = mlem ? FWD_MLEM : (*rows ? FWD_SART_ROWS : FWD_SART);
+    if (n == plan->g.n_views) KV_TRY(exact_forward_launch(plan, plan->ex, n, mode, fa));
+    else KV_TRY(exact_forward_views_launch(plan, v0, n, mode, fa));
+    if (mode == FWD_SART && plan->d_rows != nullptr && v0 + n == plan->g.n_views) {
+        keep_rows(plan);
+        *rows = true;
+    }
+    return KV_OK;
 }
 
 // Without a callback (and without tracing) the iteration loop is captured once
 // as a CUDA graph on the context's own stream and launched on the call's
 // stream; the executable graph is kept and relaunched while the buffers and
-// parameters stay the same.
+// parameters stay the same.  SART's first forward pass is launched before the
+// graph, as it may have to store the row sums: the graph begins with its
+// backprojection and is the same for a plan's first solve and the next.
 long long slab_key(const FwdSlabCfg &c) {
     return (((long long)c.R * 16 + c.S) * 8 + c.stages) * 65536 + c.group;
 }
 
-kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem) {
+kv_status iterate_loop(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem, kv_iter_cb cb,
+                       void *user, bool rows, bool projected);
+
+kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem, bool rows) {
     kv_ctx *ctx = plan->ctx;
+    const bool projected = !mlem && plan->family == KV_FAMILY_EXACT;
+    if (projected) KV_TRY(update_forward(plan, mlem, p, x, nullptr, relax, 0, plan->g.n_views, &rows));
     const bool same = plan->graph_exec != nullptr && plan->graph_p == p && plan->graph_x == x &&
                       plan->graph_iters == iters && plan->graph_mlem == (int)mlem && plan->graph_relax == relax &&
                       plan->graph_fb == plan->fwd_by && plan->graph_bb == plan->back_by &&
                       plan->graph_slab == slab_key(plan->fslab) + (slab_key(plan->fpad) << 1) && plan->graph_br == plan->back_rows &&
                       plan->graph_bs == plan->back_slices && plan->graph_vs == plan->back_vs &&
-                      plan->graph_rows == (int)(!mlem && plan->rows_valid) &&
+                      plan->graph_rows == (int)rows &&
                       plan->graph_bst == plan->bstage.R * 16 + plan->bstage.stages;
     if (!same) {
-        const bool had_rows = plan->rows_valid;
         if (plan->graph_exec != nullptr) {
             KV_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             cudaGraphExecDestroy(plan->graph_exec);
@@ -861,7 +891,7 @@ kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float 
         cudaStream_t user_stream = ctx->stream;
         ctx->stream = ctx->own_stream;
         KV_CHECK_CUDA(ctx, cudaStreamBeginCapture(ctx->own_stream, cudaStreamCaptureModeThreadLocal));
-        kv_status s = iterate(plan, p, x, iters, relax, mlem, nullptr, nullptr);
+        kv_status s = iterate_loop(plan, p, x, iters, relax, mlem, nullptr, nullptr, rows, projected);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->own_stream, &graph);
         ctx->stream = user_stream;
@@ -887,11 +917,10 @@ kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float 
         plan->graph_br = plan->back_rows;
         plan->graph_bs = plan->back_slices;
         plan->graph_vs = plan->back_vs;
-        plan->graph_rows = (int)(!mlem && had_rows);
+        plan->graph_rows = (int)rows;
         plan->graph_bst = plan->bstage.R * 16 + plan->bstage.stages;
     }
     KV_CHECK_CUDA(ctx, cudaGraphLaunch(plan->graph_exec, ctx->stream));
-    if (!mlem && plan->family == KV_FAMILY_EXACT) mark_rows(plan);
     return KV_OK;
 }
 
@@ -900,22 +929,26 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
     kv_ctx *ctx = plan->ctx;
     const size_t es = kv_storage_bytes(plan->storage);
     KV_TRY(ensure(ctx, &plan->d_ratio, plan->nproj * es));
+    bool rows = false;
     if (plan->family == KV_FAMILY_EXACT) {
         KV_TRY(ensure_sens(plan));
         ensure_pad(plan);
-        if (!mlem) ensure_rows(plan);
+        if (!mlem) rows = ready_rows(plan);
     }
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(ctx->stream, &cs);
-    if (cb == nullptr && !ctx->timing && iters >= 2 && cs == cudaStreamCaptureStatusNone)
-        return iterate_graph(plan, p, x, iters, relax, mlem);
-    const bool had_rows = plan->rows_valid;
+    if (cb == nullptr && !ctx->timing && iters >= 2 && !stream_capturing(ctx))
+        return iterate_graph(plan, p, x, iters, relax, mlem, rows);
+    return iterate_loop(plan, p, x, iters, relax, mlem, cb, user, rows, false);
+}
+
+// The loop itself; projected: the first iteration's forward pass (EXACT) has been launched.
+kv_status iterate_loop(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem, kv_iter_cb cb,
+                       void *user, bool rows, bool projected) {
+    kv_ctx *ctx = plan->ctx;
     for (int it = 0; it < iters; ++it) {
-        if (plan->family == KV_FAMILY_EXACT) {
-            FwdArgs fa{x, p, plan->d_ratio, cb ? ctx->d_red : nullptr, relax};
-            fa.pad = plan->d_pad;
-            KV_TRY(exact_forward_launch(plan, plan->ex, plan->g.n_views, mlem ? FWD_MLEM : sart_mode(plan, fa), fa));
-            if (!mlem) mark_rows(plan);
+        if (projected && it == 0) {
+            // launched before the loop
+        } else if (plan->family == KV_FAMILY_EXACT) {
+            KV_TRY(update_forward(plan, mlem, p, x, cb ? ctx->d_red : nullptr, relax, 0, plan->g.n_views, &rows));
         } else if (cb) {
             KV_TRY(rc_forward_launch(plan, plan->d_src, plan->d_org, plan->g.n_views, RC_PLAIN, (const float *)x,
                                      nullptr, (float *)plan->d_ratio, relax));
@@ -938,7 +971,6 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
             KV_TRY(rc_back_launch(plan, mlem ? RC_MLEM : RC_ART, (const float *)plan->d_ratio, (float *)x));
         }
     }
-    if (cs != cudaStreamCaptureStatusNone) plan->rows_valid = had_rows;   // captured, not run
     return KV_OK;
 }
 
@@ -954,15 +986,8 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
 // The fused update step of either family on views [v0, v0 + n) (forward +
 // ratio) and on slices [z0, z0 + n) (backprojection + update).
 kv_status update_forward_views(kv_plan *plan, bool mlem, const float *pd, const float *xd, float relax, int v0,
-                               int n) {
-    if (plan->family == KV_FAMILY_EXACT) {
-        FwdArgs fa{xd, pd, plan->d_ratio, nullptr, relax};
-        fa.pad = plan->d_pad;
-        fa.pad_ready = v0 > 0;   // view chunks of one volume, the first from view 0
-        KV_TRY(exact_forward_views_launch(plan, v0, n, mlem ? FWD_MLEM : sart_mode(plan, fa), fa));
-        if (!mlem && v0 + n == plan->g.n_views) mark_rows(plan);   // chunks in order
-        return KV_OK;
-    }
+                               int n, bool *rows) {
+    if (plan->family == KV_FAMILY_EXACT) return update_forward(plan, mlem, pd, xd, nullptr, relax, v0, n, rows);
     const size_t off = (size_t)v0 * plan->g.nu * plan->g.nv;
     return rc_forward_launch(plan, plan->d_src + 3 * (size_t)v0, plan->d_org + 3 * (size_t)v0, n,
                              mlem ? RC_MLEM : RC_ART, xd, pd + off, (float *)plan->d_ratio + off, relax);
@@ -975,7 +1000,8 @@ kv_status update_back_slab(kv_plan *plan, bool mlem, float *xd, float relax, int
     return rc_back_slab_launch(plan, mlem ? RC_MLEM : RC_ART, (const float *)plan->d_ratio, xd, z0, n);
 }
 
-kv_status overlapped_body(kv_plan *plan, const float *proj, float *volume, int iters, float relax, bool mlem) {
+kv_status overlapped_body(kv_plan *plan, const float *proj, float *volume, int iters, float relax, bool mlem,
+                          bool rows) {
     kv_ctx *ctx = plan->ctx;
     const kv_geometry &g = plan->g;
     const size_t D = (size_t)g.nu * g.nv, plane = (size_t)g.nx * g.ny;
@@ -993,12 +1019,12 @@ kv_status overlapped_body(kv_plan *plan, const float *proj, float *volume, int i
                                            cudaMemcpyHostToDevice, cs));
         KV_CHECK_CUDA(ctx, cudaEventRecord(ev[1 + c], cs));
         KV_CHECK_CUDA(ctx, cudaStreamWaitEvent(st, ev[1 + c], 0));
-        KV_TRY(update_forward_views(plan, mlem, pd, xd, relax, v0, n));
+        KV_TRY(update_forward_views(plan, mlem, pd, xd, relax, v0, n, &rows));
     }
     if (iters > 1) {
         KV_TRY(update_back_slab(plan, mlem, xd, relax, 0, g.nz));
         if (iters > 2) KV_TRY(iterate(plan, pd, xd, iters - 2, relax, mlem, nullptr, nullptr));
-        KV_TRY(update_forward_views(plan, mlem, pd, xd, relax, 0, g.n_views));
+        KV_TRY(update_forward_views(plan, mlem, pd, xd, relax, 0, g.n_views, &rows));
     }
     auto back = [&](int z0, int n) { return update_back_slab(plan, mlem, xd, relax, z0, n); };
     return pieces_to_host_body(ctx, g.nz, plane, xd, volume, 1 + kOverlapChunks, back);
@@ -1009,13 +1035,14 @@ kv_status driver_overlapped(kv_plan *plan, const float *proj, float *volume, int
     KV_TRY(ensure(ctx, &plan->d_proj32, plan->nproj * sizeof(float)));
     KV_TRY(ensure(ctx, &plan->d_vol32, plan->nvox * sizeof(float)));
     KV_TRY(ensure(ctx, &plan->d_ratio, plan->nproj * sizeof(float)));
+    bool rows = false;
     if (plan->family == KV_FAMILY_EXACT) {
         KV_TRY(ensure_sens(plan));
         ensure_pad(plan);
-        if (!mlem) ensure_rows(plan);
+        if (!mlem) rows = ready_rows(plan);
     }
     KV_TRY(ensure_copy_stream(ctx));
-    return sync_both(ctx, overlapped_body(plan, proj, volume, iters, relax, mlem));
+    return sync_both(ctx, overlapped_body(plan, proj, volume, iters, relax, mlem, rows));
 }
 
 kv_status driver(kv_plan *plan, const float *proj, float *volume, int iters, float relax, kv_mem mem,
@@ -1160,6 +1187,7 @@ extern "C" kv_status kv_plan_set_slab(kv_plan *plan, int rays_per_thread, int sl
     if (plan == nullptr) return KV_ERR_INVALID_ARG;
     if (plan->family != KV_FAMILY_EXACT)
         return kv_fail(plan->ctx, KV_ERR_UNSUPPORTED, "the slab forward projector is an EXACT-family kernel");
+    plan->rows_gen = -1;   // another kernel rounds the row sums its own way
     if (rays_per_thread == 0) {
         plan->fslab = plan->fpad = FwdSlabCfg{};
         return KV_OK;

@@ -1272,6 +1272,7 @@ kv_status exact_autotune(kv_plan *plan) {
         plan->fwd_by = r.fwd_by;
         plan->back_by = r.back_by;
         plan->fslab = r.fslab;
+        plan->rows_gen = -1;
         plan->back_rows = r.back_rows;
         plan->back_slices = r.back_slices;
         plan->back_vs = 1;

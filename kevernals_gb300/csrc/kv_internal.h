@@ -29,6 +29,7 @@ struct kv_ctx {
     std::string last_error;
     double *d_red = nullptr;         // 8 doubles for FP64 reductions
     int *d_status = nullptr;         // error bits set by kernels that check themselves (0: fine)
+    int status_gen = 0;              // errors read from d_status so far
     // lifetime: plans hold a reference; kv_ctx_destroy only releases the
     // caller's, the context is freed with its last plan
     int plans = 0;
@@ -134,7 +135,7 @@ struct kv_plan {
     float *d_proj32 = nullptr;
     void *d_pad = nullptr;           // volume with padded rows (fpad)
     float *d_rows = nullptr;         // A 1, SART's row sums (EXACT)
-    bool rows_valid = false;
+    int rows_gen = -1;                  // the context's status_gen when d_rows was stored (-1: not stored)
     cudaEvent_t rows_event = nullptr;   // recorded behind the pass that stored d_rows
     double *d_sens = nullptr;        // A^T 1 in FP64 (EXACT)
     bool sens_valid = false;
