@@ -1131,22 +1131,48 @@ extern "C" kv_status kv_batch_mlem(kv_ctx *ctx, int n, kv_plan *const *plans, co
         if (pl->family != KV_FAMILY_EXACT || pl->storage != KV_STORAGE_F32)
             return kv_fail(ctx, KV_ERR_UNSUPPORTED, "kv_batch_mlem: EXACT / FP32 plans only (plan %d)", i);
     }
+    // A plan's staging buffers serve one of its problems; further problems of a
+    // plan on host buffers get buffers of their own.
     std::vector<const float *> pd(n);
-    std::vector<float *> xd(n);
-    for (int i = 0; i < n; ++i) {
-        kv_plan *pl = plans[i];
-        KV_TRY(ensure(ctx, &pl->d_ratio, pl->nproj * sizeof(float)));
-        KV_TRY(ensure_sens(pl));
-        ensure_pad(pl);
-        float *a, *b;
-        KV_TRY(stage_in(pl, projections[i], mem, &pl->d_proj32, pl->nproj, true, &a));
-        KV_TRY(stage_in(pl, volumes[i], mem, &pl->d_vol32, pl->nvox, true, &b));
-        pd[i] = a;
-        xd[i] = b;
-    }
-    if (iterations > 0) KV_TRY(exact_batch_mlem_launch(ctx, n, plans, pd.data(), xd.data(), iterations, relax));
-    for (int i = 0; i < n; ++i) KV_TRY(stage_out(plans[i], volumes[i], mem, xd[i], plans[i]->nvox));
-    return KV_OK;
+    std::vector<float *> xd(n), own;
+    auto body = [&]() -> kv_status {
+        auto buffer = [&](size_t elems, float **out) -> kv_status {
+            KV_CHECK_CUDA(ctx, cudaMallocAsync((void **)out, elems * sizeof(float), ctx->stream));
+            own.push_back(*out);
+            return KV_OK;
+        };
+        for (int i = 0; i < n; ++i) {
+            kv_plan *pl = plans[i];
+            KV_TRY(ensure(ctx, &pl->d_ratio, pl->nproj * sizeof(float)));
+            KV_TRY(ensure_sens(pl));
+            ensure_pad(pl);
+            float *a = const_cast<float *>(projections[i]), *b = volumes[i];
+            if (mem == KV_MEM_HOST) {
+                const bool first = std::find(plans, plans + i, pl) == plans + i;
+                float *ta = nullptr, *tb = nullptr;
+                if (!first) {
+                    KV_TRY(buffer(pl->nproj, &ta));
+                    KV_TRY(buffer(pl->nvox, &tb));
+                }
+                KV_TRY(stage_in(pl, projections[i], mem, first ? &pl->d_proj32 : &ta, pl->nproj, true, &a));
+                KV_TRY(stage_in(pl, volumes[i], mem, first ? &pl->d_vol32 : &tb, pl->nvox, true, &b));
+            }
+            pd[i] = a;
+            xd[i] = b;
+        }
+        if (iterations > 0) KV_TRY(exact_batch_mlem_launch(ctx, n, plans, pd.data(), xd.data(), iterations, relax));
+        for (int i = 0; i < n; ++i)
+            if (xd[i] != volumes[i])
+                KV_CHECK_CUDA(ctx, cudaMemcpyAsync(volumes[i], xd[i], plans[i]->nvox * sizeof(float),
+                                                   mem == KV_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice,
+                                                   ctx->stream));
+        return KV_OK;
+    };
+    kv_status st = body();
+    for (float *b : own) cudaFreeAsync(b, ctx->stream);
+    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess && st == KV_OK) st = kv_fail(ctx, KV_ERR_CUDA, "batch sync");
+    KV_TRY(st);
+    return device_status(ctx);
 }
 
 extern "C" kv_status kv_plan_autotune(kv_plan *plan) {

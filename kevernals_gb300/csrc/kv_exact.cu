@@ -1093,7 +1093,6 @@ kv_status exact_batch_mlem_launch(kv_ctx *ctx, int n, kv_plan *const *plans, con
             cudaStreamSynchronize(ctx->side_streams[s]);
             if (st == KV_OK) st = kv_fail(ctx, KV_ERR_CUDA, "batch join");
         }
-    if (cudaStreamSynchronize(user) != cudaSuccess && st == KV_OK) st = kv_fail(ctx, KV_ERR_CUDA, "batch sync");
     return st;
 }
 

@@ -1,0 +1,48 @@
+"""kv_batch_mlem against one kv_mlem after another, bit for bit: repeated plans, rows that are not whole 16-byte units,
+more problems than side streams."""
+import numpy as np
+import pytest
+
+from kevernals_gb300 import build, engine
+from kevernals_gb300.geometry import linear_sweep
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    build.build()
+    return engine.Context(0)
+
+
+def problems(ctx):
+    """Twelve problems on seven plans; the first plan four times, the second three."""
+    plans = [engine.Plan(ctx, linear_sweep(nx, 28 + 4 * i, 6 + i, 0.5, 0.5, 1.0, 5 + i, 40 + 8 * i, 44, 0.4, 0.4, 15.0),
+                         "exact") for i, nx in enumerate((32, 33, 24, 41, 64, 30, 17))]
+    pick = [0, 1, 0, 2, 3, 1, 4, 0, 5, 6, 1, 0]
+    rng = np.random.default_rng(9)
+    data = [rng.random(plans[k].geometry.proj_shape, dtype=np.float32) for k in pick]
+    return [plans[k] for k in pick], data
+
+
+@pytest.mark.parametrize("host", [True, False])
+@pytest.mark.parametrize("iterations", [0, 1, 4])
+def test_batch_equals_one_by_one(ctx, host, iterations):
+    torch = pytest.importorskip("torch")
+    plans, data = problems(ctx)
+    start = [np.full(p.geometry.volume_shape, 0.5 + 0.1 * i, np.float32) for i, p in enumerate(plans)]
+    want = []
+    for plan, p, x0 in zip(plans, data, start):
+        x = x0.copy()
+        if iterations:
+            plan.mlem(p, x, iterations, 0.9)
+        want.append(x)
+    if host:
+        xs = [x.copy() for x in start]
+        engine.batch_mlem(ctx, plans, data, xs, iterations, 0.9)
+    else:
+        xs = [torch.from_numpy(x).cuda() for x in start]
+        engine.batch_mlem(ctx, plans, [torch.from_numpy(p).cuda() for p in data], xs, iterations, 0.9)
+        xs = [x.cpu().numpy() for x in xs]
+    for i, (x, w) in enumerate(zip(xs, want)):
+        assert np.array_equal(x, w), i
