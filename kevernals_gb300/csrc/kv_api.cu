@@ -1132,7 +1132,8 @@ extern "C" kv_status kv_batch_mlem(kv_ctx *ctx, int n, kv_plan *const *plans, co
             return kv_fail(ctx, KV_ERR_UNSUPPORTED, "kv_batch_mlem: EXACT / FP32 plans only (plan %d)", i);
     }
     // A plan's staging buffers serve one of its problems; further problems of a
-    // plan on host buffers get buffers of their own.
+    // plan on host buffers, and device volumes that the projector's TMA loads
+    // cannot address (not on a 16-byte boundary), get buffers of their own.
     std::vector<const float *> pd(n);
     std::vector<float *> xd(n), own;
     auto body = [&]() -> kv_status {
@@ -1156,6 +1157,10 @@ extern "C" kv_status kv_batch_mlem(kv_ctx *ctx, int n, kv_plan *const *plans, co
                 }
                 KV_TRY(stage_in(pl, projections[i], mem, first ? &pl->d_proj32 : &ta, pl->nproj, true, &a));
                 KV_TRY(stage_in(pl, volumes[i], mem, first ? &pl->d_vol32 : &tb, pl->nvox, true, &b));
+            } else if (reinterpret_cast<uintptr_t>(b) % 16 != 0) {
+                KV_TRY(buffer(pl->nvox, &b));
+                KV_CHECK_CUDA(ctx, cudaMemcpyAsync(b, volumes[i], pl->nvox * sizeof(float), cudaMemcpyDeviceToDevice,
+                                                   ctx->stream));
             }
             pd[i] = a;
             xd[i] = b;

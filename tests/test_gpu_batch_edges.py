@@ -1,5 +1,5 @@
 """kv_batch_mlem against one kv_mlem after another, bit for bit: repeated plans, rows that are not whole 16-byte units,
-more problems than side streams."""
+more problems than side streams, volumes at any address."""
 import numpy as np
 import pytest
 
@@ -46,3 +46,19 @@ def test_batch_equals_one_by_one(ctx, host, iterations):
         xs = [x.cpu().numpy() for x in xs]
     for i, (x, w) in enumerate(zip(xs, want)):
         assert np.array_equal(x, w), i
+
+
+def test_batch_takes_volumes_at_any_address(ctx):
+    """Device volumes that start 4 bytes past a 16-byte boundary."""
+    torch = pytest.importorskip("torch")
+    plans, data = problems(ctx)
+    want, xs = [], []
+    for plan, p in zip(plans, data):
+        x = np.ones(plan.geometry.volume_shape, np.float32)
+        plan.mlem(p, x, 3)
+        want.append(x)
+        n = x.size
+        xs.append(torch.ones(n + 1, device="cuda")[1:].view(x.shape))
+    engine.batch_mlem(ctx, plans, [torch.from_numpy(p).cuda() for p in data], xs, 3)
+    for i, (x, w) in enumerate(zip(xs, want)):
+        assert np.array_equal(x.cpu().numpy(), w), i
