@@ -200,8 +200,11 @@ kv_status kv_sart(kv_plan *plan, const float *projections, float *volume_inout, 
  * detector and view counts, all created on `ctx`, run side by side: each goes
  * through its own plan's kernels on one of the context's side streams, which
  * fork from and join the context's stream.  Results are identical to
- * calling kv_mlem on each plan.  No reference counterpart (the reference
- * reconstructs one case per call).  projections[i] / volumes[i] are host or
+ * calling kv_mlem on each plan, but where eight or more problems are tiny
+ * (rays x slices + 0.3 x voxels x views at most 4e5): those share persistent
+ * kernels, which sum in another order (a few roundings).  A plan may appear
+ * more than once.  No reference counterpart (the reference reconstructs one
+ * case per call).  projections[i] / volumes[i] are host or
  * device buffers according to `mem`; volumes are updated in place. */
 kv_status kv_batch_mlem(kv_ctx *ctx, int n, kv_plan *const *plans, const float *const *projections,
                         float *const *volumes, int iterations, float relax, kv_mem mem);

@@ -332,6 +332,7 @@ void ctx_free(kv_ctx *ctx) {
         cudaStreamDestroy(s);
     }
     for (cudaEvent_t e : ctx->side_events) cudaEventDestroy(e);
+    cudaFree(ctx->d_batch);
     cudaFree(ctx->d_red);
     cudaFree(ctx->d_status);
     cudaStreamDestroy(ctx->own_stream);

@@ -1020,13 +1020,89 @@ extern "C" kv_status kv_residual_noalloc(kv_plan *plan, const float *projections
 // side, each through its own plan's kernels, on a few side streams of the
 // context: largest first, every problem to the stream with the least work so
 // far (a plan that appears twice stays on one stream: its workspaces serve one
-// solve at a time).  Results are those of solving one by one, bit for bit.
-// Persistent kernels over all problems' tiles, which this replaces, had to use
-// the one-ray and one-voxel-a-thread tiles: 32 problems of up to 128 x 128 x
-// 24 voxels, 5 iterations: 14.5 -> 7.4 ms.
+// solve at a time).  Those results are those of solving one by one, bit for
+// bit.  32 problems of up to 128 x 128 x 24 voxels, 5 iterations: 14.5 ms with
+// persistent kernels over all problems' tiles -> 7.2.
+//
+// Problems too small to be worth two launches an iteration (some 2.6 us of
+// host each) share persistent kernels: their tiles are pulled from a device
+// counter, found by binary search over the problems' first tile indices, and
+// run through the one-thread-per-ray and one-thread-per-voxel tile functions
+// (another order of the sums than the plan's own kernels: a few roundings).
+// Work, rays x slices + 0.3 voxels x views, a problem: 2.6e4, 64 problems, 20
+// iterations 2.0 ms (own launches 6.6, one iteration as a graph 3.5), 256
+// problems, 5 iterations 4.2 (9.0, 6.8), 8 problems, 20 iterations 0.72 (1.14,
+// 0.84); 3.8e5, 256 problems, 5 iterations 8.6 (9.0); 5.2e5, 32 problems, 10
+// iterations 2.9 (2.2).
 namespace {
 
 constexpr int kSideStreams = 8;
+constexpr double kTinyWork = 4e5;   // see above
+constexpr int kTinyCount = 8;
+
+struct BatchItem {
+    ExGeom G;
+    ExactTables T;
+    const float *p;        // measured projections
+    float *x;              // iterate (updated in place)
+    float *ratio;          // forward output: Ls * relax * p / Ax
+    const double *sens;    // A^T 1
+    int ftx, fty;          // forward tiles per view (u, v)
+    int btx, bty;          // backprojection tiles per slice (i, j)
+    long long f0, b0;      // first forward / backprojection tile of this problem
+};
+
+__device__ __forceinline__ int batch_find(const BatchItem *items, int n, long long tile, bool fwd) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        const long long start = fwd ? items[mid].f0 : items[mid].b0;
+        if (start <= tile) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+__global__ void __launch_bounds__(256) batch_fwd_kernel(const BatchItem *__restrict__ items, int n,
+                                                        long long total, unsigned long long *counter,
+                                                        float relax) {
+    __shared__ long long s_tile;
+    while (true) {
+        if (threadIdx.x == 0 && threadIdx.y == 0) s_tile = (long long)atomicAdd(counter, 1ull);
+        __syncthreads();
+        const long long tile = s_tile;
+        __syncthreads();
+        if (tile >= total) return;
+        const BatchItem &B = items[batch_find(items, n, tile, true)];
+        const long long local = tile - B.f0;
+        const long long per_view = (long long)B.ftx * B.fty;
+        const int p = (int)(local / per_view);
+        const int rem = (int)(local % per_view);
+        FwdArgs a{B.x, B.p, B.ratio, nullptr, relax};
+        fwd_tile<float, float, FWD_MLEM>(B.G, B.T, a, nullptr, rem % B.ftx, rem / B.ftx, p, 0);
+    }
+}
+
+__global__ void __launch_bounds__(256) batch_back_kernel(const BatchItem *__restrict__ items, int n,
+                                                         long long total, unsigned long long *counter,
+                                                         float relax) {
+    __shared__ long long s_tile;
+    while (true) {
+        if (threadIdx.x == 0 && threadIdx.y == 0) s_tile = (long long)atomicAdd(counter, 1ull);
+        __syncthreads();
+        const long long tile = s_tile;
+        __syncthreads();
+        if (tile >= total) return;
+        const BatchItem &B = items[batch_find(items, n, tile, false)];
+        const long long local = tile - B.b0;
+        const long long per_slice = (long long)B.btx * B.bty;
+        const int k = (int)(local / per_slice);
+        const int rem = (int)(local % per_slice);
+        BackArgs a{B.ratio, B.x, B.sens, relax};
+        back_tile<float, float, ACC_F32, BACK_MLEM>(B.G, B.T, a, nullptr, rem % B.btx, rem / B.btx, k);
+        __syncwarp();
+    }
+}
 
 kv_status ensure_side_streams(kv_ctx *ctx) {
     while ((int)ctx->side_streams.size() < kSideStreams) {
@@ -1044,40 +1120,114 @@ kv_status ensure_side_streams(kv_ctx *ctx) {
 
 }  // namespace
 
+namespace {
+
+// The tiny problems' persistent kernels on the context's current stream; d_items holds n items, then two counters.
+kv_status batch_tiny_launch(kv_ctx *ctx, const std::vector<BatchItem> &items, long long f, long long b,
+                            BatchItem *d_items, int iters, float relax, int by, int bb) {
+    const int n = (int)items.size();
+    unsigned long long *counter = reinterpret_cast<unsigned long long *>(d_items + n);
+    cudaStream_t st = ctx->stream;
+    int occ_f = 0, occ_b = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, batch_fwd_kernel, 32 * by, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, batch_back_kernel, 32 * bb, 0);
+    const unsigned grid_f = (unsigned)std::min<long long>(f, (long long)ctx->sm_count * std::max(1, occ_f));
+    const unsigned grid_b = (unsigned)std::min<long long>(b, (long long)ctx->sm_count * std::max(1, occ_b));
+    KV_CHECK_CUDA(ctx, cudaMemcpyAsync(d_items, items.data(), n * sizeof(BatchItem), cudaMemcpyHostToDevice, st));
+    for (int it = 0; it < iters; ++it) {
+        KV_CHECK_CUDA(ctx, cudaMemsetAsync(counter, 0, 2 * sizeof *counter, st));
+        {
+            LaunchTimer lt(ctx, "batch_fwd");
+            batch_fwd_kernel<<<grid_f, dim3(32, by), 0, st>>>(d_items, n, f, counter, relax);
+        }
+        LaunchTimer lt(ctx, "batch_back");
+        batch_back_kernel<<<grid_b, dim3(32, bb), 0, st>>>(d_items, n, b, counter + 1, relax);
+    }
+    KV_CHECK_LAUNCH(ctx, "batch kernels");
+    return KV_OK;
+}
+
+}  // namespace
+
 // `iters` MLEM iterations of every problem, forked from and joined to the
 // context stream.  Plans must be EXACT / FP32 with their sensitivity images
 // computed and workspaces allocated; p[i] / x[i] are device buffers.
 kv_status exact_batch_mlem_launch(kv_ctx *ctx, int n, kv_plan *const *plans, const float *const *p,
                                   float *const *x, int iters, float relax) {
     KV_TRY(ensure_side_streams(ctx));
-    std::vector<int> order(n), stream_of(n);
+    std::vector<int> order(n), stream_of(n, -1);
+    std::vector<char> tiny(n);
     std::vector<double> cost(n), load(kSideStreams, 0.0);
+    int n_tiny = 0;
     for (int i = 0; i < n; ++i) {
         const kv_geometry &g = plans[i]->g;
         order[i] = i;
         cost[i] = (double)plans[i]->nproj * g.nz + 0.3 * (double)plans[i]->nvox * g.n_views;
+        // the first problem of its plan only: the persistent kernels run all at once
+        tiny[i] = cost[i] <= kTinyWork && std::find(plans, plans + i, plans[i]) == plans + i;
+        n_tiny += tiny[i];
     }
+    if (n_tiny < kTinyCount) std::fill(tiny.begin(), tiny.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    // the tiny problems, and later problems of their plans behind them, on stream 0
+    const int by = plans[0]->fwd_by, bb = plans[0]->back_by;
+    std::vector<BatchItem> items;
+    long long f = 0, b = 0;
+    for (int i = 0; i < n; ++i) {
+        if (!tiny[i]) continue;
+        const kv_plan *pl = plans[i];
+        BatchItem it;
+        it.G = exgeom(pl, pl->g.n_views);
+        it.T = pl->ex;
+        it.p = p[i];
+        it.x = x[i];
+        it.ratio = static_cast<float *>(pl->d_ratio);
+        it.sens = pl->d_sens;
+        it.ftx = (pl->g.nu + 31) / 32;
+        it.fty = (pl->g.nv + by - 1) / by;
+        it.btx = (pl->g.nx + 31) / 32;
+        it.bty = (pl->g.ny + bb - 1) / bb;
+        it.f0 = f;
+        it.b0 = b;
+        f += (long long)it.ftx * it.fty * pl->g.n_views;
+        b += (long long)it.btx * it.bty * pl->g.nz;
+        items.push_back(it);
+        stream_of[i] = 0;
+        load[0] += cost[i];
+    }
     for (int k = 0; k < n; ++k) {
         const int i = order[k];
+        if (tiny[i]) continue;
         int s = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        for (int m = 0; m < k; ++m)
-            if (plans[order[m]] == plans[i]) s = stream_of[order[m]];
+        for (int m = 0; m < n; ++m)
+            if (plans[m] == plans[i] && stream_of[m] >= 0) s = stream_of[m];
         stream_of[i] = s;
         load[s] += cost[i];
     }
+    // their descriptors and the two tile counters: a buffer that the context keeps (the call waits for its kernels)
+    const size_t bytes = items.size() * sizeof(BatchItem) + 2 * sizeof(unsigned long long);
+    if (!items.empty() && ctx->batch_bytes < bytes) {
+        cudaFree(ctx->d_batch);
+        ctx->d_batch = nullptr;
+        ctx->batch_bytes = 0;
+        KV_CHECK_CUDA(ctx, cudaMalloc(&ctx->d_batch, bytes));
+        ctx->batch_bytes = bytes;
+    }
     cudaStream_t user = ctx->stream;
     cudaEvent_t fork = ctx->side_events[kSideStreams];
-    KV_CHECK_CUDA(ctx, cudaEventRecord(fork, user));
-    kv_status st = KV_OK;
+    kv_status st = cudaEventRecord(fork, user) == cudaSuccess ? KV_OK : kv_fail(ctx, KV_ERR_CUDA, "batch fork");
+    for (int s = 0; s < kSideStreams && st == KV_OK; ++s)
+        if (cudaStreamWaitEvent(ctx->side_streams[s], fork, 0) != cudaSuccess)
+            st = kv_fail(ctx, KV_ERR_CUDA, "batch fork");
+    if (st == KV_OK && !items.empty()) {
+        ctx->stream = ctx->side_streams[0];
+        st = batch_tiny_launch(ctx, items, f, b, static_cast<BatchItem *>(ctx->d_batch), iters, relax, by, bb);
+    }
     for (int k = 0; k < n && st == KV_OK; ++k) {
         const int i = order[k];
+        if (tiny[i]) continue;
         kv_plan *pl = plans[i];
         ctx->stream = ctx->side_streams[stream_of[i]];
-        if (cudaStreamWaitEvent(ctx->stream, fork, 0) != cudaSuccess) {
-            st = kv_fail(ctx, KV_ERR_CUDA, "batch fork");
-            break;
-        }
         for (int it = 0; it < iters && st == KV_OK; ++it) {
             FwdArgs fa{x[i], p[i], pl->d_ratio, nullptr, relax};
             fa.pad = pl->d_pad;

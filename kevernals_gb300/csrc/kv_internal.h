@@ -45,6 +45,8 @@ struct kv_ctx {
     // batched solves: side streams and their join events (created on first use)
     std::vector<cudaStream_t> side_streams;
     std::vector<cudaEvent_t> side_events;
+    void *d_batch = nullptr;         // descriptors of the batch's tiny problems
+    size_t batch_bytes = 0;
 };
 
 // Brackets one kernel launch with CUDA events on the context stream when the
