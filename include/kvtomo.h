@@ -244,7 +244,8 @@ kv_status kv_plan_set_slab(kv_plan *plan, int rays_per_thread, int slices, int s
  * from cache.  Shapes (rows, slices): (1, 1), (2, 1), (2, 2), (4, 1),
  * (4, 2), (8, 1); all give bit-identical volumes.  Rows 0 selects
  * one voxel per thread in blocks of 32 x back_rows of kv_plan_set_tuning.
- * Default (8, 1). */
+ * Default (8, 1).  A volume of few blocks sums each voxel's terms by four or
+ * eight groups of views, in every shape. */
 kv_status kv_plan_get_back_shape(const kv_plan *plan, int *rows_per_thread, int *slices_per_thread);
 kv_status kv_plan_set_back_shape(kv_plan *plan, int rows_per_thread, int slices_per_thread);
 

@@ -1276,7 +1276,6 @@ extern "C" kv_status kv_plan_set_back_shape(kv_plan *plan, int rows_per_thread, 
         return kv_fail(plan->ctx, KV_ERR_INVALID_ARG,
                        "gather backprojector shape must be rows 0, (1, 1), (2, 1), (2, 2), (4, 1), (4, 2) or (8, 1)");
     if (rows_per_thread == 0) slices_per_thread = 1;
-    plan->back_vs = 1;   // a shape asked for is the plain one
     plan->back_rows = rows_per_thread;
     plan->back_slices = slices_per_thread;
     return KV_OK;

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kThreads) exact_back_stage_kernel(const __grid
     if (threadIdx.x == 0)
         for (int p = 0; p < A.stages && p < G.n_views; ++p) issue(p, p);
 
-    // sums by view groups, added in order, where the plan's gather kernel forms them so (A.vs groups; 1: one sum)
+    // sums by view groups, added in order, as the plan's gather kernels form them (A.vs groups; 1: one sum)
     float acc[R], total[R];
 #pragma unroll
     for (int q = 0; q < R; ++q) acc[q] = total[q] = 0.f;
@@ -349,7 +349,7 @@ kv_status back_stage_launch(kv_plan *plan, BackMode mode, const BackArgs &a, int
     A.stage_bytes = (uint32_t)c.BU * c.BV * sizeof(float);
     A.org_off = L.org_off;
     A.status = plan->ctx->d_status;
-    A.vs = plan->back_rows == 8 ? plan->back_vs : 1;
+    A.vs = plan->back_vs;
     const ExGeom G{g.nx, g.ny, g.nz, g.nu, g.nv, n_views};
     dim3 grid(nzs, (g.ny + 8 * c.R - 1) / (8 * c.R), (g.nx + 31) / 32);
     const void *fn = c.R == 8 ? (const void *)exact_back_stage_kernel<8> : (const void *)exact_back_stage_kernel<4>;

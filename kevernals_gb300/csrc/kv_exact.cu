@@ -327,7 +327,7 @@ __device__ __forceinline__ void back_rows(const ProjT *row, int nu, int nvc, con
 
 template <typename VolT, typename ProjT, int ACC, int MODE>
 __device__ __forceinline__ void back_tile(const ExGeom &G, const ExactTables &T, const BackArgs &a,
-                                          double *sens_out, int bx, int by, int k) {
+                                          double *sens_out, int bx, int by, int k, int vs) {
     const int lane = threadIdx.x, warp = threadIdx.y;
     const int i = bx * 32 + lane;
     const int j = by * blockDim.y + warp;
@@ -335,9 +335,13 @@ __device__ __forceinline__ void back_tile(const ExGeom &G, const ExactTables &T,
     const bool live_i = i < G.nx;
     const bool live_j = j < G.ny;   // warp-uniform
     const ProjT *yp = static_cast<const ProjT *>(a.yp);
-    float acc = 0.f, comp = 0.f;
+    float acc = 0.f, comp = 0.f, total = 0.f;   // vs > 1: sums by view groups, added in order
     if (live_j) {
-        for (int p = 0; p < G.n_views; ++p) {
+        for (int p = 0, group = 0; p < G.n_views; ++p) {
+            for (; group + 1 < vs && p == (group + 1) * G.n_views / vs; ++group) {
+                total += acc;
+                acc = 0.f;
+            }
             const float *hr = T.hr + (size_t)p * (G.nz + 1);
             const float htop = hr[k + 1];
             const float4 r0 = T.rng[(size_t)p * (G.nz + 1) + k];
@@ -407,6 +411,7 @@ __device__ __forceinline__ void back_tile(const ExGeom &G, const ExactTables &T,
         }
     }
     if (!live_i || !live_j) return;
+    if (vs > 1) acc = total + acc;
     const size_t idx = ((size_t)k * G.ny + j) * G.nx + i;
     if (sens_out != nullptr) {
         sens_out[idx] = ACC == ACC_DF ? (double)acc + (double)comp : (double)acc;
@@ -428,9 +433,9 @@ __device__ __forceinline__ void back_tile(const ExGeom &G, const ExactTables &T,
 
 template <typename VolT, typename ProjT, int ACC, int MODE>
 __global__ void __launch_bounds__(256) exact_back_kernel(ExGeom G, ExactTables T, BackArgs a,
-                                                         double *sens_out, int z0) {
+                                                         double *sens_out, int z0, int vs) {
     // slices z0 .. z0 + gridDim.z - 1 (z0 = 0 and gridDim.z = nz for the whole volume)
-    back_tile<VolT, ProjT, ACC, MODE>(G, T, a, sens_out, blockIdx.x, blockIdx.y, z0 + (int)blockIdx.z);
+    back_tile<VolT, ProjT, ACC, MODE>(G, T, a, sens_out, blockIdx.x, blockIdx.y, z0 + (int)blockIdx.z, vs);
 }
 
 // ---------------------------------------------------------------------------
@@ -489,20 +494,22 @@ __device__ __forceinline__ void back_chunk_r(const ExGeom &G, const ExactTables 
 }
 
 // VS > 1: the warps are VS groups of views for 8 / VS row warps, so that a volume of few blocks does not leave every
-// warp a chain of all views; the groups' sums meet in shared memory, in the order of the views.
+// warp a chain of all views; the groups' sums meet in shared memory, in the order of the views.  VS = 0: each warp has
+// all views, summed in the same `vs` groups, for the other shapes on such a volume: equal bits whatever the shape.
 template <typename VolT, typename ProjT, int ACC, int R, int S, int VS>
 __device__ __forceinline__ void back_tile_r(const ExGeom &G, const ExactTables &T, const BackArgs &a,
-                                            double *sens_out, int bx, int by, int k0, int kend, int mode) {
+                                            double *sens_out, int bx, int by, int k0, int kend, int mode, int vs) {
     constexpr int CW = 32 / R;                 // candidates of one voxel row filled per pass
-    constexpr int RW = 8 / VS;                 // row warps
-    static_assert(VS == 1 || (S == 1 && ACC == ACC_F32 && R == 8), "view groups: eight rows, one slice, plain sums");
+    constexpr int RW = VS == 0 ? 8 : 8 / (VS == 0 ? 1 : VS);   // row warps
+    static_assert(VS <= 1 || (S == 1 && R == 8), "view groups: eight rows, one slice");
+    static_assert(VS == 1 || ACC == ACC_F32, "view groups: plain sums");
     const int lane = threadIdx.x, warp = threadIdx.y;
     const int i = bx * 32 + lane;
     const int jw = by * RW * R + warp % RW;    // voxel row of q = 0; rows jw + RW q
     const int qf = lane / CW, cf = lane % CW;  // this lane fills candidate cf (+ CW f) of row qf
     const int jf = jw + RW * qf;
-    const int p_begin = VS == 1 ? 0 : warp / RW * G.n_views / VS;
-    const int p_end = VS == 1 ? G.n_views : (warp / RW + 1) * G.n_views / VS;
+    const int p_begin = VS <= 1 ? 0 : warp / RW * G.n_views / (VS == 0 ? 1 : VS);
+    const int p_end = VS <= 1 ? G.n_views : (warp / RW + 1) * G.n_views / (VS == 0 ? 1 : VS);
     __shared__ float2 ysh[8][R][32];
     const bool live_i = i < G.nx;
     const ProjT *yp = static_cast<const ProjT *>(a.yp);
@@ -511,7 +518,23 @@ __device__ __forceinline__ void back_tile_r(const ExGeom &G, const ExactTables &
     for (int kk = 0; kk < S; ++kk)
 #pragma unroll
         for (int q = 0; q < R; ++q) acc[kk][q] = comp[kk][q] = 0.f;
+    float total[VS == 0 ? S : 1][R];   // VS == 0: the groups before this one
+    int group = 0;
+#pragma unroll
+    for (int kk = 0; kk < (VS == 0 ? S : 1); ++kk)
+#pragma unroll
+        for (int q = 0; q < R; ++q) total[kk][q] = 0.f;
     for (int p = p_begin; p < p_end; ++p) {
+        if constexpr (VS == 0) {
+            for (; group + 1 < vs && p == (group + 1) * G.n_views / vs; ++group)
+#pragma unroll
+                for (int kk = 0; kk < S; ++kk)
+#pragma unroll
+                    for (int q = 0; q < R; ++q) {
+                        total[kk][q] += acc[kk][q];
+                        acc[kk][q] = 0.f;
+                    }
+        }
 #pragma unroll
         for (int kk = 0; kk < S; ++kk) {
             const int k = k0 + kk;
@@ -583,7 +606,13 @@ __device__ __forceinline__ void back_tile_r(const ExGeom &G, const ExactTables &
             }
         }
     }
-    if (VS > 1) {
+    if constexpr (VS == 0) {
+#pragma unroll
+        for (int kk = 0; kk < S; ++kk)
+#pragma unroll
+            for (int q = 0; q < R; ++q) acc[kk][q] = total[kk][q] + acc[kk][q];
+    }
+    if constexpr (VS > 1) {
         // warp (g, w) takes rows q = g R / VS .. of row warp w, the groups' sums added in order
         constexpr int QN = R / VS;
         __shared__ float part[8][R][32];
@@ -604,8 +633,8 @@ __device__ __forceinline__ void back_tile_r(const ExGeom &G, const ExactTables &
         const int k = k0 + kk;
         if (k >= kend) break;
 #pragma unroll
-        for (int q = 0; q < R / VS; ++q) {
-            const int j = jw + RW * (VS == 1 ? q : warp / RW * (R / VS) + q);
+        for (int q = 0; q < (VS <= 1 ? R : R / (VS == 0 ? 1 : VS)); ++q) {
+            const int j = jw + RW * (VS <= 1 ? q : warp / RW * (R / (VS == 0 ? 1 : VS)) + q);
             if (j >= G.ny) continue;
             const size_t idx = ((size_t)k * G.ny + j) * G.nx + i;
             if (sens_out != nullptr) {
@@ -638,9 +667,9 @@ __device__ __forceinline__ void back_tile_r(const ExGeom &G, const ExactTables &
 // kernel argument, not a template parameter.
 template <typename VolT, typename ProjT, int ACC, int R, int S, int VS>
 __global__ void __launch_bounds__(256) exact_back_r_kernel(ExGeom G, ExactTables T, BackArgs a,
-                                                           double *sens_out, int z0, int nzs, int mode) {
+                                                           double *sens_out, int z0, int nzs, int mode, int vs) {
     back_tile_r<VolT, ProjT, ACC, R, S, VS>(G, T, a, sens_out, blockIdx.z, blockIdx.y, z0 + S * (int)blockIdx.x,
-                                        z0 + nzs, mode);
+                                        z0 + nzs, mode, vs);
 }
 
 ExGeom exgeom(const kv_plan *plan, int n_views) {
@@ -767,23 +796,36 @@ kv_status fwd_dispatch(kv_plan *plan, const ExactTables &t, int P, FwdMode mode,
     return KV_OK;
 }
 
-template <typename VolT, typename ProjT, int ACC, int R, int S, int VS = 1>
+template <typename VolT, typename ProjT, int ACC, int R, int S, int VS>
 void back_r_launch(const ExGeom &G, const ExactTables &t, BackMode mode, const BackArgs &a, double *sens_out,
-                   int z0, int nzs, cudaStream_t st) {
-    dim3 block(32, 8), grid((nzs + S - 1) / S, (G.ny + 8 / VS * R - 1) / (8 / VS * R), (G.nx + 31) / 32);
-    exact_back_r_kernel<VolT, ProjT, ACC, R, S, VS><<<grid, block, 0, st>>>(G, t, a, sens_out, z0, nzs, (int)mode);
+                   int z0, int nzs, int vs, cudaStream_t st) {
+    constexpr int rows = VS > 1 ? 8 / (VS == 0 ? 1 : VS) * R : 8 * R;   // of a block
+    dim3 block(32, 8), grid((nzs + S - 1) / S, (G.ny + rows - 1) / rows, (G.nx + 31) / 32);
+    exact_back_r_kernel<VolT, ProjT, ACC, R, S, VS><<<grid, block, 0, st>>>(G, t, a, sens_out, z0, nzs, (int)mode, vs);
 }
 
-// (rows per thread, slices per thread): (1, 1), (2, 1), (2, 2), (4, 1), (4, 2) or (8, 1)
+// (rows per thread, slices per thread): (1, 1), (2, 1), (2, 2), (4, 1), (4, 2) or (8, 1); vs: groups of views
 template <typename VolT, typename ProjT, int ACC>
 void back_r_dispatch(int R, int S, const ExGeom &G, const ExactTables &t, BackMode mode, const BackArgs &a,
-                     double *sens_out, int z0, int nzs, cudaStream_t st) {
-    if (R == 1) back_r_launch<VolT, ProjT, ACC, 1, 1>(G, t, mode, a, sens_out, z0, nzs, st);
-    else if (R == 2 && S == 1) back_r_launch<VolT, ProjT, ACC, 2, 1>(G, t, mode, a, sens_out, z0, nzs, st);
-    else if (R == 2) back_r_launch<VolT, ProjT, ACC, 2, 2>(G, t, mode, a, sens_out, z0, nzs, st);
-    else if (R == 4 && S == 1) back_r_launch<VolT, ProjT, ACC, 4, 1>(G, t, mode, a, sens_out, z0, nzs, st);
-    else if (R == 4) back_r_launch<VolT, ProjT, ACC, 4, 2>(G, t, mode, a, sens_out, z0, nzs, st);
-    else back_r_launch<VolT, ProjT, ACC, 8, 1>(G, t, mode, a, sens_out, z0, nzs, st);
+                     double *sens_out, int z0, int nzs, int vs, cudaStream_t st) {
+    if constexpr (ACC == ACC_F32) {
+        if (vs > 1) {
+            if (R == 1) back_r_launch<VolT, ProjT, ACC, 1, 1, 0>(G, t, mode, a, sens_out, z0, nzs, vs, st);
+            else if (R == 2 && S == 1) back_r_launch<VolT, ProjT, ACC, 2, 1, 0>(G, t, mode, a, sens_out, z0, nzs, vs, st);
+            else if (R == 2) back_r_launch<VolT, ProjT, ACC, 2, 2, 0>(G, t, mode, a, sens_out, z0, nzs, vs, st);
+            else if (R == 4 && S == 1) back_r_launch<VolT, ProjT, ACC, 4, 1, 0>(G, t, mode, a, sens_out, z0, nzs, vs, st);
+            else if (R == 4) back_r_launch<VolT, ProjT, ACC, 4, 2, 0>(G, t, mode, a, sens_out, z0, nzs, vs, st);
+            else if (vs == 8) back_r_launch<VolT, ProjT, ACC, 8, 1, 8>(G, t, mode, a, sens_out, z0, nzs, vs, st);
+            else back_r_launch<VolT, ProjT, ACC, 8, 1, 4>(G, t, mode, a, sens_out, z0, nzs, vs, st);
+            return;
+        }
+    }
+    if (R == 1) back_r_launch<VolT, ProjT, ACC, 1, 1, 1>(G, t, mode, a, sens_out, z0, nzs, 1, st);
+    else if (R == 2 && S == 1) back_r_launch<VolT, ProjT, ACC, 2, 1, 1>(G, t, mode, a, sens_out, z0, nzs, 1, st);
+    else if (R == 2) back_r_launch<VolT, ProjT, ACC, 2, 2, 1>(G, t, mode, a, sens_out, z0, nzs, 1, st);
+    else if (R == 4 && S == 1) back_r_launch<VolT, ProjT, ACC, 4, 1, 1>(G, t, mode, a, sens_out, z0, nzs, 1, st);
+    else if (R == 4) back_r_launch<VolT, ProjT, ACC, 4, 2, 1>(G, t, mode, a, sens_out, z0, nzs, 1, st);
+    else back_r_launch<VolT, ProjT, ACC, 8, 1, 1>(G, t, mode, a, sens_out, z0, nzs, 1, st);
 }
 
 template <typename VolT, typename ProjT>
@@ -791,18 +833,9 @@ kv_status back_dispatch(kv_plan *plan, BackMode mode, const BackArgs &a, int z0,
     ExGeom G = exgeom(plan, plan->g.n_views);
     if (std::is_same<VolT, float>::value && plan->bstage.R > 0)
         return back_stage_launch(plan, mode, a, z0, nzs, plan->g.n_views);
-    if (plan->back_rows == 8 && plan->back_vs > 1) {
-        LaunchTimer lt(plan->ctx, "exact_back");
-        cudaStream_t st = plan->ctx->stream;
-        if (plan->back_vs == 8) back_r_launch<VolT, ProjT, ACC_F32, 8, 1, 8>(G, plan->ex, mode, a, nullptr, z0, nzs, st);
-        else if (plan->back_vs == 4) back_r_launch<VolT, ProjT, ACC_F32, 8, 1, 4>(G, plan->ex, mode, a, nullptr, z0, nzs, st);
-        else back_r_launch<VolT, ProjT, ACC_F32, 8, 1, 2>(G, plan->ex, mode, a, nullptr, z0, nzs, st);
-        KV_CHECK_LAUNCH(plan->ctx, "exact_back_r_kernel");
-        return KV_OK;
-    }
     if (plan->back_rows > 0) {
         LaunchTimer lt(plan->ctx, "exact_back");
-        back_r_dispatch<VolT, ProjT, ACC_F32>(plan->back_rows, plan->back_slices, G, plan->ex, mode, a, nullptr, z0, nzs, plan->ctx->stream);
+        back_r_dispatch<VolT, ProjT, ACC_F32>(plan->back_rows, plan->back_slices, G, plan->ex, mode, a, nullptr, z0, nzs, plan->back_vs, plan->ctx->stream);
         KV_CHECK_LAUNCH(plan->ctx, "exact_back_r_kernel");
         return KV_OK;
     }
@@ -812,9 +845,9 @@ kv_status back_dispatch(kv_plan *plan, BackMode mode, const BackArgs &a, int z0,
     const ExactTables &t = plan->ex;
     LaunchTimer lt(plan->ctx, "exact_back");
     switch (mode) {
-    case BACK_PLAIN: exact_back_kernel<VolT, ProjT, ACC_F32, BACK_PLAIN><<<grid, block, 0, st>>>(G, t, a, nullptr, z0); break;
-    case BACK_MLEM: exact_back_kernel<VolT, ProjT, ACC_F32, BACK_MLEM><<<grid, block, 0, st>>>(G, t, a, nullptr, z0); break;
-    case BACK_SART: exact_back_kernel<VolT, ProjT, ACC_F32, BACK_SART><<<grid, block, 0, st>>>(G, t, a, nullptr, z0); break;
+    case BACK_PLAIN: exact_back_kernel<VolT, ProjT, ACC_F32, BACK_PLAIN><<<grid, block, 0, st>>>(G, t, a, nullptr, z0, plan->back_vs); break;
+    case BACK_MLEM: exact_back_kernel<VolT, ProjT, ACC_F32, BACK_MLEM><<<grid, block, 0, st>>>(G, t, a, nullptr, z0, plan->back_vs); break;
+    case BACK_SART: exact_back_kernel<VolT, ProjT, ACC_F32, BACK_SART><<<grid, block, 0, st>>>(G, t, a, nullptr, z0, plan->back_vs); break;
     }
     KV_CHECK_LAUNCH(plan->ctx, "exact_back_kernel");
     return KV_OK;
@@ -922,9 +955,9 @@ kv_status exact_sensitivity_launch(kv_plan *plan, double *sens) {
     {
         LaunchTimer lt(plan->ctx, "exact_back_sens_f64");
         if (plan->back_rows > 0)
-            back_r_dispatch<float, float, ACC_DF>(plan->back_rows, plan->back_slices, G, plan->ex, BACK_PLAIN, a, sens, 0, G.nz, st);
+            back_r_dispatch<float, float, ACC_DF>(plan->back_rows, plan->back_slices, G, plan->ex, BACK_PLAIN, a, sens, 0, G.nz, 1, st);
         else
-            exact_back_kernel<float, float, ACC_DF, BACK_PLAIN><<<grid, block, 0, st>>>(G, plan->ex, a, sens, 0);
+            exact_back_kernel<float, float, ACC_DF, BACK_PLAIN><<<grid, block, 0, st>>>(G, plan->ex, a, sens, 0, 1);
     }
     cudaError_t e = cudaGetLastError();
     cudaFreeAsync(ls, st);
@@ -1099,7 +1132,7 @@ __global__ void __launch_bounds__(256) batch_back_kernel(const BatchItem *__rest
         const int k = (int)(local / per_slice);
         const int rem = (int)(local % per_slice);
         BackArgs a{B.ratio, B.x, B.sens, relax};
-        back_tile<float, float, ACC_F32, BACK_MLEM>(B.G, B.T, a, nullptr, rem % B.btx, rem / B.btx, k);
+        back_tile<float, float, ACC_F32, BACK_MLEM>(B.G, B.T, a, nullptr, rem % B.btx, rem / B.btx, k, 1);
         __syncwarp();
     }
 }
@@ -1277,7 +1310,7 @@ float time_back(kv_ctx *ctx, const ExGeom &G, const ExactTables &T, const void *
     float best = 1e30f;
     for (int rep = 0; rep < 2; ++rep) {
         cudaEventRecord(e0, ctx->stream);
-        exact_back_kernel<VolT, ProjT, ACC, BACK_PLAIN><<<grid, block, 0, ctx->stream>>>(G, T, a, nullptr, 0);
+        exact_back_kernel<VolT, ProjT, ACC, BACK_PLAIN><<<grid, block, 0, ctx->stream>>>(G, T, a, nullptr, 0, 1);
         cudaEventRecord(e1, ctx->stream);
         cudaEventSynchronize(e1);
         float ms = 0.f;
@@ -1365,7 +1398,7 @@ kv_status tune_shapes(kv_plan *plan, int P, TuneResult &best) {
     bt = 1e30f;
     for (const auto &sh : bshapes) {
         const float ms = median3(ctx, e0, e1, [&] {
-            back_r_dispatch<VolT, ProjT, ACC>(sh[0], sh[1], G, plan->ex, BACK_PLAIN, ba, nullptr, 0, g.nz, ctx->stream);
+            back_r_dispatch<VolT, ProjT, ACC>(sh[0], sh[1], G, plan->ex, BACK_PLAIN, ba, nullptr, 0, g.nz, 1, ctx->stream);
         });
         if (ms < bt) {
             bt = ms;
@@ -1376,7 +1409,7 @@ kv_status tune_shapes(kv_plan *plan, int P, TuneResult &best) {
     {
         dim3 block(32, best.back_by), grid((G.nx + 31) / 32, (G.ny + best.back_by - 1) / best.back_by, g.nz);
         const float ms = median3(ctx, e0, e1, [&] {
-            exact_back_kernel<VolT, ProjT, ACC, BACK_PLAIN><<<grid, block, 0, ctx->stream>>>(G, plan->ex, ba, nullptr, 0);
+            exact_back_kernel<VolT, ProjT, ACC, BACK_PLAIN><<<grid, block, 0, ctx->stream>>>(G, plan->ex, ba, nullptr, 0, 1);
         });
         if (ms < bt) {
             bt = ms;
@@ -1424,7 +1457,6 @@ kv_status exact_autotune(kv_plan *plan) {
         plan->rows_gen = -1;
         plan->back_rows = r.back_rows;
         plan->back_slices = r.back_slices;
-        plan->back_vs = 1;
         plan->bstage = r.bstage;
     };
     {

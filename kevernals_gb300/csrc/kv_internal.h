@@ -148,7 +148,7 @@ struct kv_plan {
     int back_by = 8;                 // backprojector block = 32 x back_by voxels (one voxel per thread)
     int back_rows = 8;               // voxel rows per thread of the gather backprojector (0: one voxel per thread)
     int back_slices = 1;             // slices per thread of the gather backprojector
-    int back_vs = 1;                 // view groups of a block (with 8 rows, 1 slice; chosen by the plan only)
+    int back_vs = 1;                 // groups of views the backprojector's sums are formed in (8, 4 or 1; fixed at creation)
 
     // captured iteration loop (kv_mlem / kv_sart without callback), reused
     // while the buffers and parameters are the same
