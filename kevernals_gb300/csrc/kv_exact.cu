@@ -24,6 +24,7 @@
 #include "kv_exact_common.cuh"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <mutex>
 #include <type_traits>
@@ -1366,8 +1367,8 @@ struct TuneResult {
 std::mutex g_tune_mutex;
 std::vector<std::pair<std::vector<long long>, TuneResult>> g_tune_cache;
 
-// The slab forward shapes and gather backprojector shapes, timed through the
-// plan's own launchers on its first (at most) 12 views.
+// The slab forward shapes (the plan's own among them) and gather backprojector
+// shapes, timed through the plan's own launchers on its first P views.
 template <typename VolT, typename ProjT, int ACC>
 kv_status tune_shapes(kv_plan *plan, int P, TuneResult &best) {
     kv_ctx *ctx = plan->ctx;
@@ -1376,9 +1377,11 @@ kv_status tune_shapes(kv_plan *plan, int P, TuneResult &best) {
     cudaEventCreate(&e1);
     const kv_geometry &g = plan->g;
     float bt = 1e30f;
-    static const int shapes[][3] = {{8, 4, 2}, {4, 4, 3}, {8, 2, 2}, {4, 2, 3}, {2, 4, 3}};
     const int group = fwd_slab_default_group(g.n_views);
     const FwdSlabCfg keep = plan->fslab;
+    std::vector<std::array<int, 3>> shapes = {{8, 4, 2}, {4, 4, 3}, {8, 2, 2}, {4, 2, 3}, {2, 4, 3}};
+    const std::array<int, 3> own = {keep.R, keep.S, keep.stages};
+    if (keep.R > 0 && std::find(shapes.begin(), shapes.end(), own) == shapes.end()) shapes.push_back(own);
     const FwdArgs fa{plan->d_vol, nullptr, plan->d_ratio, nullptr, 1.f};
     for (const auto &sh : shapes) {
         FwdSlabCfg c;
@@ -1398,7 +1401,7 @@ kv_status tune_shapes(kv_plan *plan, int P, TuneResult &best) {
     bt = 1e30f;
     for (const auto &sh : bshapes) {
         const float ms = median3(ctx, e0, e1, [&] {
-            back_r_dispatch<VolT, ProjT, ACC>(sh[0], sh[1], G, plan->ex, BACK_PLAIN, ba, nullptr, 0, g.nz, 1, ctx->stream);
+            back_r_dispatch<VolT, ProjT, ACC>(sh[0], sh[1], G, plan->ex, BACK_PLAIN, ba, nullptr, 0, g.nz, plan->back_vs, ctx->stream);
         });
         if (ms < bt) {
             bt = ms;
@@ -1409,7 +1412,7 @@ kv_status tune_shapes(kv_plan *plan, int P, TuneResult &best) {
     {
         dim3 block(32, best.back_by), grid((G.nx + 31) / 32, (G.ny + best.back_by - 1) / best.back_by, g.nz);
         const float ms = median3(ctx, e0, e1, [&] {
-            exact_back_kernel<VolT, ProjT, ACC, BACK_PLAIN><<<grid, block, 0, ctx->stream>>>(G, plan->ex, ba, nullptr, 0, 1);
+            exact_back_kernel<VolT, ProjT, ACC, BACK_PLAIN><<<grid, block, 0, ctx->stream>>>(G, plan->ex, ba, nullptr, 0, plan->back_vs);
         });
         if (ms < bt) {
             bt = ms;
@@ -1444,7 +1447,7 @@ kv_status tune_shapes(kv_plan *plan, int P, TuneResult &best) {
 }  // namespace
 
 // Times the candidate shapes on the plan's own tables with a subset of its
-// views (at most 6: the cost per view is nearly uniform), on zero-filled
+// views (at most 6 or 12: the cost per view is nearly uniform), on zero-filled
 // buffers (the Siddon walk does not depend on the values).
 kv_status exact_autotune(kv_plan *plan) {
     kv_ctx *ctx = plan->ctx;
@@ -1483,7 +1486,8 @@ kv_status exact_autotune(kv_plan *plan) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return kv_fail(ctx, KV_ERR_CUDA, "autotune: %s", cudaGetErrorString(e));
     // slab forward and gather backprojector shapes
-    const int P = g.n_views < 12 ? g.n_views : 12;
+    // (all views where they are summed in groups: the volume is small, and what the groups gain grows with the views)
+    const int P = g.n_views < 12 || plan->back_vs > 1 ? g.n_views : 12;
     switch (plan->storage) {
     case KV_STORAGE_BF16: KV_TRY((tune_shapes<__nv_bfloat16, __nv_bfloat16, ACC_F32>(plan, P, r))); break;
     case KV_STORAGE_F16: KV_TRY((tune_shapes<__half, __half, ACC_F32>(plan, P, r))); break;
