@@ -1456,11 +1456,16 @@ kv_status exact_autotune(kv_plan *plan) {
     auto apply = [plan](const TuneResult &r) {
         plan->fwd_by = r.fwd_by;
         plan->back_by = r.back_by;
-        plan->fslab = r.fslab;
+        // the shapes only: boxes and patches are sized for this plan's own views (another plan of the same sizes may
+        // have tuned them)
+        FwdSlabCfg f;
+        if (r.fslab.R > 0 && fwd_slab_fit(plan, r.fslab.R, r.fslab.S, r.fslab.stages, r.fslab.group, &f, nullptr))
+            plan->fslab = f;
         plan->rows_gen = -1;
         plan->back_rows = r.back_rows;
         plan->back_slices = r.back_slices;
-        plan->bstage = r.bstage;
+        BackStageCfg b;
+        plan->bstage = r.bstage.R > 0 && back_stage_fit(plan, r.bstage.R, r.bstage.stages, &b, nullptr) ? b : BackStageCfg{};
     };
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);

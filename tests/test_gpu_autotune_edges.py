@@ -1,4 +1,4 @@
-"""The tuner on small plans."""
+"""The tuner on small plans and on plans of equal sizes."""
 import numpy as np
 import pytest
 
@@ -45,3 +45,18 @@ def test_tuned_small_plan_is_not_slower(ctx, geom):
     assert after[0] < 1.5 * before[0] and after[1] < 1.5 * before[1]
     assert torch.equal(out, want[0])
     assert float((proj - want[1]).norm() / want[1].norm()) < 1e-6
+
+
+def test_plans_of_equal_sizes_keep_their_own_boxes(ctx):
+    """The cached result of a narrow sweep is a shape; a wide sweep of the same sizes needs larger boxes for it."""
+    def sweep(angle):
+        return linear_sweep(24, 40, 16, 0.5, 0.5, 2.0, 5, 40, 64, 0.4, 0.4, angle)
+    engine.Plan(ctx, sweep(2.0), "exact").autotune()
+    g = sweep(30.0)
+    rng = np.random.default_rng(1)
+    x, y = rng.random(g.volume_shape, dtype=np.float32), rng.random(g.proj_shape, dtype=np.float32)
+    plan, tuned = engine.Plan(ctx, g, "exact"), engine.Plan(ctx, g, "exact")
+    tuned.autotune()
+    ref = plan.forward(x)
+    assert np.linalg.norm(tuned.forward(x) - ref) < 1e-6 * np.linalg.norm(ref)
+    assert np.array_equal(tuned.back(y), plan.back(y))

@@ -25,8 +25,9 @@ def fresh(ctx, g, p, n):
 
 
 def test_a_solve_after_a_failed_one(ctx):
-    """A pass that gives up (boxes tuned for a narrower sweep of the same sizes) leaves row sums unwritten; the next
-    solve, with another kernel, must not read them (its sums differ from a fresh plan's by a few roundings)."""
+    """A pass that gives up leaves row sums unwritten; the next solve, with another kernel, must not read them (its
+    sums differ from a fresh plan's by a few roundings).  The first solve runs a shape tuned for a narrower sweep of the
+    same sizes, whose boxes rays of this one leave unless the plan sizes its own; it may fail or not."""
     narrow, wide = sweep(1.0), sweep(30.0)
     engine.Plan(ctx, narrow, "exact").autotune()
     p = np.random.default_rng(1).random(wide.proj_shape, dtype=np.float32)
