@@ -602,11 +602,11 @@ kv_status saa_launch(kv_plan *plan, const int32_t *d_shift, const int32_t *h_shi
     const kv_geometry &g = plan->g;
     kv_ctx *ctx = plan->ctx;
     // the staged kernel where its band fits and TMA can address the stack; eight slices a block where two blocks
-    // stay resident
+    // stay resident.  Four slices as far as shared memory goes: the direct kernel, next, is slower and takes 1536 views
     if ((g.nu * 4) % 16 == 0 && reinterpret_cast<uintptr_t>(proj) % 16 == 0 && kvtma::encoder() != nullptr) {
         kv_status s = KV_OK;
         if (saa_band_launch<8>(plan, d_shift, h_shift, proj, out, 100 * 1024, &s) ||
-            saa_band_launch<4>(plan, d_shift, h_shift, proj, out, 160 * 1024, &s))
+            saa_band_launch<4>(plan, d_shift, h_shift, proj, out, 208 * 1024, &s))
             return s;
     }
     const int kb = 8;
