@@ -273,10 +273,13 @@ kv_status kv_plan_set_back_staging(kv_plan *plan, int rows_per_thread, int stage
  * Channels-last BF16 (bit patterns) [D][H][W][C]: in1 has c1 channels, in2
  * (may be NULL when c2 = 0) c2 channels concatenated after them, out cout
  * channels; w is [cout][27][c1 + c2] BF16 (taps z, y, x), bias cout floats
- * or NULL; FP32 accumulation.  kernel: 0 = tcgen05 / TMA implicit GEMM where
- * it covers the call, else mma.sync (equal bits); 1 = tcgen05 only, for
- * volumes of whole 128-voxel tiles; 2 = mma.sync only.  Channel counts: multiples of 16 (the
- * tcgen05 kernel: 16, 32, 64 or 128 per input, cout <= 256).  Stream-ordered
+ * or NULL; FP32 accumulation.  kernel: 0 = tcgen05 / TMA implicit GEMM on
+ * volumes of whole 128-voxel tiles (KV_ERR_UNSUPPORTED where it does not cover
+ * the channels), on other volumes where it covers the call, else mma.sync
+ * (equal bits for finite weights); 1 = tcgen05 only, for volumes of whole
+ * tiles; 2 = mma.sync only.  W is a multiple of 16 but for volumes of whole
+ * tiles with kernel 0 or 1.  Channel counts: multiples of 16 (the tcgen05
+ * kernel: 16, 32, 64 or 128 per input, cout <= 256).  Stream-ordered
  * on the context's stream; a tensor-core pipeline wait that gives up is
  * reported by the next kv_sync. */
 kv_status kv_conv3_bf16(kv_ctx *ctx, const uint16_t *in1, int32_t c1, const uint16_t *in2, int32_t c2,

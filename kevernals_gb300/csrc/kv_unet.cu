@@ -985,9 +985,9 @@ extern "C" kv_status kv_conv3_bf16(kv_ctx *ctx, const uint16_t *in1, int32_t c1,
     const bool tiles = convtc::tile_shape(D, H, W);
     if (kernel == 1 && !tiles)
         return kv_fail(ctx, KV_ERR_UNSUPPORTED, "kv_conv3_bf16: the volume is not a whole number of 128-voxel tiles");
-    // volumes that are not whole tiles take the tensor-core kernel too where it covers the call, else mma.sync; the
-    // two sum in the same order, with equal bits
-    if (kernel != 2) {
+    // volumes that are not whole tiles, of the widths that mma.sync takes, take the tensor-core kernel too where it
+    // covers the call, else mma.sync; the two sum in the same order, with equal bits
+    if (kernel != 2 && (tiles || W % 16 == 0)) {
         const char *why = convtc::launch(a, c1, c2 ? b : nullptr, c2, wb, bias, relu != 0, nullptr, nullptr, o, cout, D, H, W,
                                          ctx->d_status, ctx->sm_count, ctx->stream);
         if (why == nullptr) {

@@ -136,3 +136,36 @@ def test_conv_limits_are_refused(ctx, c1, c2, cout):
         st = _lib.lib().kv_conv3_bf16(ctx.handle, p, c1, p if c2 else None, c2, p, C.c_void_p(f.data_ptr()), 1, p,
                                       cout, 1, 2, 128, kernel)
         assert _lib.STATUS_NAMES[st] == "KV_ERR_UNSUPPORTED"
+
+
+@pytest.mark.parametrize("dims", [(1, 3, 24), (2, 5, 8), (1, 1, 100), (3, 2, 136), (1, 1, 1)])
+@pytest.mark.parametrize("kernel", [0, 1, 2])
+def test_conv_widths_are_refused(ctx, dims, kernel):
+    """Widths that are not multiples of 16, on volumes that are not whole tiles: an error, nothing run."""
+    torch = pytest.importorskip("torch")
+    from kevernals_gb300 import _lib
+    t = torch.zeros(2 * 128 * 256 * 27, dtype=torch.int16, device="cuda")
+    f = torch.zeros(256, device="cuda")
+    p = C.c_void_p(t.data_ptr())
+    st = _lib.lib().kv_conv3_bf16(ctx.handle, p, 16, None, 0, p, C.c_void_p(f.data_ptr()), 1, p, 16, *dims, kernel)
+    assert _lib.STATUS_NAMES[st] == "KV_ERR_UNSUPPORTED"
+
+
+@pytest.mark.parametrize("dims", [(2, 16, 8), (4, 32, 4), (64, 2, 1), (1, 64, 2)])
+def test_conv_narrow_whole_tiles(ctx, dims):
+    """Whole tiles of volumes narrower than 16 voxels, against FP64 at the bound of the layers above."""
+    torch = pytest.importorskip("torch")
+    import torch.nn.functional as F
+    rng = np.random.default_rng(sum(dims))
+    a, af = _bf16_bits(rng.standard_normal((*dims, 32)).astype(np.float32))
+    w, wf = _bf16_bits((rng.standard_normal((16, 27, 32)) / np.sqrt(27 * 32)).astype(np.float32))
+    bias = (rng.standard_normal(16) * 0.1).astype(np.float32)
+    xt = torch.from_numpy(af.astype(np.float64)).permute(3, 0, 1, 2)[None]
+    wt = torch.from_numpy(wf.astype(np.float64)).permute(0, 2, 1).reshape(16, 32, 3, 3, 3)
+    bt = torch.from_numpy(bias.astype(np.float64))
+    ref = F.conv3d(xt, wt, bt, padding=1)[0].permute(1, 2, 3, 0).numpy()
+    mag = F.conv3d(xt.abs(), wt.abs(), bt.abs(), padding=1)[0].permute(1, 2, 3, 0).numpy()
+    for kernel in (0, 1):
+        bits = _conv(ctx, a, 32, a, 0, w, bias, False, 16, dims, kernel)
+        got = (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+        assert np.all(np.abs(got - ref) <= 2 ** -8 * np.abs(ref) + 2 ** -20 * mag)
