@@ -862,20 +862,17 @@ kv_status update_forward(kv_plan *plan, bool mlem, const void *p, const void *x,
 // Without a callback (and without tracing) the iteration loop is captured once
 // as a CUDA graph on the context's own stream and launched on the call's
 // stream; the executable graph is kept and relaunched while the buffers and
-// parameters stay the same.  SART's first forward pass is launched before the
-// graph, as it may have to store the row sums: the graph begins with its
-// backprojection and is the same for a plan's first solve and the next.
+// parameters stay the same.  (A SART solve that stores the row sums is launched
+// plainly: its graph would serve no other solve.)
 long long slab_key(const FwdSlabCfg &c) {
     return (((long long)c.R * 16 + c.S) * 8 + c.stages) * 65536 + c.group;
 }
 
 kv_status iterate_loop(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem, kv_iter_cb cb,
-                       void *user, bool rows, bool projected);
+                       void *user, bool rows);
 
 kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem, bool rows) {
     kv_ctx *ctx = plan->ctx;
-    const bool projected = !mlem && plan->family == KV_FAMILY_EXACT;
-    if (projected) KV_TRY(update_forward(plan, mlem, p, x, nullptr, relax, 0, plan->g.n_views, &rows));
     const bool same = plan->graph_exec != nullptr && plan->graph_p == p && plan->graph_x == x &&
                       plan->graph_iters == iters && plan->graph_mlem == (int)mlem && plan->graph_relax == relax &&
                       plan->graph_fb == plan->fwd_by && plan->graph_bb == plan->back_by &&
@@ -892,7 +889,7 @@ kv_status iterate_graph(kv_plan *plan, const void *p, void *x, int iters, float 
         cudaStream_t user_stream = ctx->stream;
         ctx->stream = ctx->own_stream;
         KV_CHECK_CUDA(ctx, cudaStreamBeginCapture(ctx->own_stream, cudaStreamCaptureModeThreadLocal));
-        kv_status s = iterate_loop(plan, p, x, iters, relax, mlem, nullptr, nullptr, rows, projected);
+        kv_status s = iterate_loop(plan, p, x, iters, relax, mlem, nullptr, nullptr, rows);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->own_stream, &graph);
         ctx->stream = user_stream;
@@ -930,25 +927,25 @@ kv_status iterate(kv_plan *plan, const void *p, void *x, int iters, float relax,
     kv_ctx *ctx = plan->ctx;
     const size_t es = kv_storage_bytes(plan->storage);
     KV_TRY(ensure(ctx, &plan->d_ratio, plan->nproj * es));
-    bool rows = false;
+    bool rows = false, stores = false;
     if (plan->family == KV_FAMILY_EXACT) {
         KV_TRY(ensure_sens(plan));
         ensure_pad(plan);
-        if (!mlem) rows = ready_rows(plan);
+        if (!mlem) {
+            rows = ready_rows(plan);
+            stores = !rows && plan->d_rows != nullptr;
+        }
     }
-    if (cb == nullptr && !ctx->timing && iters >= 2 && !stream_capturing(ctx))
+    if (cb == nullptr && !ctx->timing && iters >= 2 && !stores && !stream_capturing(ctx))
         return iterate_graph(plan, p, x, iters, relax, mlem, rows);
-    return iterate_loop(plan, p, x, iters, relax, mlem, cb, user, rows, false);
+    return iterate_loop(plan, p, x, iters, relax, mlem, cb, user, rows);
 }
 
-// The loop itself; projected: the first iteration's forward pass (EXACT) has been launched.
 kv_status iterate_loop(kv_plan *plan, const void *p, void *x, int iters, float relax, bool mlem, kv_iter_cb cb,
-                       void *user, bool rows, bool projected) {
+                       void *user, bool rows) {
     kv_ctx *ctx = plan->ctx;
     for (int it = 0; it < iters; ++it) {
-        if (projected && it == 0) {
-            // launched before the loop
-        } else if (plan->family == KV_FAMILY_EXACT) {
+        if (plan->family == KV_FAMILY_EXACT) {
             KV_TRY(update_forward(plan, mlem, p, x, cb ? ctx->d_red : nullptr, relax, 0, plan->g.n_views, &rows));
         } else if (cb) {
             KV_TRY(rc_forward_launch(plan, plan->d_src, plan->d_org, plan->g.n_views, RC_PLAIN, (const float *)x,
