@@ -473,7 +473,15 @@ void default_shapes(kv_plan *plan) {
         best = cost;
         pick = c;
     }
-    (padded ? plan->fpad : plan->fslab) = pick;
+    // Rows that are not whole 16-byte units: the copy with padded rows costs a
+    // launch and a pass over the volume, which thin volumes of few rays do not
+    // earn back against the one-thread-per-ray kernel (an MLEM iteration of 14 x
+    // 14 x 4, 9 views: 1.13 of its time, 14 x 14 x 12 0.97, 5 x 5 x 20 1.11; 127
+    // x 127 x 2, 9 views, 6.5e5 rays x slices, 1.02, 127 x 127 x 3 0.98; 127 x 127
+    // x 20 0.84).
+    const double work = (double)plan->nproj * g.nz;
+    if (!padded) plan->fslab = pick;
+    else if (work >= 7e5 || (g.nz >= 12 && work >= 2.5e4)) plan->fpad = pick;
     const long long blocks = (long long)g.nz * ((g.ny + 63) / 64) * ((g.nx + 31) / 32);
     plan->back_vs = blocks * 2 <= sms ? 8 : (2 * blocks <= 3 * sms ? 4 : 1);
 }

@@ -48,3 +48,44 @@ def test_slab_shape_at_the_shared_memory_limit(ctx):
     assert plan.slab == (4, 8, 4, 5)
     # the same lengths, a slice's sums in the same order: equal bits for every shape
     assert np.array_equal(plan.forward(vol), ref)
+
+
+@pytest.mark.parametrize("storage,tol", [("f32", 1e-6), ("bf16", 2 ** -7), ("f16", 2 ** -10)])
+@pytest.mark.parametrize("nx", [33, 34, 36, 39])
+def test_padded_rows_of_a_thick_volume(ctx, storage, tol, nx):
+    """Iterations on rows that are not whole 16-byte units, in a volume thick enough for the padded copy, against the
+    one-thread-per-ray kernel, at the bounds of test_padded_rows_match_the_ray_kernel."""
+    g = linear_sweep(nx, 29, 13, 0.7, 0.45, 1.3, 4, 37, 41, 0.55, 0.35, 22.0)
+    p = np.random.default_rng(3).random(g.proj_shape, dtype=np.float32)
+    for sart in (False, True):
+        xs = []
+        for ray in (False, True):
+            plan = engine.Plan(ctx, g, "exact", storage)
+            if ray:
+                plan.set_slab(0)
+            x = np.full(g.volume_shape, 0.0 if sart else 1.0, np.float32)
+            ctx.read_timing()
+            ctx.set_timing(True)
+            (plan.sart if sart else plan.mlem)(p, x, 3)
+            ctx.set_timing(False)
+            whole = nx * (4 if storage == "f32" else 2) % 16 == 0
+            assert ("pad_rows" in ctx.read_timing()) == (not ray and not whole)
+            xs.append(x)
+        assert np.linalg.norm(xs[0] - xs[1]) < tol * np.linalg.norm(xs[1])
+
+
+@pytest.mark.parametrize("geom,padded", [
+    ((13, 13, 4, 0.5, 0.5, 1.0, 9, 20, 20, 0.4, 0.4, 15.0), False),
+    ((5, 5, 20, 0.5, 0.5, 1.0, 25, 6, 6, 0.4, 0.4, 15.0), False),
+    ((13, 13, 12, 0.5, 0.5, 1.0, 9, 20, 20, 0.4, 0.4, 15.0), True),
+    ((61, 61, 3, 0.5, 0.5, 1.0, 27, 96, 96, 0.4, 0.4, 15.0), True),
+])
+def test_thin_volumes_of_few_rays_are_not_padded(ctx, geom, padded):
+    g = linear_sweep(*geom)
+    plan = engine.Plan(ctx, g, "exact")
+    x = np.ones(g.volume_shape, np.float32)
+    ctx.read_timing()
+    ctx.set_timing(True)
+    plan.mlem(np.ones(g.proj_shape, np.float32), x, 1)
+    ctx.set_timing(False)
+    assert ("pad_rows" in ctx.read_timing()) == padded
