@@ -43,14 +43,17 @@ __device__ __forceinline__ bool rc_sup_eq(float a, float b) {
 // product is exact in double): rounding never carries it across an integer, so v and the double sum have the same
 // integer part unless v is an integer itself.  Only then is the sum formed in double, out of line: inlined, the
 // compiler ran the double arithmetic for every index and selected afterwards, and the FP64 pipe bounded the kernel
-// (15 views of 512 x 512 through 256 x 256 x 64 voxels: 3.9 -> 0.53 ms).
+// (15 views of 512 x 512 through 256 x 256 x 64 voxels: 3.9 -> 0.53 ms).  A NaN (a source or detector so far off that
+// its position in voxels overflows) takes the double path too, where it becomes no voxel's index; as a float it would
+// convert to 0.
 __device__ __noinline__ int rc_index_double(float base, float c, float d) {
     return (int)((double)base + (double)c * (double)d);
 }
 
 __device__ __forceinline__ int rc_index(float base, float c, float d) {
     const float v = fmaf(c, d, base);
-    return v != rintf(v) ? (int)v : rc_index_double(base, c, d);
+    const float r = rintf(v);
+    return v < r || v > r ? (int)v : rc_index_double(base, c, d);
 }
 
 // Window pixels [q0, q1] cut to those whose ray can meet the voxel: a ray's parameter lies in [mn, mx] there (the
