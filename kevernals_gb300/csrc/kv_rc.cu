@@ -204,15 +204,13 @@ __global__ void __launch_bounds__(128) rc_forward_kernel(RcGeom G, const float *
 // needs them for every voxel): tab[p][u] = x, then [p][v] = y.
 __global__ void rc_table_kernel(RcGeom G, const float *__restrict__ src, const float *__restrict__ org,
                                 float *__restrict__ tab) {
-    const int p = blockIdx.y, q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < G.nu) {
-        const float ox = org[3 * p], sx = src[3 * p] / G.dx;
+    const int p = blockIdx.x;
+    const float ox = org[3 * p], sx = src[3 * p] / G.dx;
+    for (int q = threadIdx.x; q < G.nu; q += blockDim.x)
         tab[(size_t)p * G.nu + q] = (ox + ((float)q + 0.5F) * G.du) / G.dx - sx;
-    }
-    if (q < G.nv) {
-        const float oy = org[3 * p + 1], sy = src[3 * p + 1] / G.dy;
+    const float oy = org[3 * p + 1], sy = src[3 * p + 1] / G.dy;
+    for (int q = threadIdx.x; q < G.nv; q += blockDim.x)
         tab[(size_t)G.n_views * G.nu + (size_t)p * G.nv + q] = (oy + ((float)q + 0.5F) * G.dv) / G.dy - sy;
-    }
 }
 
 // What of a view depends on the slice only, computed once per block.
@@ -382,8 +380,8 @@ kv_status rc_build_tables(kv_plan *plan) {
     const RcGeom G = rcgeom(plan, plan->g.n_views);
     const size_t n = (size_t)G.n_views * ((size_t)G.nu + G.nv);
     KV_CHECK_CUDA(plan->ctx, cudaMalloc((void **)&plan->d_rctab, n * sizeof(float)));
-    const int m = G.nu > G.nv ? G.nu : G.nv;
-    rc_table_kernel<<<dim3((m + 127) / 128, G.n_views), 128, 0, plan->ctx->stream>>>(G, plan->d_src, plan->d_org, plan->d_rctab);
+    // a block a view: their number has no other limit
+    rc_table_kernel<<<G.n_views, 256, 0, plan->ctx->stream>>>(G, plan->d_src, plan->d_org, plan->d_rctab);
     KV_CHECK_LAUNCH(plan->ctx, "rc_table_kernel");
     return KV_OK;
 }

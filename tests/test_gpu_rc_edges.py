@@ -24,3 +24,11 @@ def test_index_that_is_not_a_number_is_no_voxel(ctx):
     src[:, 0] = 1e38
     plan = engine.Plan(ctx, dataclasses.replace(g, src=src), "rc")
     assert not plan.forward(np.ones(g.volume_shape, np.float32)).any()
+
+
+def test_more_views_than_a_grid_is_high(ctx):
+    """65,537 views: the backprojector, whose grid is the volume's, takes them; equal to the oracle, bit for bit."""
+    from oracle import oracle as O
+    g = linear_sweep(6, 5, 3, 0.5, 0.5, 1.0, 65537, 4, 4, 1.0, 1.0, 10.0)
+    p = np.ones(g.proj_shape, np.float32)
+    assert np.array_equal(engine.Plan(ctx, g, "rc").back(p), O.rc_back(g, p))
