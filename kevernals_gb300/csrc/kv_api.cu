@@ -528,12 +528,16 @@ extern "C" kv_status kv_plan_create(kv_ctx *ctx, const kv_geometry *g, kv_family
             cudaMalloc((void **)&plan->d_org, bytes) != cudaSuccess) {
             s = kv_fail(ctx, KV_ERR_OOM, "plan tables");
         } else {
-            // every stream that uses the plan later finds the tables done
+            // every stream that uses the plan later finds the tables done; on the context's own stream, as the
+            // caller's may be capturing
+            cudaStream_t user = ctx->stream;
+            ctx->stream = ctx->own_stream;
             cudaMemcpyAsync(plan->d_src, plan->src.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
             cudaMemcpyAsync(plan->d_org, plan->det.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
             s = rc_build_tables(plan);
             if (cudaStreamSynchronize(ctx->stream) != cudaSuccess && s == KV_OK)
                 s = kv_fail(ctx, KV_ERR_CUDA, "plan tables");
+            ctx->stream = user;
         }
     }
     if (s != KV_OK) {

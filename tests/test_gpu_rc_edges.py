@@ -32,3 +32,20 @@ def test_more_views_than_a_grid_is_high(ctx):
     g = linear_sweep(6, 5, 3, 0.5, 0.5, 1.0, 65537, 4, 4, 1.0, 1.0, 10.0)
     p = np.ones(g.proj_shape, np.float32)
     assert np.array_equal(engine.Plan(ctx, g, "rc").back(p), O.rc_back(g, p))
+
+
+def test_plan_made_while_its_stream_captures(ctx):
+    """In a relaxed capture: the plan's tables are not part of the graph, which holds what was launched beside them."""
+    torch = pytest.importorskip("torch")
+    g = linear_sweep(16, 12, 6, 0.5, 0.5, 1.0, 3, 20, 18, 0.4, 0.4, 10.0)
+    x, y = torch.zeros(64, device="cuda"), np.random.default_rng(1).random(g.proj_shape, dtype=np.float32)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        ctx.use_torch_stream()
+        plan = engine.Plan(ctx, g, "rc")
+        x += 1
+    ctx.use_torch_stream()
+    graph.replay()
+    assert float(x.sum()) == 64.0
+    assert np.array_equal(plan.back(y), engine.Plan(ctx, g, "rc").back(y))
