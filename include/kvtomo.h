@@ -232,7 +232,14 @@ kv_status kv_plan_set_tuning(kv_plan *plan, int fwd_rows, int back_rows);
  * kernel.  Plans take a default shape when their geometry suits it (at most
  * two column and four row planes crossed per ray and slice); set returns
  * KV_ERR_UNSUPPORTED with a reason when a shape does not fit the geometry.
- * get reports rays_per_thread = 0 when the plan runs the per-ray kernel. */
+ * get reports rays_per_thread = 0 when the plan runs the per-ray kernel.
+ * Volumes whose rows are not a whole number of 16 bytes: get reports 0, and
+ * kv_forward and kv_residual run the per-ray kernel; kv_mlem, kv_sart and kv_batch_mlem run a slab shape of their own on
+ * a copy with padded rows where the volume is not thin (the same lengths summed
+ * in another order), until set is called with 0.
+ * Either kernel multiplies only lengths inside the volume; the slab kernel also
+ * reads, at length zero, up to two columns beside a ray's own, so that a voxel
+ * that is not finite makes the rays that pass there NaN. */
 kv_status kv_plan_get_slab(const kv_plan *plan, int *rays_per_thread, int *slices, int *stages, int *view_group);
 kv_status kv_plan_set_slab(kv_plan *plan, int rays_per_thread, int slices, int stages, int view_group);
 
@@ -315,7 +322,9 @@ kv_status kv_unet_forward(kv_unet *net, const float *in, float *out, int32_t D, 
  * stays a sum over the other voxels divided by D*H*W). */
 kv_status kv_unet_train_step(kv_unet *net, const float *in, const float *target, int32_t D, int32_t H,
                              int32_t W, float lr, float *loss, kv_mem mem);
-/* Loss and FP32 parameter gradients (host buffer of kv_unet_num_params). */
+/* Loss and FP32 parameter gradients (host buffer of kv_unet_num_params).  The
+ * weight gradients pair voxels outside the volume as zeros: an activation or
+ * gradient at the border that is not finite makes those taps NaN too. */
 kv_status kv_unet_gradients(kv_unet *net, const float *in, const float *target, int32_t D, int32_t H,
                             int32_t W, float *loss, float *grads, kv_mem mem);
 /* Checkpoint state: parameters, Adam moments (3 * num_params host floats) and

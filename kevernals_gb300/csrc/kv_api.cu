@@ -439,7 +439,10 @@ namespace {
 //
 // Slab forward: the shapes that fit, by the number of rounds of resident CTAs
 // times what a round takes (two CTAs of R = 8, three of R = 4 or 2 a SM where
-// shared memory allows; rounds measured 1 : 0.78 : 0.54 on a full GPU).  Large detectors take R = 8
+// shared memory allows).  Rounds measured on a full GPU, three geometries, R =
+// 8, 4, 2 with four slices a slab: 1 : 0.73-0.78 : 0.48-0.53; with two slices R
+// = 4 0.90-0.96, R = 2 0.62-0.70, taken a little higher, as those shapes are for
+// boxes that do not fit otherwise.  Large detectors take R = 8
 // (512 x 512 x 15 views: 321 us, R = 4: 336); 96 x 128 x 30 views R = 4 (20.6
 // us, R = 8: 24.4), 56 x 64 x 7 views R = 2 (12.8, R = 8: 18.1).
 //
@@ -448,7 +451,8 @@ namespace {
 // rows a thread and no split, 8 x 128 x 64 voxels, 49 views (32 blocks): 121
 // -> 24 us at 8 groups; 16 x 64 x 96, 30 views (48): 74 -> 25; 24 x 128 x 128,
 // 15 views (192): 41 -> 35 at 4; 41 x 187 x 213 (861) would lose, 112 -> 154
-// at 2, as warps on different views share no detector rows in L1.
+// at 2, as warps on different views share no detector rows in L1.  The groups
+// are the plan's: every backprojection kernel sums in them, with equal bits.
 void default_shapes(kv_plan *plan) {
     const kv_geometry &g = plan->g;
     const int sms = plan->ctx->sm_count > 0 ? plan->ctx->sm_count : 1;

@@ -24,7 +24,9 @@
 // An output plane is finished with dz = 2, read out, and its slot zeroed for
 // the plane three further on: every MMA accumulates.  Sums run over dz, then
 // (dy, dx), then 16-channel segments -- the tap order of the mma.sync kernel,
-// with equal bits -- so a plane's segments are all in shared memory at once.
+// with equal bits (for finite weights: planes outside the volume are not
+// loaded, so an infinite weight does not meet their zeros) -- so a plane's
+// segments are all in shared memory at once.
 // The weights stay there for the CTA's life where they fit beside the plane
 // buffers; else they stream through a ring, one (dy, dx) of up to four
 // segments at a time, each piece used for every sub-tile.
@@ -734,7 +736,8 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
     auto ok_c = [](int c) { return c == 16 || c == 32 || c == 64 || c == 128; };
     if (!ok_c(c1) || (c2 != 0 && !ok_c(c2))) return "input channels must be 16, 32, 64 or 128";
     if (N % 16 != 0 || N < 16 || N > 256) return "output channels must be a multiple of 16 up to 256";
-    // the operator's limits: four segments of one width, and 128 + N rows of every segment twice in 200 KB
+    // The operator's limits: four segments of one width, and 128 + N rows of every segment twice in 200 KB.  This kernel
+    // could take more (plan_shape); they are the interface's, tested, so that no caller comes to rely on others.
     const int kseg = std::min(std::min(c1, 64), c2 != 0 ? c2 : 64), segs = K / kseg;
     if (segs > 4) return "too many input channel segments";
     if (2 * (size_t)segs * (align1k(kTileM * kseg * 2) + align1k(N * kseg * 2)) > 200 * 1024)

@@ -1066,8 +1066,9 @@ extern "C" kv_status kv_residual_noalloc(kv_plan *plan, const float *projections
 // Work, rays x slices + 0.3 voxels x views, a problem: 2.6e4, 64 problems, 20
 // iterations 2.0 ms (own launches 6.6, one iteration as a graph 3.5), 256
 // problems, 5 iterations 4.2 (9.0, 6.8), 8 problems, 20 iterations 0.72 (1.14,
-// 0.84); 3.8e5, 256 problems, 5 iterations 8.6 (9.0); 5.2e5, 32 problems, 10
-// iterations 2.9 (2.2).
+// 0.84); 3.8e5, 256 problems, 5 iterations 8.9 (9.0); 5.2e5, 32 problems, 10
+// iterations 2.9 (2.2).  At full size (16 problems of up to 512 x 512 x 96
+// voxels, 5 iterations) side by side 93.4 ms, one by one 96.2.
 namespace {
 
 constexpr int kSideStreams = 8;

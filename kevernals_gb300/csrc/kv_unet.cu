@@ -369,7 +369,8 @@ __global__ void pool_bwd_skip_mask(const bf16 *__restrict__ dp, const bf16 *__re
     }
 }
 
-// nearest x2 upsampling (channels-last): out D x H x W from in D/2 x H/2 x W/2; a thread writes the eight children
+// nearest x2 upsampling (channels-last): out D x H x W from in D/2 x H/2 x W/2; a thread writes the four children of one
+// x, so that a warp writes consecutive voxels
 __global__ void upsample_fwd(const bf16 *__restrict__ in, bf16 *__restrict__ out, int D, int H, int W, int C) {
     const int c8 = C / 8, w2 = W / 2, h2 = H / 2;
     const long long n = (long long)(D / 2) * h2 * W * c8;   // a thread: one x, the four (z, y) children
