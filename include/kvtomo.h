@@ -237,9 +237,9 @@ kv_status kv_plan_set_tuning(kv_plan *plan, int fwd_rows, int back_rows);
  * kv_forward and kv_residual run the per-ray kernel; kv_mlem, kv_sart and kv_batch_mlem run a slab shape of their own on
  * a copy with padded rows where the volume is not thin (the same lengths summed
  * in another order), until set is called with 0.
- * Either kernel multiplies only lengths inside the volume; the slab kernel also
- * reads, at length zero, up to two columns beside a ray's own, so that a voxel
- * that is not finite makes the rays that pass there NaN. */
+ * A voxel that is not finite reaches the rays that meet it and, where a plan's
+ * own rows are whole 16-byte units, those that pass within two columns of it
+ * (read at length zero); on padded rows and in kv_batch_mlem no others. */
 kv_status kv_plan_get_slab(const kv_plan *plan, int *rays_per_thread, int *slices, int *stages, int *view_group);
 kv_status kv_plan_set_slab(kv_plan *plan, int rays_per_thread, int slices, int stages, int view_group);
 

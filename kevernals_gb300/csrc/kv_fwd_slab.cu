@@ -31,6 +31,7 @@
 // from view to view, so one group sweeps the volume through L2 about once.
 #include "kv_internal.h"
 #include "kv_exact_common.cuh"
+#include "kv_exact_ray.cuh"
 #include "kv_tma.cuh"
 
 #include <algorithm>
@@ -61,6 +62,7 @@ struct SlabArgs {
     uint32_t stage_bytes;            // bytes one box load delivers: BX * BY * S * element size
     uint32_t desc_off, hr_off, yt_off, yi_off, org_off;   // byte offsets in dynamic shared memory
     int *status;                     // error bits (0: fine)
+    int pitch;                       // elements from one volume row to the next
 };
 
 // c - (c mod a) with a non-negative remainder.
@@ -183,9 +185,22 @@ __device__ __forceinline__ void slice_rays(const unsigned char *box, const YDesc
     }
 }
 
-template <typename VolT, typename ProjT, int MODE, int R>
+// A ray's sum from the voxels it meets.  The slab's lockstep also reads, at length zero, up to two columns beside
+// them, and 0 x inf is NaN; out of line, for sums that are not finite only.
+template <typename VolT>
+__device__ __noinline__ float ray_again(const ExGeom &G, const ExactTables &T, const VolT *vol, int pitch, int u, int v,
+                                        int p) {
+    float acc = 0.f, wsum = 0.f;
+    ray_walk<VolT, false>(G, T, vol, pitch, u, v, p, acc, wsum);
+    return acc;
+}
+
+// MET: sums that are not finite are formed again from the voxels the ray meets (a variant of its own: the call costs
+// the others 1.5 %).
+template <typename VolT, typename ProjT, int MODE, int R, bool MET>
 __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(const __grid_constant__ CUtensorMap vmap,
-                                                            const ExGeom G, const ExactTables T, const FwdArgs a,
+                                                            const __grid_constant__ ExGeom G,
+                                                            const __grid_constant__ ExactTables T, const FwdArgs a,
                                                             double *partials, const SlabArgs A) {
     constexpr int TV = 8 * R;
     constexpr bool SART = MODE == FWD_SART;
@@ -393,7 +408,10 @@ __global__ void __launch_bounds__(kThreads, R >= 8 ? 2 : 3) fwd_slab_kernel(cons
         const int vl = warp + 8 * q, v = v0 + vl;
         if (!live_u || v >= G.nv) continue;
         const float ls = ray_factor(X.w, s_yt[vl].w, VI);
-        const float qv = __fadd_rn(acc[q][0], acc[q][1]) * ls;
+        float sum = __fadd_rn(acc[q][0], acc[q][1]);
+        if (MET && !(fabsf(sum) < __int_as_float(0x7f800000)))
+            sum = ray_again(G, T, static_cast<const VolT *>(a.vol), A.pitch, u, v, p);
+        const float qv = sum * ls;
         const size_t ray = ((size_t)p * G.nv + v) * G.nu + u;
         ProjT *out = static_cast<ProjT *>(a.out);
         float pm = 0.f;
@@ -485,24 +503,17 @@ SmemLayout smem_layout(int R, int S, int stages, int BX, int BY, int nz, int es)
 template <typename VolT, typename ProjT, int R>
 kv_status slab_launch_r(kv_plan *plan, const CUtensorMap &map, const ExGeom &G, const ExactTables &t, FwdMode mode,
                         const FwdArgs &a, double *partials, const SlabArgs &A, unsigned grid, size_t smem) {
-    cudaStream_t st = plan->ctx->stream;
-    const void *fn = nullptr;
+    void (*fn)(const CUtensorMap, const ExGeom, const ExactTables, const FwdArgs, double *, const SlabArgs) = nullptr;
     switch (mode) {
-    case FWD_PLAIN: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_PLAIN, R>; break;
-    case FWD_MLEM: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_MLEM, R>; break;
-    case FWD_SART: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_SART, R>; break;
-    case FWD_RESID: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_RESID, R>; break;
-    case FWD_SART_ROWS: fn = (const void *)fwd_slab_kernel<VolT, ProjT, FWD_SART_ROWS, R>; break;
+    case FWD_PLAIN: fn = fwd_slab_kernel<VolT, ProjT, FWD_PLAIN, R, false>; break;
+    case FWD_RESID: fn = fwd_slab_kernel<VolT, ProjT, FWD_RESID, R, false>; break;
+    case FWD_MLEM: fn = a.only_met ? fwd_slab_kernel<VolT, ProjT, FWD_MLEM, R, true> : fwd_slab_kernel<VolT, ProjT, FWD_MLEM, R, false>; break;
+    case FWD_SART: fn = a.only_met ? fwd_slab_kernel<VolT, ProjT, FWD_SART, R, true> : fwd_slab_kernel<VolT, ProjT, FWD_SART, R, false>; break;
+    case FWD_SART_ROWS: fn = a.only_met ? fwd_slab_kernel<VolT, ProjT, FWD_SART_ROWS, R, true> : fwd_slab_kernel<VolT, ProjT, FWD_SART_ROWS, R, false>; break;
     }
-    KV_CHECK_CUDA(plan->ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KV_CHECK_CUDA(plan->ctx, cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     LaunchTimer lt(plan->ctx, "exact_fwd");
-    switch (mode) {
-    case FWD_PLAIN: fwd_slab_kernel<VolT, ProjT, FWD_PLAIN, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
-    case FWD_MLEM: fwd_slab_kernel<VolT, ProjT, FWD_MLEM, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
-    case FWD_SART: fwd_slab_kernel<VolT, ProjT, FWD_SART, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
-    case FWD_RESID: fwd_slab_kernel<VolT, ProjT, FWD_RESID, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
-    case FWD_SART_ROWS: fwd_slab_kernel<VolT, ProjT, FWD_SART_ROWS, R><<<grid, kThreads, smem, st>>>(map, G, t, a, partials, A); break;
-    }
+    fn<<<grid, kThreads, smem, plan->ctx->stream>>>(map, G, t, a, partials, A);
     KV_CHECK_LAUNCH(plan->ctx, "fwd_slab_kernel");
     return KV_OK;
 }
@@ -635,6 +646,8 @@ kv_status fwd_slab_launch(kv_plan *plan, const FwdSlabCfg &c, const ExactTables 
     A.yi_off = L.yi_off;
     A.org_off = L.org_off;
     A.status = plan->ctx->d_status;
+    A.pitch = c.pitch;
+    a.only_met = a.only_met || c.pitch != g.nx;
     const ExGeom G{g.nx, g.ny, g.nz, g.nu, g.nv, P};
     const unsigned grid = (unsigned)((size_t)A.n_ut * A.n_vt * P);
     switch (plan->storage) {

@@ -254,6 +254,8 @@ struct FwdArgs {
     float *rows = nullptr;    // [P][nv][nu] row sums: stored by FWD_SART (null: not), read by FWD_SART_ROWS
     void *pad = nullptr;   // the plan's d_pad where the caller owns the plan's workspaces, else null: no padded slab
     bool pad_ready = false;   // d_pad already holds vol
+    bool only_met = false;    // FWD_MLEM, FWD_SART*: a voxel that is not finite reaches only the rays that meet it
+                              // (always so with d_pad)
 };
 struct BackArgs {
     const void *yp;        // ProjT [P][nv][nu], scaled by the ray factor Ls

@@ -94,3 +94,25 @@ def test_batch_of_tiny_problems(ctx, host):
         assert np.linalg.norm(x - w) <= 1e-5 * np.linalg.norm(w), i
         if plans[i] in large or i >= len(plans) - 4:   # its plan's own kernels
             assert np.array_equal(x, w), i
+
+
+def test_batch_with_voxels_that_are_not_finite(ctx):
+    """They reach the rays that meet them and no others, on whole and broken 16-byte rows: against one solve after
+    another with the one-thread-per-ray kernel, which reads only what a ray meets."""
+    torch = pytest.importorskip("torch")
+    plans, data = problems(ctx)
+    plans, data = plans[:5], data[:5]
+    want, xs = [], []
+    for i, (plan, p) in enumerate(zip(plans, data)):
+        x = np.random.default_rng(i).random(plan.geometry.volume_shape, dtype=np.float32) + 0.5
+        x[2, x.shape[1] // 2, x.shape[2] // 3] = (np.inf, np.nan)[i % 2]
+        xs.append(torch.from_numpy(x.copy()).cuda())
+        ray = engine.Plan(ctx, plan.geometry, "exact")
+        ray.set_slab(0)
+        ray.mlem(p, x, 2)
+        want.append(x)
+    engine.batch_mlem(ctx, plans, [torch.from_numpy(p).cuda() for p in data], xs, 2)
+    for x, w in zip(xs, want):
+        x, ok = x.cpu().numpy(), np.isfinite(w)
+        assert np.array_equal(np.isfinite(x), ok)
+        assert np.linalg.norm((x - w)[ok]) < 1e-6 * np.linalg.norm(w[ok])

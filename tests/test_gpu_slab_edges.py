@@ -89,3 +89,33 @@ def test_thin_volumes_of_few_rays_are_not_padded(ctx, geom, padded):
     plan.mlem(np.ones(g.proj_shape, np.float32), x, 1)
     ctx.set_timing(False)
     assert ("pad_rows" in ctx.read_timing()) == padded
+
+
+@pytest.mark.parametrize("storage", ["f32", "bf16"])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_nonfinite_voxel_reaches_only_the_rays_that_meet_it(ctx, storage, bad):
+    """Iterations on padded rows against the one-thread-per-ray kernel, from a volume with voxels that are not finite: the
+    same voxels become so, the others agree at the bounds above (the slab's lockstep reads, at length zero, up to two
+    columns beside a ray's own)."""
+    g = linear_sweep(39, 46, 19, 0.5, 0.5, 2.0, 5, 61, 54, 0.4, 0.4, 20.0)
+    rng = np.random.default_rng(8)
+    p = rng.random(g.proj_shape, dtype=np.float32)
+    start = rng.random(g.volume_shape, dtype=np.float32) + 0.5
+    start[9, 20, 17] = start[3, 11, 30] = bad
+    for sart in (False, True):
+        for n in (1, 2):
+            xs = []
+            for ray in (False, True):
+                plan = engine.Plan(ctx, g, "exact", storage)
+                if ray:
+                    plan.set_slab(0)
+                x = start.copy()
+                if sart:
+                    plan.sart(p, x, n, 0.5)
+                else:
+                    plan.mlem(p, x, n)
+                xs.append(x)
+            ok = np.isfinite(xs[1])
+            assert np.array_equal(np.isfinite(xs[0]), ok) and not ok.all()
+            d = np.linalg.norm((xs[0] - xs[1])[ok]) / np.linalg.norm(xs[1][ok])
+            assert d < (1e-6 if storage == "f32" else 2 ** -7)
