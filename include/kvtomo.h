@@ -322,9 +322,10 @@ kv_status kv_unet_forward(kv_unet *net, const float *in, float *out, int32_t D, 
  * stays a sum over the other voxels divided by D*H*W). */
 kv_status kv_unet_train_step(kv_unet *net, const float *in, const float *target, int32_t D, int32_t H,
                              int32_t W, float lr, float *loss, kv_mem mem);
-/* Loss and FP32 parameter gradients (host buffer of kv_unet_num_params).  The
- * weight gradients pair voxels outside the volume as zeros: an activation or
- * gradient at the border that is not finite makes those taps NaN too. */
+/* Loss and FP32 parameter gradients (host buffer of kv_unet_num_params).  An
+ * activation or gradient that is not finite makes the weight gradients NaN that
+ * it enters; at the border, the taps that pair it with the outside of the volume
+ * may be NaN or not. */
 kv_status kv_unet_gradients(kv_unet *net, const float *in, const float *target, int32_t D, int32_t H,
                             int32_t W, float *loss, float *grads, kv_mem mem);
 /* Checkpoint state: parameters, Adam moments (3 * num_params host floats) and

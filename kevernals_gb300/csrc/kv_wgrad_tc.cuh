@@ -27,9 +27,10 @@
 // the thirteen layers at 128 x 256 x 128 voxels: 13.5 ms with mma.sync, one tap
 // a CTA, -> 1.24 ms (0.54 TFLOP, 440 TFLOP/s).
 //
-// A voxel outside the volume enters as zero on either side, so a non-finite
-// activation or gradient at the border also reaches the taps that pair it with
-// the outside.
+// Along x and y a voxel outside the volume enters as zero: X's halo columns, dY's
+// halo rows.  Along z planes outside are not visited.  So a non-finite activation
+// in a border row, or gradient in a border column, also reaches the taps that
+// pair it with the outside; other border values do not.
 //
 // Warp roles (256 threads): warp 0 issues the TMA loads, warps 1-3 the MMAs of
 // dz = 0, 1, 2, warps 4-7 read the accumulators out.  Every wait is bounded,
