@@ -120,7 +120,7 @@ __device__ __forceinline__ bool in_volume(int col, int row, int nx, int ny) {
 // and third row are zero where there is none (make_desc), so only the rows
 // beyond compare with the ray's count (compared at every row, 60 views of 2048
 // x 2048 and 128 slices take 48.4 ms; from the third on 46.4; from the fourth,
-// as here, 45.6; never, 45.2).
+// as here, 45.3-45.6; never, 45.2).
 // Lengths in clamp form: with a1 = min(max(X1, lo), hi) and a2 likewise, the
 // ray spends a1 - lo in its first column, a2 - a1 in the second and hi - a2
 // in the third.  Where min(hi, X_{c+1}) - max(lo, X_c) is positive these are
