@@ -283,7 +283,7 @@ kv_status kv_plan_set_back_staging(kv_plan *plan, int rows_per_thread, int stage
  * or NULL; FP32 accumulation.  kernel: 0 = tcgen05 / TMA implicit GEMM on
  * volumes of whole 128-voxel tiles (KV_ERR_UNSUPPORTED where it does not cover
  * the channels), on other volumes where it covers the call, else mma.sync
- * (equal bits for finite weights); 1 = tcgen05 only, for volumes of whole
+ * (equal bits); 1 = tcgen05 only, for volumes of whole
  * tiles; 2 = mma.sync only.  W is a multiple of 16 but for volumes of whole
  * tiles with kernel 0 or 1.  Channel counts: multiples of 16 (the tcgen05
  * kernel: 16, 32, 64 or 128 per input, cout <= 256).  Stream-ordered

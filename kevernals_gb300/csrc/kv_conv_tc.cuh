@@ -24,9 +24,10 @@
 // An output plane is finished with dz = 2, read out, and its slot zeroed for
 // the plane three further on: every MMA accumulates.  Sums run over dz, then
 // (dy, dx), then 16-channel segments -- the tap order of the mma.sync kernel,
-// with equal bits (for finite weights: planes outside the volume are not
-// loaded, so an infinite weight does not meet their zeros) -- so a plane's
-// segments are all in shared memory at once.
+// with equal bits -- so a plane's segments are all in shared memory at once.
+// Planes outside the volume are not loaded; a weight that is not finite would
+// have made their zeros NaN, which a variant's epilogue adds (z_border; 1 % of the
+// network's time, which does without: its outputs are lost then anyway).
 // The weights stay there for the CTA's life where they fit beside the plane
 // buffers; else they stream through a ring, one (dy, dx) of up to four
 // segments at a time, each piece used for every sub-tile.
@@ -107,6 +108,7 @@ struct Params {
     uint32_t b_seg_bytes;         // weights of one segment (resident: nine taps, streamed: one)
     uint32_t chunks;              // ring of streamed weights, kChunkSegs segments each
     uint32_t tmem_cols;
+    const __nv_bfloat16 *w;       // [N][27][16 nseg], for z_border
     const float *bias;            // nullptr: none
     int relu;
     const __nv_bfloat16 *mask;    // nullptr: none; else outputs where mask <= 0 become 0
@@ -236,7 +238,48 @@ __device__ __forceinline__ void issue_taps(uint32_t t0, uint32_t t1, uint32_t a,
     __syncwarp();
 }
 
-template <int CG>
+// What the taps that reach a plane of zeros below (dz = 0, needed where `below`) or above (dz = 2, `above`) the volume
+// add to each of the channels n0 .. n0 + CG - 1: 0, or NaN where a weight is not finite.  Called by the WARPS warps that
+// drain accumulators while the first plane's MMAs run; their barrier makes it visible to them.
+template <int CG, int WARPS>
+__device__ __forceinline__ void z_border(const __nv_bfloat16 *w, int n0, int K, float (*border)[CG], bool below, bool above,
+                                         int warp, int lane) {
+    const int units = 9 * K / 8;   // of 16 bytes; the nine taps of one dz are contiguous
+    auto not_finite = [](uint4 q) {
+        const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+        bool bad = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bad |= (v[j] & 0x7f80u) == 0x7f80u || (v[j] & 0x7f800000u) == 0x7f800000u;
+        return bad;
+    };
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int n = warp; n < CG; n += WARPS) {
+        const uint4 *lo = reinterpret_cast<const uint4 *>(w + (size_t)(n0 + n) * 27 * K), *hi = lo + 2 * units;
+        bool bad_lo = false, bad_hi = false;
+        for (int i0 = lane; i0 < units; i0 += 128) {   // eight loads in flight
+            uint4 q[4], r[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                q[j] = below && i0 + 32 * j < units ? __ldg(lo + i0 + 32 * j) : zero;
+                r[j] = above && i0 + 32 * j < units ? __ldg(hi + i0 + 32 * j) : zero;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                bad_lo |= not_finite(q[j]);
+                bad_hi |= not_finite(r[j]);
+            }
+        }
+        const bool nan_lo = __any_sync(0xffffffffu, bad_lo), nan_hi = __any_sync(0xffffffffu, bad_hi);
+        if (lane == 0) {
+            border[0][n] = nan_lo ? __int_as_float(0x7fffffff) : 0.f;
+            border[1][n] = nan_hi ? __int_as_float(0x7fffffff) : 0.f;
+        }
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * WARPS) : "memory");
+}
+
+// ANY_W: the weights may hold infinities and NaN.
+template <int CG, bool ANY_W>
 __global__ void __launch_bounds__(threads(CG), 1)
     conv3_march_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1,
                        const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b2,
@@ -248,6 +291,7 @@ __global__ void __launch_bounds__(threads(CG), 1)
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_flag;
     __shared__ unsigned long long issued_sh, b_issued_sh;   // planes / pieces of weights loaded by TMA
+    __shared__ float border[2][CG];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
 
@@ -467,6 +511,12 @@ __global__ void __launch_bounds__(threads(CG), 1)
 #pragma unroll
             for (int j = 0; j < 17; ++j) hw[j] = __ldg(j < 16 ? P.head.w + j : P.head.b);
         }
+        if (ANY_W && u_begin < u_end) {
+            const long long first = u_begin % P.D, last = first + (u_end - u_begin) - 1;
+            const bool below = first == 0 || last >= P.D, above = last >= P.D - 1;   // of the output planes of this share
+            if (below || above)
+                z_border<CG, 4 * kSets>(P.w, cg * CG, P.nseg * kSeg, border, below, above, warp - 1 - kIssuers, lane);
+        }
         uint32_t plane_phase = 0;
         bool ok = true;
         for (long long u = u_begin; u < u_end && ok;) {
@@ -493,6 +543,16 @@ __global__ void __launch_bounds__(threads(CG), 1)
                         tc_wait_ld();
 #pragma unroll
                         for (int q = 0; q < CG / 16; ++q) tc_zero16(ta + (uint32_t)(16 * q));
+                        if (ANY_W && (zo == 0 || zo == P.D - 1)) {   // of its own: in the loop below it cost the network 7 %
+                            const float *lo = border[0], *hi = border[1];
+                            if (zo != 0) lo = hi;
+                            if (zo != P.D - 1) hi = lo;
+#pragma unroll
+                            for (int q = 0; q < CG / 16; ++q)
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    v[q][j] = __float_as_uint(__uint_as_float(v[q][j]) + (lo[16 * q + j] + hi[16 * q + j]));
+                        }
                         if (live) {
                             const size_t o = (((size_t)zo * P.H + y) * P.W + x) * P.N + cg * CG;
 #pragma unroll
@@ -726,11 +786,12 @@ inline bool plan_shape(Params &P, int CG, int sm_count, int *grid, size_t *smem)
 
 // out[v][N] = conv3(in1 (c1 channels) ++ in2 (c2 channels), w [N][27][c1+c2]) + bias, ReLU optional, zero where
 // `mask` (a tensor like out; nullptr: none) is not positive; out may be nullptr where `head` takes the result.
+// any_w: the weights may hold infinities and NaN (which meet the zeros outside the volume).
 // Returns a message on a configuration this kernel does not cover (nullptr: launched).
 inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 *in2, int c2,
                           const __nv_bfloat16 *w, const float *bias, bool relu, const __nv_bfloat16 *mask,
-                          const Head *head, __nv_bfloat16 *out, int N, int D, int H, int W, int *status, int sm_count,
-                          cudaStream_t stream) {
+                          const Head *head, __nv_bfloat16 *out, int N, int D, int H, int W, bool any_w, int *status,
+                          int sm_count, cudaStream_t stream) {
     if (encoder() == nullptr) return "cuTensorMapEncodeTiled is not available";
     const int K = c1 + c2;
     auto ok_c = [](int c) { return c == 16 || c == 32 || c == 64 || c == 128; };
@@ -759,6 +820,7 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
     if (!plan_shape(P, CG, sm_count, &grid, &smem)) return "no tile shape for this volume";
     P.tmem_cols = 32;
     while (P.tmem_cols < (uint32_t)(3 * CG * P.T)) P.tmem_cols <<= 1;
+    P.w = w;
     P.bias = bias;
     P.relu = relu ? 1 : 0;
     P.mask = mask;
@@ -780,10 +842,10 @@ inline const char *launch(const __nv_bfloat16 *in1, int c1, const __nv_bfloat16 
         return nullptr;
     };
     switch (CG) {
-    case 16: return go(conv3_march_kernel<16>);
-    case 32: return go(conv3_march_kernel<32>);
-    case 48: return go(conv3_march_kernel<48>);
-    default: return go(conv3_march_kernel<64>);
+    case 16: return any_w ? go(conv3_march_kernel<16, true>) : go(conv3_march_kernel<16, false>);
+    case 32: return any_w ? go(conv3_march_kernel<32, true>) : go(conv3_march_kernel<32, false>);
+    case 48: return any_w ? go(conv3_march_kernel<48, true>) : go(conv3_march_kernel<48, false>);
+    default: return any_w ? go(conv3_march_kernel<64, true>) : go(conv3_march_kernel<64, false>);
     }
 }
 

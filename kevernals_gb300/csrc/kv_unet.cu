@@ -595,7 +595,7 @@ kv_status conv3(kv_unet *u, int layer, const bf16 *in1, const bf16 *in2, bf16 *o
     const float *bias = weights_t ? nullptr : u->p + L.b;
     LaunchTimer lt(ctx, weights_t ? "unet_conv_dgrad" : "unet_conv_fwd");
     // tcgen05 / TMA implicit GEMM (kv_conv_tc.cuh); covers every level of every volume the network takes
-    const char *why = convtc::launch(in1, c1, in2, c2, w, bias, !weights_t, mask, head, out, cout, D, H, W,
+    const char *why = convtc::launch(in1, c1, in2, c2, w, bias, !weights_t, mask, head, out, cout, D, H, W, false,
                                      u->tc_status, ctx->sm_count, ctx->stream);
     if (why != nullptr) return kv_fail(ctx, KV_ERR_UNSUPPORTED, "tensor-core convolution: %s", why);
     KV_CHECK_LAUNCH(ctx, "unet conv3 (tcgen05)");
@@ -990,7 +990,7 @@ extern "C" kv_status kv_conv3_bf16(kv_ctx *ctx, const uint16_t *in1, int32_t c1,
     // covers the call, else mma.sync; the two sum in the same order, with equal bits
     if (kernel != 2 && (tiles || W % 16 == 0)) {
         const char *why = convtc::launch(a, c1, c2 ? b : nullptr, c2, wb, bias, relu != 0, nullptr, nullptr, o, cout, D, H, W,
-                                         ctx->d_status, ctx->sm_count, ctx->stream);
+                                         true, ctx->d_status, ctx->sm_count, ctx->stream);
         if (why == nullptr) {
             KV_CHECK_LAUNCH(ctx, "kv_conv3_bf16 (tcgen05)");
             return KV_OK;

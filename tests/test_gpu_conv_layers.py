@@ -169,3 +169,25 @@ def test_conv_narrow_whole_tiles(ctx, dims):
         bits = _conv(ctx, a, 32, a, 0, w, bias, False, 16, dims, kernel)
         got = (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
         assert np.all(np.abs(got - ref) <= 2 ** -8 * np.abs(ref) + 2 ** -20 * mag)
+
+
+@pytest.mark.parametrize("shape", [(16, 16, 128, 16, 0, 16), (4, 32, 32, 64, 0, 64), (3, 5, 128, 16, 16, 48), (1, 8, 16, 32, 0, 32),
+                                   (2, 9, 64, 64, 32, 32), (5, 4, 256, 128, 64, 64)],
+                         ids=lambda s: "x".join(map(str, s[:3])) + f"_{s[3]}+{s[4]}to{s[5]}")
+@pytest.mark.parametrize("tap", [4, 13, 22])   # of the plane before, this one, the one after
+def test_conv_weights_that_are_not_finite(ctx, shape, tap):
+    """An infinity and a NaN among the weights, one a channel: the zeros outside the volume make NaN of them, as in the
+    mma.sync kernel; every other channel is untouched."""
+    pytest.importorskip("torch")
+    D, H, W, c1, c2, cout = shape
+    rng = np.random.default_rng(sum(shape))
+    a, _ = _bf16_bits(np.abs(rng.standard_normal((D, H, W, c1))).astype(np.float32) + 0.1)
+    b, _ = _bf16_bits(np.abs(rng.standard_normal((D, H, W, max(c2, 1)))).astype(np.float32) + 0.1)
+    w, _ = _bf16_bits((rng.standard_normal((cout, 27, c1 + c2)) / np.sqrt(27 * (c1 + c2))).astype(np.float32))
+    w[3, tap, 5], w[cout - 2, tap, c1 + c2 - 1] = 0x7f80, 0x7fc0
+    bias = (rng.standard_normal(cout) * 0.1).astype(np.float32)
+    want = _conv(ctx, a, c1, b, c2, w, bias, False, cout, (D, H, W), 2)
+    got = _conv(ctx, a, c1, b, c2, w, bias, False, cout, (D, H, W), 0)
+    nan_w, nan_g = (want & 0x7fff) > 0x7f80, (got & 0x7fff) > 0x7f80
+    assert nan_w.any() and np.array_equal(nan_g, nan_w)
+    assert np.array_equal(got[~nan_w], want[~nan_w])
